@@ -3,19 +3,20 @@
 //
 // Reference: tree_create (src/tree.cpp:273-601) builds the tree recursively on the host,
 // splitting each node at the midpoint of its box's longest dimension with the in-place
-// two-pointer partition particles_sort (src/particles.cpp:979-1018).  Here all nodes of one
-// depth are split together:
+// two-pointer partition particles_sort (src/particles.cpp:979-1018).  Here one cooperative launch
+// splits all nodes of one depth together, level after level:
 //   1. classify: leaf or split, split dimension and midpoint (tree.cpp:314-348);
-//   2. partition every split node's range with the exact permutation of the two-pointer
+//   2. number the children in node order;
+//   3. partition every split node's range with the exact permutation of the two-pointer
 //      loop: with m = #(x < xmid), the k-th element >= xmid in [b, b+m) (counted from the left)
 //      swaps with the k-th element < xmid in [b+m, e) (counted from the right);
-//   3. create the children.
+//   4. create the children.
 // The upsweep then runs deepest level first: leaf tight boxes, centres, radii and P2M
 // (tree.cpp:498-571), interior unions, the two centre/radius candidates and M2M in double
 // (tree.cpp:355-497).  Particles are reordered by moving x, y, z and an index; velocities
 // and rungs are gathered through the index at the end (same final arrays as swapping all
 // fields in the reference's loop).
-#include <cub/cub.cuh>
+#include <cstddef>
 
 #include "ct_internal.cuh"
 #include "ct_ops.cuh"
@@ -23,394 +24,587 @@
 namespace ct {
 namespace {
 
-constexpr int TPB = 256;
-constexpr int PER_T = 8;
-constexpr int TILE = TPB * PER_T;
+// ---------------------------------------------------------------- the levels
+// One cooperative launch builds every level: a resident grid whose blocks meet at grid barriers
+// between the phases of a level.  What bounded the build before was the level's structure, not its
+// data: twelve launches, two scans and a host round trip a level (16^3 particles: 0.87 ms for 11
+// levels and 64 KB of positions; 10^6 clustered particles: 2.7 ms for 28 levels).  A level whose
+// split nodes all hold at most WARP_NODE particles takes two barriers, others five.
+constexpr int LTPB = 512;             // threads of a level block
+constexpr int LWARPS = LTPB / 32;
+constexpr int TILE_ROWS = 8;
+constexpr int TILE = LTPB * TILE_ROWS;  // particles of a tile
+constexpr int WARP_NODE = 1024;       // nodes up to this size are partitioned by one warp: its lanes
+                                      // hold the 32 ballots of the node's particles
+constexpr int NODE_SPLIT = 2, NODE_TILES = 4;  // NodeW.flags while a level is built
 
-struct BuildScratch {
-	int32_t* idx;        // particle index being permuted [n]
-	int32_t* posL;       // partition scratch [n]
-	int32_t* posR;       // partition scratch [n]
-	int32_t* split;      // per node of the level: 1 if split
-	int32_t* rank;       // exclusive scan of split
-	int32_t* ntiles;     // tiles per node of the level
-	int32_t* tile_off;   // exclusive scan of ntiles
-	int32_t* xdim;       // split dimension per node of the level
-	uint32_t* xmidf;     // fixed32 midpoint per node of the level
-	double* xmid;        // double midpoint per node of the level
-	int32_t* node_m;     // # below midpoint per node of the level
-	int32_t* node_nmis;  // # swaps per node of the level
-	int32_t* tile_node;  // per tile: node (local index in level)
-	int32_t* tile_lt;    // per tile: # below midpoint
-	int32_t* tile_offL;  // per tile: # misplaced-left in earlier tiles of the node
-	int32_t* tile_offR;  // per tile: # misplaced-right in later tiles of the node
-	int32_t* totals;     // [0] nsplit, [1] ntiles (device)
-	void* cub_tmp;
-	size_t cub_bytes;
+// A node partitioned in tiles by the whole grid.
+struct TileNode {
+	int32_t node;   // index of the node
+	int32_t t0;     // its first tile
+	int32_t nt;     // its tiles
+	int32_t m;      // particles below the midpoint
+	int32_t nswap;  // swaps
 };
 
-__device__ __forceinline__ int block_sum_int(int v, int* sh) {
-	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-	for (int o = 16; o; o >>= 1) {
-		v += __shfl_down_sync(0xffffffffu, v, o);
-	}
+struct LevelCtl {
+	unsigned int arrived;  // barrier arrivals of this launch
+	int error;             // a barrier gave up
+	int status;            // 0 done, 1 the node arrays are full before `level`
+	int level;
+	int64_t lb, le;        // nodes of `level`
+	int64_t need;          // nodes the arrays must hold
+	int64_t start[MAX_DEPTH + 2];
+};
+
+struct LevelArgs {
+	NodeW* nodes;
+	double* gbox;
+	uint64_t* key;
+	int32_t* depth;
+	int32_t* parent;
+	uint32_t* x[3];
+	int32_t* idx;   // particle index being permuted
+	int32_t* posL;  // partition scratch [n]
+	int32_t* posR;
+	TileNode* tnode;
+	int32_t* tile_of;  // tile -> entry of tnode
+	int32_t* tile_lt;  // tile -> particles below the midpoint
+	int4* blk;         // per block: split nodes, tile nodes, tiles of its share of a level
+	LevelCtl* ctl;
+	int* flags;
+	const int64_t* off;
+	int64_t pb, n, node_cap;
+	int nroot, bucket, resume;
+	double theta, hsoft;
+};
+
+// All blocks of the (cooperative) grid meet; false when one gave up waiting.  The counter only
+// grows, `round` is the calling block's number of barriers so far.
+__device__ __forceinline__ bool grid_meet(LevelCtl* ctl, unsigned int& round) {
 	__syncthreads();
-	if (lane == 0) {
-		sh[w] = v;
-	}
-	__syncthreads();
-	int t = 0;
-	for (int i = 0; i < (int) (blockDim.x >> 5); i++) {
-		t += sh[i];
-	}
-	__syncthreads();
-	return t;
-}
-
-// Exclusive block scan of ints; returns the block total through *total.
-__device__ __forceinline__ int block_excl_scan(int v, int* sh, int* total) {
-	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-	int inc = v;
-	for (int o = 1; o < 32; o <<= 1) {
-		const int t = __shfl_up_sync(0xffffffffu, inc, o);
-		if (lane >= o) {
-			inc += t;
-		}
-	}
-	__syncthreads();
-	if (lane == 31) {
-		sh[w] = inc;
-	}
-	__syncthreads();
-	int base = 0, tot = 0;
-	for (int i = 0; i < (int) (blockDim.x >> 5); i++) {
-		if (i < w) {
-			base += sh[i];
-		}
-		tot += sh[i];
-	}
-	__syncthreads();
-	*total = tot;
-	return base + inc - v;
-}
-
-// One root per sub-box: node s covers the unit box and particles [off[s], off[s+1]), except
-// that a single box starts at the active range [pbeg, pend).
-__global__ void k_init_roots(int nroot, const int64_t* off, NodeW* nodes, double* gbox, uint64_t* key, int32_t* depth, int32_t* parent, int32_t pbeg,
-		int32_t pend) {
-	const int s = blockIdx.x * blockDim.x + threadIdx.x;
-	if (s >= nroot) {
-		return;
-	}
-	NodeW r;
-	r.x = r.y = r.z = 0;
-	r.radius = 0.f;
-	r.pbeg = nroot == 1 ? pbeg : (int32_t) off[s];
-	r.pend = nroot == 1 ? pend : (int32_t) off[s + 1];
-	r.child = -1;
-	r.flags = 1;
-	nodes[s] = r;
-	for (int d = 0; d < 3; d++) {
-		gbox[6 * s + d] = 0.0;
-		gbox[6 * s + 3 + d] = 1.0;
-	}
-	key[s] = 1;
-	depth[s] = 0;
-	parent[s] = -1;
-}
-
-__global__ void k_iota(int32_t* idx, int64_t n) {
-	for (int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < n; i += (int64_t) gridDim.x * blockDim.x) {
-		idx[i] = (int32_t) i;
-	}
-}
-
-// Leaf or split (tree.cpp:314-348).
-__global__ void k_classify(int64_t lb, int nl, const NodeW* nodes, const double* gbox, const int32_t* depth, double theta, double hsoft, int bucket,
-		BuildScratch s, int* flags) {
-	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nl; i += gridDim.x * blockDim.x) {
-		const int64_t ni = lb + i;
-		const NodeW nd = nodes[ni];
-		const int nparts = nd.pend - nd.pbeg;
-		const double* gb = gbox + 6 * ni;
-		float box_r = 0.0f;
-		for (int dim = 0; dim < 3; dim++) {
-			const double h = 0.5 * (gb[3 + dim] - gb[dim]);
-			box_r += h * h;
-		}
-		box_r = sqrtf(box_r);
-		const bool ewald_satisfied = (box_r < 0.25 * (theta / (1.0 + theta)) && box_r < 0.125 - 0.25 * hsoft);
-		bool split = nparts > bucket || (!ewald_satisfied && nparts > 0);
-		if (split && depth[ni] >= MAX_DEPTH - 1) {
-			atomicOr(flags + 2, 1);
-			split = false;
-		}
-		int xdim = 0;
-		double max_span = -1.0;
-		for (int dim = 0; dim < 3; dim++) {
-			const double span = gb[3 + dim] - gb[dim];
-			if (span > max_span) {
-				max_span = span;
-				xdim = dim;
+	int bad = 0;
+	round++;
+	if (threadIdx.x == 0) {
+		__threadfence();
+		const unsigned int target = round * gridDim.x;
+		if (atomicAdd(&ctl->arrived, 1u) + 1u != target) {
+			const volatile unsigned int* arrived = &ctl->arrived;
+			const volatile int* error = &ctl->error;
+			unsigned long long t0, t;
+			asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+			while ((int) (*arrived - target) < 0 && !bad) {
+				asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+				bad = *error != 0 || t - t0 > 30000000000ull;  // 30 s: another kernel may hold the SMs for a while
+			}
+			if (bad) {
+				atomicExch(&ctl->error, 1);
 			}
 		}
-		const double xm = 0.5 * (gb[3 + xdim] + gb[xdim]);
-		s.split[i] = split;
-		s.ntiles[i] = split ? (nparts + TILE - 1) / TILE : 0;
-		s.xdim[i] = xdim;
-		s.xmid[i] = xm;
-		s.xmidf[i] = fixed_from_double(xm);
+		__threadfence();
 	}
+	return !__syncthreads_or(bad);
 }
 
-__global__ void k_tile_map(int nl, BuildScratch s) {
-	const int lane = threadIdx.x & 31;
-	const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-	const int nw = (gridDim.x * blockDim.x) >> 5;
-	for (int i = wid; i < nl; i += nw) {
-		const int nt = s.ntiles[i];
-		const int t0 = s.tile_off[i];
-		for (int t = lane; t < nt; t += 32) {
-			s.tile_node[t0 + t] = i;
+// Longest side of a node's box and its midpoint (tree.cpp:336-348).
+__device__ __forceinline__ int split_dim(const double* gb, double& xm) {
+	int xdim = 0;
+	double max_span = -1.0;
+	for (int dim = 0; dim < 3; dim++) {
+		const double span = gb[3 + dim] - gb[dim];
+		if (span > max_span) {
+			max_span = span;
+			xdim = dim;
 		}
 	}
+	xm = 0.5 * (gb[3 + xdim] + gb[xdim]);
+	return xdim;
 }
 
-__device__ __forceinline__ void tile_range(const NodeW& nd, int t, int t0, int* tb, int* te) {
-	*tb = nd.pbeg + (t - t0) * TILE;
-	*te = min(*tb + TILE, nd.pend);
-}
-
-// P1: elements below the midpoint per tile.
-__global__ void __launch_bounds__(TPB) k_count(int64_t lb, int ntile, const NodeW* nodes, const uint32_t* x0, const uint32_t* x1, const uint32_t* x2,
-		BuildScratch s) {
-	__shared__ int sh[32];
-	const uint32_t* xs[3] = { x0, x1, x2 };
-	for (int t = blockIdx.x; t < ntile; t += gridDim.x) {
-		const int i = s.tile_node[t];
-		const NodeW nd = nodes[lb + i];
-		int tb, te;
-		tile_range(nd, t, s.tile_off[i], &tb, &te);
-		const uint32_t* xd = xs[s.xdim[i]];
-		const uint32_t xm = s.xmidf[i];
-		int c = 0;
-		const int p0 = tb + threadIdx.x * PER_T;
-		for (int j = 0; j < PER_T; j++) {
-			const int p = p0 + j;
-			if (p < te) {
-				c += xd[p] < xm;
-			}
-		}
-		c = block_sum_int(c, sh);
-		if (threadIdx.x == 0) {
-			s.tile_lt[t] = c;
-		}
-	}
-}
-
-// P2: per split node, midpoint count m and per-tile offsets of misplaced elements.
-__global__ void __launch_bounds__(TPB) k_node_scan(int64_t lb, int nl, const NodeW* nodes, const uint32_t* x0, const uint32_t* x1, const uint32_t* x2,
-		BuildScratch s) {
-	__shared__ int sh[32];
-	__shared__ int s_strad[3];
-	const uint32_t* xs[3] = { x0, x1, x2 };
-	for (int i = blockIdx.x; i < nl; i += gridDim.x) {
-		if (!s.split[i]) {
-			continue;
-		}
-		const NodeW nd = nodes[lb + i];
-		const int t0 = s.tile_off[i];
-		const int nt = s.ntiles[i];
-		int m = 0;
-		for (int k = threadIdx.x; k < nt; k += TPB) {
-			m += s.tile_lt[t0 + k];
-		}
-		m = block_sum_int(m, sh);
-		const int sp = nd.pbeg + m;
-		const uint32_t* xd = xs[s.xdim[i]];
-		const uint32_t xm = s.xmidf[i];
-		// the tile holding the split point strictly inside it
-		const int ts = (sp - nd.pbeg) / TILE;
-		int sL = 0, sR = 0;
-		if (ts < nt) {
-			int tb, te;
-			tile_range(nd, t0 + ts, t0, &tb, &te);
-			if (tb < sp && sp < te) {
-				const int p0 = tb + threadIdx.x * PER_T;
-				for (int j = 0; j < PER_T; j++) {
-					const int p = p0 + j;
-					if (p < te) {
-						const bool lt = xd[p] < xm;
-						sL += (p < sp) && !lt;
-						sR += (p >= sp) && lt;
-					}
-				}
-			}
-		}
-		sL = block_sum_int(sL, sh);
-		sR = block_sum_int(sR, sh);
-		if (threadIdx.x == 0) {
-			s_strad[0] = sL;
-			s_strad[1] = sR;
-		}
-		__syncthreads();
-		// prefix of misplaced-left (left to right) and inclusive prefix of misplaced-right
-		int carryL = 0, carryR = 0;
-		for (int k0 = 0; k0 < nt; k0 += TPB) {
-			const int k = k0 + threadIdx.x;
-			int mL = 0, mR = 0;
-			if (k < nt) {
-				int tb, te;
-				tile_range(nd, t0 + k, t0, &tb, &te);
-				const int lt = s.tile_lt[t0 + k];
-				if (te <= sp) {
-					mL = (te - tb) - lt;
-				} else if (tb >= sp) {
-					mR = lt;
-				} else {
-					mL = s_strad[0];
-					mR = s_strad[1];
-				}
-			}
-			int totL, totR;
-			const int exL = block_excl_scan(mL, sh, &totL);
-			const int exR = block_excl_scan(mR, sh, &totR);
-			if (k < nt) {
-				s.tile_offL[t0 + k] = carryL + exL;
-				s.tile_offR[t0 + k] = carryR + exR + mR;  // inclusive, fixed below
-			}
-			carryL += totL;
-			carryR += totR;
-		}
-		__syncthreads();
-		for (int k = threadIdx.x; k < nt; k += TPB) {
-			s.tile_offR[t0 + k] = carryR - s.tile_offR[t0 + k];  // misplaced-right in later tiles
-		}
-		if (threadIdx.x == 0) {
-			s.node_m[i] = m;
-			s.node_nmis[i] = carryL;
-		}
-		__syncthreads();
-	}
-}
-
-// P3: positions of the misplaced elements, ranked from the left (left region) and from the
-// right (right region).
-__global__ void __launch_bounds__(TPB) k_positions(int64_t lb, int ntile, const NodeW* nodes, const uint32_t* x0, const uint32_t* x1,
-		const uint32_t* x2, BuildScratch s) {
-	__shared__ int sh[32];
-	const uint32_t* xs[3] = { x0, x1, x2 };
-	for (int t = blockIdx.x; t < ntile; t += gridDim.x) {
-		const int i = s.tile_node[t];
-		const NodeW nd = nodes[lb + i];
-		int tb, te;
-		tile_range(nd, t, s.tile_off[i], &tb, &te);
-		const int sp = nd.pbeg + s.node_m[i];
-		const uint32_t* xd = xs[s.xdim[i]];
-		const uint32_t xm = s.xmidf[i];
-		const int p0 = tb + threadIdx.x * PER_T;
-		unsigned mskL = 0, mskR = 0;
-		for (int j = 0; j < PER_T; j++) {
-			const int p = p0 + j;
-			if (p < te) {
-				const bool lt = xd[p] < xm;
-				if (p < sp && !lt) {
-					mskL |= 1u << j;
-				}
-				if (p >= sp && lt) {
-					mskR |= 1u << j;
-				}
-			}
-		}
-		int totL, totR;
-		const int exL = block_excl_scan(__popc(mskL), sh, &totL);
-		const int exR = block_excl_scan(__popc(mskR), sh, &totR);
-		const int baseL = s.tile_offL[t] + exL;
-		const int baseR = s.tile_offR[t];
-		int cL = 0, cR = 0;
-		for (int j = 0; j < PER_T; j++) {
-			const int p = p0 + j;
-			if (mskL & (1u << j)) {
-				s.posL[nd.pbeg + baseL + cL] = p;
-				cL++;
-			}
-			if (mskR & (1u << j)) {
-				cR++;
-				// misplaced-right elements of this tile after p: totR - (exR + cR)
-				s.posR[nd.pbeg + baseR + (totR - (exR + cR))] = p;
-			}
-		}
-	}
-}
-
-// P4: the swaps.
-__global__ void __launch_bounds__(TPB) k_swap(int64_t lb, int ntile, const NodeW* nodes, uint32_t* x0, uint32_t* x1, uint32_t* x2, BuildScratch s) {
-	for (int t = blockIdx.x; t < ntile; t += gridDim.x) {
-		const int i = s.tile_node[t];
-		const NodeW nd = nodes[lb + i];
-		int tb, te;
-		tile_range(nd, t, s.tile_off[i], &tb, &te);
-		const int nmis = s.node_nmis[i];
-		for (int p = tb + threadIdx.x; p < te; p += TPB) {
-			const int k = p - nd.pbeg;
-			if (k < nmis) {
-				const int a = s.posL[nd.pbeg + k];
-				const int b = s.posR[nd.pbeg + k];
-				uint32_t t0 = x0[a];
-				x0[a] = x0[b];
-				x0[b] = t0;
-				t0 = x1[a];
-				x1[a] = x1[b];
-				x1[b] = t0;
-				t0 = x2[a];
-				x2[a] = x2[b];
-				x2[b] = t0;
-				const int32_t ti = s.idx[a];
-				s.idx[a] = s.idx[b];
-				s.idx[b] = ti;
-			}
-		}
-	}
-}
-
-__global__ void k_children(int64_t lb, int nl, int64_t cb, NodeW* nodes, double* gbox, uint64_t* key, int32_t* depth, int32_t* parent, BuildScratch s) {
-	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nl; i += gridDim.x * blockDim.x) {
-		const int64_t ni = lb + i;
-		NodeW nd = nodes[ni];
-		if (!s.split[i]) {
-			nd.child = -1;
-			nd.flags = 1;
-			nodes[ni] = nd;
-			continue;
-		}
-		const int64_t l = cb + 2 * (int64_t) s.rank[i];
-		const int64_t r = l + 1;
-		nd.child = (int32_t) l;
-		nd.flags = 0;
-		nodes[ni] = nd;
-		const int mid = nd.pbeg + s.node_m[i];
+// The two children of node ni, split at particle `mid`, by the lanes of a warp.
+__device__ __forceinline__ void make_children(const LevelArgs& a, int64_t ni, const NodeW& nd, int mid, int xd, double xm, int level, int lane) {
+	const int64_t l = nd.child;
+	if (lane < 2) {
 		NodeW c;
 		c.x = c.y = c.z = 0;
 		c.radius = 0.f;
 		c.child = -1;
 		c.flags = 1;
-		c.pbeg = nd.pbeg;
-		c.pend = mid;
-		nodes[l] = c;
-		c.pbeg = mid;
-		c.pend = nd.pend;
-		nodes[r] = c;
-		const int xd = s.xdim[i];
-		for (int d = 0; d < 6; d++) {
-			gbox[6 * l + d] = gbox[6 * ni + d];
-			gbox[6 * r + d] = gbox[6 * ni + d];
+		c.pbeg = lane == 0 ? nd.pbeg : mid;
+		c.pend = lane == 0 ? mid : nd.pend;
+		a.nodes[l + lane] = c;
+		a.key[l + lane] = (a.key[ni] << 1) + lane;
+		a.depth[l + lane] = level + 1;
+		a.parent[l + lane] = (int32_t) ni;
+	}
+	if (lane < 12) {
+		const int side = lane / 6, d = lane % 6;
+		a.gbox[6 * (l + side) + d] = d == (side == 0 ? 3 + xd : xd) ? xm : a.gbox[6 * ni + d];
+	}
+}
+
+__device__ __forceinline__ void swap_particles(const LevelArgs& a, int p, int q) {
+#pragma unroll
+	for (int d = 0; d < 3; d++) {
+		const uint32_t t = a.x[d][p];
+		a.x[d][p] = a.x[d][q];
+		a.x[d][q] = t;
+	}
+	const int32_t t = a.idx[p];
+	a.idx[p] = a.idx[q];
+	a.idx[q] = t;
+}
+
+// The partition of a node of at most WARP_NODE particles by one warp: lane c keeps the ballot of
+// particles 32 c .. 32 c + 31.  With m of them below the midpoint, the k-th particle at or above it
+// in the first m (from the left) changes places with the k-th below it in the rest (from the
+// right), which is the reference's two-pointer loop.  pos: WARP_NODE offsets in shared memory.
+__device__ __forceinline__ int warp_partition(const LevelArgs& a, const NodeW& nd, const uint32_t* xd, uint32_t xm, uint16_t* pos, int lane) {
+	const int n = nd.pend - nd.pbeg;
+	const uint32_t* xp = xd + nd.pbeg;
+	unsigned mine = 0;
+	for (int c0 = 0; c0 * 32 < n; c0 += 8) {
+		uint32_t v[8];
+#pragma unroll
+		for (int j = 0; j < 8; j++) {
+			const int p = 32 * (c0 + j) + lane;
+			v[j] = p < n ? xp[p] : 0xffffffffu;
 		}
-		gbox[6 * l + 3 + xd] = s.xmid[i];
-		gbox[6 * r + xd] = s.xmid[i];
-		key[l] = key[ni] << 1;
-		key[r] = (key[ni] << 1) + 1;
-		depth[l] = depth[r] = depth[ni] + 1;
-		parent[l] = parent[r] = (int32_t) ni;
+#pragma unroll
+		for (int j = 0; j < 8; j++) {
+			const unsigned lt = __ballot_sync(0xffffffffu, 32 * (c0 + j) + lane < n && v[j] < xm);
+			mine = lane == c0 + j ? lt : mine;
+		}
+	}
+	int m = __popc(mine);
+	for (int o = 16; o; o >>= 1) {
+		m += __shfl_xor_sync(0xffffffffu, m, o);
+	}
+	// this lane's 32 particles: those before the split point that are not below, and below after it
+	const int first = 32 * lane;
+	const unsigned valid = first >= n ? 0u : (n - first >= 32 ? 0xffffffffu : (1u << (n - first)) - 1u);
+	const unsigned before = first >= m ? 0u : (m - first >= 32 ? 0xffffffffu : (1u << (m - first)) - 1u);
+	unsigned L = before & ~mine & valid, R = mine & ~before;
+	int cl = __popc(L), cr = __popc(R);
+	int il = cl, ir = cr;
+	for (int o = 1; o < 32; o <<= 1) {
+		const int tl = __shfl_up_sync(0xffffffffu, il, o), tr = __shfl_up_sync(0xffffffffu, ir, o);
+		il += lane >= o ? tl : 0;
+		ir += lane >= o ? tr : 0;
+	}
+	const int ns = __shfl_sync(0xffffffffu, il, 31);  // as many on the right
+	if (ns > 0) {
+		uint16_t* pl = pos;
+		uint16_t* pr = pos + WARP_NODE / 2;
+		int k = il - cl;
+		while (L) {
+			pl[k++] = (uint16_t) (first + __ffs(L) - 1);
+			L &= L - 1;
+		}
+		k = ns - 1 - (ir - cr);
+		while (R) {
+			pr[k--] = (uint16_t) (first + __ffs(R) - 1);
+			R &= R - 1;
+		}
+		__syncwarp();
+		for (int q = lane; q < ns; q += 32) {
+			swap_particles(a, nd.pbeg + pl[q], nd.pbeg + pr[q]);
+		}
+		__syncwarp();
+	}
+	return m;
+}
+
+__global__ void __launch_bounds__(LTPB, 2) k_tree_levels(const LevelArgs a) {
+	__shared__ uint16_t s_pos[LWARPS][WARP_NODE];
+	__shared__ int s_cnt[TILE_ROWS * LWARPS];
+	__shared__ int s_scan[3][LWARPS];
+	__shared__ int s_sum[2][LWARPS];
+	__shared__ int s_next;
+	const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+	const unsigned lt_lane = (1u << lane) - 1u;
+	LevelCtl* ctl = a.ctl;
+	unsigned int round = 0;
+	int level = 0;
+	int64_t lb = 0, le = a.nroot;
+	if (a.resume) {
+		level = ctl->level;
+		lb = ctl->lb;
+		le = ctl->le;
+	} else {
+		const int64_t gt = blockIdx.x * (int64_t) LTPB + tid, gs = gridDim.x * (int64_t) LTPB;
+		for (int64_t i = gt; i < a.n; i += gs) {
+			a.idx[i] = (int32_t) i;
+		}
+		// one root per box: node s covers the unit box and particles [off[s], off[s+1]), except that
+		// a single box starts at the active range
+		for (int64_t s = gt; s < a.nroot; s += gs) {
+			NodeW r;
+			r.x = r.y = r.z = 0;
+			r.radius = 0.f;
+			r.pbeg = a.nroot == 1 ? (int32_t) a.pb : (int32_t) a.off[s];
+			r.pend = a.nroot == 1 ? (int32_t) a.n : (int32_t) a.off[s + 1];
+			r.child = -1;
+			r.flags = 1;
+			a.nodes[s] = r;
+			for (int d = 0; d < 3; d++) {
+				a.gbox[6 * s + d] = 0.0;
+				a.gbox[6 * s + 3 + d] = 1.0;
+			}
+			a.key[s] = 1;
+			a.depth[s] = 0;
+			a.parent[s] = -1;
+		}
+		if (!grid_meet(ctl, round)) {
+			return;
+		}
+	}
+	for (;; level++) {
+		const int64_t nl = le - lb;
+		const int64_t share = (nl + gridDim.x - 1) / gridDim.x;  // consecutive nodes of a block
+		const int64_t cb = lb + min(nl, share * blockIdx.x), ce = lb + min(nl, share * (blockIdx.x + 1));
+		// ---- leaf or split (tree.cpp:314-348), counted per block
+		int nsplit = 0, ntn = 0, ntile = 0;
+		for (int64_t ni = cb + tid; ni < ce; ni += LTPB) {
+			const int2 pr = *reinterpret_cast<const int2*>(&a.nodes[ni].pbeg);
+			const int nparts = pr.y - pr.x;
+			const double* gb = a.gbox + 6 * ni;
+			float box_r = 0.0f;
+			for (int dim = 0; dim < 3; dim++) {
+				const double h = 0.5 * (gb[3 + dim] - gb[dim]);
+				box_r += h * h;
+			}
+			box_r = sqrtf(box_r);
+			const bool ewald_satisfied = (box_r < 0.25 * (a.theta / (1.0 + a.theta)) && box_r < 0.125 - 0.25 * a.hsoft);
+			bool split = nparts > a.bucket || (!ewald_satisfied && nparts > 0);
+			if (split && level >= MAX_DEPTH - 1) {
+				atomicOr(a.flags + 2, 1);
+				split = false;
+			}
+			const bool tiles = split && nparts > WARP_NODE;
+			a.nodes[ni].flags = split ? (tiles ? NODE_SPLIT | NODE_TILES : NODE_SPLIT) : 1;
+			nsplit += split;
+			ntn += tiles;
+			ntile += tiles ? (nparts + TILE - 1) / TILE : 0;
+		}
+		for (int o = 16; o; o >>= 1) {
+			nsplit += __shfl_xor_sync(0xffffffffu, nsplit, o);
+			ntn += __shfl_xor_sync(0xffffffffu, ntn, o);
+			ntile += __shfl_xor_sync(0xffffffffu, ntile, o);
+		}
+		if (lane == 0) {
+			s_scan[0][w] = nsplit;
+			s_scan[1][w] = ntn;
+			s_scan[2][w] = ntile;
+		}
+		__syncthreads();
+		if (tid == 0) {
+			int4 t = make_int4(0, 0, 0, 0);
+			for (int i = 0; i < LWARPS; i++) {
+				t.x += s_scan[0][i];
+				t.y += s_scan[1][i];
+				t.z += s_scan[2][i];
+			}
+			a.blk[blockIdx.x] = t;
+		}
+		if (!grid_meet(ctl, round)) {
+			return;
+		}
+		// ---- totals of the level and of the blocks before this one (a warp: at most a few hundred)
+		int base[3] = { 0, 0, 0 }, tot[3] = { 0, 0, 0 };
+		for (int i = lane; i < (int) gridDim.x; i += 32) {
+			const int4 t = __ldcg(a.blk + i);
+			const bool prev = i < (int) blockIdx.x;
+			tot[0] += t.x;
+			tot[1] += t.y;
+			tot[2] += t.z;
+			base[0] += prev ? t.x : 0;
+			base[1] += prev ? t.y : 0;
+			base[2] += prev ? t.z : 0;
+		}
+		for (int o = 16; o; o >>= 1) {
+			for (int q = 0; q < 3; q++) {
+				tot[q] += __shfl_xor_sync(0xffffffffu, tot[q], o);
+				base[q] += __shfl_xor_sync(0xffffffffu, base[q], o);
+			}
+		}
+		const int64_t next_le = le + 2 * (int64_t) tot[0];
+		if (next_le > a.node_cap) {
+			// every block sees the same totals: all stop here, before the level changes anything
+			if (blockIdx.x == 0 && tid == 0) {
+				ctl->status = 1;
+				ctl->level = level;
+				ctl->lb = lb;
+				ctl->le = le;
+				ctl->need = next_le;
+			}
+			return;
+		}
+		if (blockIdx.x == 0 && tid == 0) {
+			ctl->start[level] = lb;
+			ctl->start[level + 1] = le;
+			ctl->level = level;
+		}
+		// ---- children's indices in node order, tile nodes listed
+		for (int64_t n0 = cb; n0 < ce; n0 += LTPB) {
+			const int64_t ni = n0 + tid;
+			const int f = ni < ce ? a.nodes[ni].flags : 1;
+			const int sp = (f & NODE_SPLIT) != 0, tn = (f & NODE_TILES) != 0;
+			int nt = 0;
+			if (tn) {
+				const int2 pr = *reinterpret_cast<const int2*>(&a.nodes[ni].pbeg);
+				nt = (pr.y - pr.x + TILE - 1) / TILE;
+			}
+			int inc = nt;
+			for (int o = 1; o < 32; o <<= 1) {
+				const int t = __shfl_up_sync(0xffffffffu, inc, o);
+				inc += lane >= o ? t : 0;
+			}
+			const unsigned ms = __ballot_sync(0xffffffffu, sp), mt = __ballot_sync(0xffffffffu, tn);
+			__syncthreads();
+			if (lane == 31) {
+				s_scan[0][w] = __popc(ms);
+				s_scan[1][w] = __popc(mt);
+				s_scan[2][w] = inc;
+			}
+			__syncthreads();
+			int e0 = base[0], e1 = base[1], e2 = base[2];
+			for (int i = 0; i < LWARPS; i++) {
+				const int q0 = s_scan[0][i], q1 = s_scan[1][i], q2 = s_scan[2][i];
+				e0 += i < w ? q0 : 0;
+				e1 += i < w ? q1 : 0;
+				e2 += i < w ? q2 : 0;
+				base[0] += q0;
+				base[1] += q1;
+				base[2] += q2;
+			}
+			if (sp) {
+				a.nodes[ni].child = (int32_t) (le + 2 * (int64_t) (e0 + __popc(ms & lt_lane)));
+				a.nodes[ni].flags = 0;
+			}
+			if (tn) {
+				TileNode t;
+				t.node = (int32_t) ni;
+				t.t0 = e2 + inc - nt;
+				t.nt = nt;
+				t.m = t.nswap = 0;
+				a.tnode[e1 + __popc(mt & lt_lane)] = t;
+				for (int q = 0; q < nt; q++) {
+					a.tile_of[t.t0 + q] = e1 + __popc(mt & lt_lane);
+				}
+			}
+		}
+		// ---- nodes of at most WARP_NODE particles: a warp each, taken from the block's share
+		if (tid == 0) {
+			s_next = 0;
+		}
+		__syncthreads();
+		for (;;) {
+			int k = 0;
+			if (lane == 0) {
+				k = atomicAdd(&s_next, 1);
+			}
+			const int64_t ni = cb + __shfl_sync(0xffffffffu, k, 0);
+			if (ni >= ce) {
+				break;
+			}
+			const NodeW nd = a.nodes[ni];
+			if (nd.child < 0 || nd.pend - nd.pbeg > WARP_NODE) {
+				continue;
+			}
+			double xm;
+			const int xd = split_dim(a.gbox + 6 * ni, xm);
+			const int m = warp_partition(a, nd, xd == 0 ? a.x[0] : xd == 1 ? a.x[1] : a.x[2], fixed_from_double(xm), s_pos[w], lane);
+			make_children(a, ni, nd, nd.pbeg + m, xd, xm, level, lane);
+		}
+		if (tot[2] > 0) {
+			if (!grid_meet(ctl, round)) {
+				return;
+			}
+			// ---- larger nodes, tile by tile: particles below the midpoint
+			for (int t = blockIdx.x; t < tot[2]; t += gridDim.x) {
+				const TileNode tn = a.tnode[a.tile_of[t]];
+				const int2 pr = *reinterpret_cast<const int2*>(&a.nodes[tn.node].pbeg);
+				double xm;
+				const int xd = split_dim(a.gbox + 6 * (int64_t) tn.node, xm);
+				const uint32_t* x = xd == 0 ? a.x[0] : xd == 1 ? a.x[1] : a.x[2];
+				const uint32_t xf = fixed_from_double(xm);
+				const int p0 = pr.x + (t - tn.t0) * TILE + tid;
+				int c = 0;
+#pragma unroll
+				for (int j = 0; j < TILE_ROWS; j++) {
+					const int p = p0 + j * LTPB;
+					c += p < pr.y && x[min(p, pr.y - 1)] < xf;
+				}
+				c = __reduce_add_sync(0xffffffffu, c);
+				if (lane == 0) {
+					s_sum[0][w] = c;
+				}
+				__syncthreads();
+				if (tid == 0) {
+					int s = 0;
+					for (int i = 0; i < LWARPS; i++) {
+						s += s_sum[0][i];
+					}
+					a.tile_lt[t] = s;
+				}
+				__syncthreads();
+			}
+			if (!grid_meet(ctl, round)) {
+				return;
+			}
+			// positions of the particles on the wrong side of the split point: before it ranked from the
+			// node's left, after it from the node's right.  Earlier tiles hold only particles before a
+			// particle on the left, later ones only particles after one on the right, so the counts
+			// below the midpoint of whole tiles give both ranks.
+			for (int t = blockIdx.x; t < tot[2]; t += gridDim.x) {
+				const int ti = a.tile_of[t];
+				const TileNode tn = a.tnode[ti];
+				const int2 pr = *reinterpret_cast<const int2*>(&a.nodes[tn.node].pbeg);
+				double xm;
+				const int xd = split_dim(a.gbox + 6 * (int64_t) tn.node, xm);
+				const uint32_t* x = xd == 0 ? a.x[0] : xd == 1 ? a.x[1] : a.x[2];
+				const uint32_t xf = fixed_from_double(xm);
+				const int tb = pr.x + (t - tn.t0) * TILE, te = min(tb + TILE, pr.y);
+				unsigned below = 0;  // bit j: row j's particle of this thread
+#pragma unroll
+				for (int j = 0; j < TILE_ROWS; j++) {
+					const int p = tb + j * LTPB + tid;
+					below |= (unsigned) (p < te && x[min(p, te - 1)] < xf) << j;
+				}
+				int all = 0, prev = 0;
+				for (int q = tid; q < tn.nt; q += LTPB) {
+					const int c = __ldcg(a.tile_lt + tn.t0 + q);
+					all += c;
+					prev += q < t - tn.t0 ? c : 0;
+				}
+				all = __reduce_add_sync(0xffffffffu, all);
+				prev = __reduce_add_sync(0xffffffffu, prev);
+				if (lane == 0) {
+					s_sum[0][w] = all;
+					s_sum[1][w] = prev;
+				}
+				__syncthreads();
+				int m = 0, lt_prev = 0;
+				for (int i = 0; i < LWARPS; i++) {
+					m += s_sum[0][i];
+					lt_prev += s_sum[1][i];
+				}
+				const int sp = pr.x + m;
+				unsigned wrong = 0;
+				int right = 0;  // wrong ones after the split point
+#pragma unroll
+				for (int j = 0; j < TILE_ROWS; j++) {
+					const int p = tb + j * LTPB + tid;
+					const bool lt = below >> j & 1u;
+					const bool bad = p < te && (p < sp ? !lt : lt);
+					const unsigned mk = __ballot_sync(0xffffffffu, bad);
+					wrong |= (unsigned) bad << j;
+					right += bad && p >= sp;
+					if (lane == 0) {
+						s_cnt[j * LWARPS + w] = __popc(mk);
+					}
+				}
+				__syncthreads();
+				// prefix of the rows' warps in particle order, by every warp for itself
+				int mybase[TILE_ROWS], run = 0;
+				{
+					constexpr int PER = TILE_ROWS * LWARPS / 32;
+					int c[PER], s = 0;
+					for (int i = 0; i < PER; i++) {
+						c[i] = s_cnt[lane * PER + i];
+						s += c[i];
+					}
+					int inc = s;
+					for (int o = 1; o < 32; o <<= 1) {
+						const int v = __shfl_up_sync(0xffffffffu, inc, o);
+						inc += lane >= o ? v : 0;
+					}
+					run = __shfl_sync(0xffffffffu, inc, 31);
+					int ex[PER];
+					int e = inc - s;
+					for (int i = 0; i < PER; i++) {
+						ex[i] = e;
+						e += c[i];
+					}
+#pragma unroll
+					for (int j = 0; j < TILE_ROWS; j++) {
+						const int q = j * LWARPS + w;
+						int v = 0;
+						for (int i = 0; i < PER; i++) {
+							const int u = __shfl_sync(0xffffffffu, ex[i], q / PER);
+							v = q % PER == i ? u : v;
+						}
+						mybase[j] = v;
+					}
+				}
+				right = __reduce_add_sync(0xffffffffu, right);
+				__syncthreads();
+				if (lane == 0) {
+					s_sum[0][w] = right;
+				}
+				__syncthreads();
+				int nright = 0;
+				for (int i = 0; i < LWARPS; i++) {
+					nright += s_sum[0][i];
+				}
+				const int lt_tile = __ldcg(a.tile_lt + t);
+				const int after = m - lt_prev - lt_tile;  // below the midpoint in later tiles
+				const int leftbase = (tb - pr.x) - lt_prev;
+#pragma unroll
+				for (int j = 0; j < TILE_ROWS; j++) {
+					const bool bad = wrong >> j & 1u;
+					const unsigned mk = __ballot_sync(0xffffffffu, bad);
+					if (bad) {
+						const int p = tb + j * LTPB + tid;
+						const int e = mybase[j] + __popc(mk & lt_lane);
+						if (p < sp) {
+							a.posL[pr.x + leftbase + e] = p;
+						} else {
+							a.posR[pr.x + after + (run - e - 1)] = p;
+						}
+					}
+				}
+				if (tid == 0) {
+					if (t == tn.t0) {
+						a.tnode[ti].m = m;
+					}
+					// the tile that holds the split point (or the last one, when nothing lies after it)
+					if ((tb <= sp && sp < te) || (sp == pr.y && te == pr.y)) {
+						a.tnode[ti].nswap = after + nright;
+					}
+				}
+				__syncthreads();
+			}
+			if (!grid_meet(ctl, round)) {
+				return;
+			}
+			for (int t = blockIdx.x; t < tot[2]; t += gridDim.x) {
+				const TileNode* tp = a.tnode + a.tile_of[t];
+				const int node = tp->node, t0 = tp->t0;
+				const int m = __ldcg(&tp->m), ns = __ldcg(&tp->nswap);
+				const int pbeg = a.nodes[node].pbeg;
+				for (int k = (t - t0) * TILE + tid; k < min(ns, (t - t0 + 1) * TILE); k += LTPB) {
+					swap_particles(a, __ldcg(a.posL + pbeg + k), __ldcg(a.posR + pbeg + k));
+				}
+				if (t == t0 && w == 0) {
+					double xm;
+					const int xd = split_dim(a.gbox + 6 * (int64_t) node, xm);
+					make_children(a, node, a.nodes[node], pbeg + m, xd, xm, level, lane);
+				}
+			}
+		}
+		if (tot[0] == 0) {
+			break;
+		}
+		lb = le;
+		le = next_le;
+		if (!grid_meet(ctl, round)) {
+			return;
+		}
+	}
+	if (blockIdx.x == 0 && tid == 0) {
+		ctl->status = 0;
 	}
 }
 
@@ -745,82 +939,63 @@ ct_status tree_build_t(Ctx* c, Box* b, const ct_tree_params* p) {
 	// upper estimate; start smaller and grow per level as needed.
 	CT_TRY(ensure_nodes(c, b, std::max<int64_t>(4 * np / std::max(p->bucket, 1) + 4096, 8192)));
 	ct_status s1 = CT_OK;
-	BuildScratch s;
-	const int64_t npad = std::max<int64_t>(np, 1);
-	s.idx = (int32_t*) scratch(c, 0, sizeof(int32_t) * n, &s1);
-	s.posL = (int32_t*) scratch(c, 1, sizeof(int32_t) * n, &s1);
-	s.posR = (int32_t*) scratch(c, 2, sizeof(int32_t) * n, &s1);
-	CT_TRY(s1);
-	(void) npad;
-	c->launches++;
-	k_iota<<<grid_for(c, n, 256), 256, 0, st>>>(s.idx, n);
-	c->launches++;
 	const int nroot = b->nsub;
 	CT_TRY(ensure_nodes(c, b, nroot + 1));
-	k_init_roots<<<(nroot + 127) / 128, 128, 0, st>>>(nroot, b->d_sub_off, b->nodes, b->gbox, b->key, b->depth, b->parent, (int32_t) pb, (int32_t) n);
-	CT_CUDA(c, cudaMemsetAsync(c->d_flags, 0, 4 * sizeof(int), st));
-	std::vector<int64_t> levels;
-	levels.push_back(0);
-	int64_t lb = 0, le = nroot;
-	int32_t* h_tot = (int32_t*) c->pinned;
-	while (le > lb) {
-		levels.push_back(le);
-		const int nl = (int) (le - lb);
-		// per-level scratch (node- and tile-sized arrays)
-		const int64_t max_tiles = (np + TILE - 1) / TILE + nl + 1;
-		s.split = (int32_t*) scratch(c, 3, sizeof(int32_t) * (nl + 1), &s1);
-		s.rank = (int32_t*) scratch(c, 4, sizeof(int32_t) * (nl + 1), &s1);
-		s.ntiles = (int32_t*) scratch(c, 5, sizeof(int32_t) * (nl + 1), &s1);
-		s.tile_off = (int32_t*) scratch(c, 6, sizeof(int32_t) * (nl + 1), &s1);
-		s.xdim = (int32_t*) scratch(c, 7, sizeof(int32_t) * nl, &s1);
-		s.xmidf = (uint32_t*) scratch(c, 8, sizeof(uint32_t) * nl, &s1);
-		s.xmid = (double*) scratch(c, 9, sizeof(double) * nl, &s1);
-		s.node_m = (int32_t*) scratch(c, 10, sizeof(int32_t) * nl, &s1);
-		s.node_nmis = (int32_t*) scratch(c, 11, sizeof(int32_t) * nl, &s1);
-		s.tile_node = (int32_t*) scratch(c, 12, sizeof(int32_t) * max_tiles, &s1);
-		s.tile_lt = (int32_t*) scratch(c, 13, sizeof(int32_t) * max_tiles, &s1);
-		s.tile_offL = (int32_t*) scratch(c, 14, sizeof(int32_t) * max_tiles, &s1);
-		s.tile_offR = (int32_t*) scratch(c, 15, sizeof(int32_t) * max_tiles, &s1);
-		s.totals = c->d_flags + 8;
-		CT_TRY(s1);
-		size_t need = 0;
-		cub::DeviceScan::ExclusiveSum(nullptr, need, s.split, s.rank, nl + 1, st);
-		s.cub_bytes = need;
-		s.cub_tmp = scratch(c, 16, need + 256, &s1);
-		CT_TRY(s1);
-		c->launches++;
-		k_classify<<<grid_for(c, nl, 256), 256, 0, st>>>(lb, nl, b->nodes, b->gbox, b->depth, p->theta, p->hsoft, p->bucket, s, c->d_flags);
-		CT_CUDA(c, cudaMemsetAsync(s.split + nl, 0, sizeof(int32_t), st));
-		CT_CUDA(c, cudaMemsetAsync(s.ntiles + nl, 0, sizeof(int32_t), st));
-		CT_CUDA(c, cub::DeviceScan::ExclusiveSum(s.cub_tmp, need, s.split, s.rank, nl + 1, st));
-		CT_CUDA(c, cub::DeviceScan::ExclusiveSum(s.cub_tmp, need, s.ntiles, s.tile_off, nl + 1, st));
-		CT_CUDA(c, cudaMemcpyAsync(h_tot, s.rank + nl, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-		CT_CUDA(c, cudaMemcpyAsync(h_tot + 1, s.tile_off + nl, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-		CT_CUDA(c, cudaStreamSynchronize(st));
-		const int nsplit = h_tot[0];
-		const int ntile = h_tot[1];
-		if (nsplit > 0) {
-			CT_TRY(ensure_nodes(c, b, le + 2 * (int64_t) nsplit));
-			c->launches++;
-			k_tile_map<<<grid_for(c, (int64_t) nl * 32, 256), 256, 0, st>>>(nl, s);
-			const int gt = std::min(ntile, c->nsm * 16);
-			c->launches++;
-			k_count<<<gt, TPB, 0, st>>>(lb, ntile, b->nodes, b->x[0], b->x[1], b->x[2], s);
-			c->launches++;
-			k_node_scan<<<std::min(nl, c->nsm * 16), TPB, 0, st>>>(lb, nl, b->nodes, b->x[0], b->x[1], b->x[2], s);
-			c->launches++;
-			k_positions<<<gt, TPB, 0, st>>>(lb, ntile, b->nodes, b->x[0], b->x[1], b->x[2], s);
-			c->launches++;
-			k_swap<<<gt, TPB, 0, st>>>(lb, ntile, b->nodes, b->x[0], b->x[1], b->x[2], s);
-		}
-		c->launches++;
-		k_children<<<grid_for(c, nl, 256), 256, 0, st>>>(lb, nl, le, b->nodes, b->gbox, b->key, b->depth, b->parent, s);
-		CT_CUDA(c, cudaGetLastError());
-		lb = le;
-		le = le + 2 * (int64_t) nsplit;
+	// one block an SM (two boxes built by two contexts fit side by side), fewer for a few particles
+	const int nblk = (int) std::max<int64_t>(1, std::min<int64_t>(c->nsm, std::max<int64_t>(np / 64, nroot)));
+	LevelArgs la;
+	la.idx = (int32_t*) scratch(c, 0, sizeof(int32_t) * n, &s1);
+	la.posL = (int32_t*) scratch(c, 1, sizeof(int32_t) * n, &s1);
+	la.posR = (int32_t*) scratch(c, 2, sizeof(int32_t) * n, &s1);
+	// nodes in tiles hold more than WARP_NODE particles each
+	const int64_t max_tn = np / WARP_NODE + 1, max_tiles = np / TILE + max_tn + 1;
+	la.tnode = (TileNode*) scratch(c, 3, sizeof(TileNode) * max_tn, &s1);
+	la.tile_of = (int32_t*) scratch(c, 4, sizeof(int32_t) * max_tiles, &s1);
+	la.tile_lt = (int32_t*) scratch(c, 5, sizeof(int32_t) * max_tiles, &s1);
+	la.blk = (int4*) scratch(c, 6, sizeof(int4) * c->nsm, &s1);
+	la.ctl = (LevelCtl*) scratch(c, 7, sizeof(LevelCtl), &s1);
+	CT_TRY(s1);
+	for (int d = 0; d < 3; d++) {
+		la.x[d] = b->x[d];
 	}
+	la.flags = c->d_flags;
+	la.off = b->d_sub_off;
+	la.pb = pb;
+	la.n = n;
+	la.nroot = nroot;
+	la.bucket = p->bucket;
+	la.theta = p->theta;
+	la.hsoft = p->hsoft;
+	CT_CUDA(c, cudaMemsetAsync(c->d_flags, 0, 4 * sizeof(int), st));
+	int32_t* h_tot = (int32_t*) c->pinned;
+	LevelCtl* hc = (LevelCtl*) ((char*) c->pinned + 64);
+	for (la.resume = 0;; la.resume = 1) {
+		la.nodes = b->nodes;
+		la.gbox = b->gbox;
+		la.key = b->key;
+		la.depth = b->depth;
+		la.parent = b->parent;
+		la.node_cap = b->node_cap;
+		// (a resumed build keeps the level it stopped before)
+		CT_CUDA(c, cudaMemsetAsync(la.ctl, 0, offsetof(LevelCtl, level), st));
+		c->launches++;
+		void* args[] = { (void*) &la };
+		CT_CUDA(c, cudaLaunchCooperativeKernel((const void*) k_tree_levels, dim3(nblk), dim3(LTPB), args, 0, st));
+		CT_CUDA(c, cudaMemcpyAsync(hc, la.ctl, sizeof(LevelCtl), cudaMemcpyDeviceToHost, st));
+		CT_CUDA(c, cudaStreamSynchronize(st));
+		if (hc->error) {
+			return fail(c, CT_ERR_CUDA, "tree build: the blocks of the cooperative grid did not meet");
+		}
+		if (hc->status == 0) {
+			break;
+		}
+		// the levels so far stay; the level that did not fit starts again with room for its children
+		CT_TRY(ensure_nodes(c, b, hc->need));
+	}
+	std::vector<int64_t> levels(hc->start, hc->start + hc->level + 2);
 	b->level_start = levels;  // level k = [levels[k], levels[k+1])
-	b->nnodes = le;
+	b->nnodes = levels.back();
+	const int32_t* perm = la.idx;
 	// apply the permutation to velocities and rungs
 	{
 		ct_status s2 = CT_OK;
@@ -835,7 +1010,7 @@ ct_status tree_build_t(Ctx* c, Box* b, const ct_tree_params* p) {
 		CT_CUDA(c, cudaMemcpyAsync(tr + pb, b->rung + pb, np, cudaMemcpyDeviceToDevice, st));
 		if (np > 0) {
 			c->launches++;
-			k_gather_particles<<<grid_for(c, np, 256), 256, 0, st>>>(pb, n, s.idx, t0, t1, t2, tr, b->v[0], b->v[1], b->v[2], b->rung);
+			k_gather_particles<<<grid_for(c, np, 256), 256, 0, st>>>(pb, n, perm, t0, t1, t2, tr, b->v[0], b->v[1], b->v[2], b->rung);
 		}
 	}
 	// upsweep, deepest level first
