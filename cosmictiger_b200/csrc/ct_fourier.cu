@@ -141,18 +141,41 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
 	return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
-__device__ __forceinline__ float2 filtered(float2 v, float kx, float ky, float kz, float box_size, int N) {
-	const float fx = (float) cloud_filter(kx * box_size / N);
-	const float fy = (float) cloud_filter(ky * box_size / N);
-	const float fz = (float) cloud_filter(kz * box_size / N);
-	v = make_float2(v.x * fx, v.y * fx);
-	v = make_float2(v.x * fy, v.y * fy);
-	return make_float2(v.x * fz, v.y * fz);
-}
-
 __device__ __forceinline__ float wavenumber(int I, int N, float box_size) {
 	const int i = I < N / 2 ? I : I - N;
 	return 2.f * (float) M_PI / box_size * float(i);
+}
+
+// Per-axis values of one call, by grid index: the inverse window at the axis' wavenumber and the
+// lattice point's stencil (first cell and six weights).  Evaluated once an axis; every mode and
+// every point used to evaluate its own in double, which bounded the field and interpolation passes
+// (256^3: 161 us a field against 25 us of memory traffic, 1,260 us an interpolation against 70).
+struct AxisTables {
+	float* filter;  // [N]
+	int* cell;      // [N]
+	double* weight; // [6][N]
+};
+
+__global__ void k_ic_axis(int N, float box_size, AxisTables t) {
+	const int I = blockIdx.x * blockDim.x + threadIdx.x;
+	if (I >= N) {
+		return;
+	}
+	t.filter[I] = (float) cloud_filter(wavenumber(I, N, box_size) * box_size / N);
+	const double x0 = fixed_to_double(fixed_from_double(I * (1.0 / N)));
+	const int i1 = (int) (x0 * N);
+	const double f = x0 * N - i1;
+	t.cell[I] = i1;
+	for (int j = 0; j < 6; j++) {
+		t.weight[j * N + I] = cloud_weight((float) (-(j + CLOUD_MIN) + f));
+	}
+}
+
+// Grid of one (x, y) row of modes or points a block row: blockIdx.y = I1, blockIdx.z = I0.
+__device__ __forceinline__ float2 filtered(float2 v, float fx, float fy, float fz) {
+	v = make_float2(v.x * fx, v.y * fx);
+	v = make_float2(v.x * fy, v.y * fy);
+	return make_float2(v.x * fz, v.y * fz);
 }
 
 // The uniforms (x, y) of every mode, as floats, row by row (the generators are sequential).
@@ -215,16 +238,19 @@ __global__ void __launch_bounds__(FT_TPB) k_ic_amplitude(int N, float box_size, 
 
 // One field: Y = A (-i k_dim1)(-i k_dim2) / k^2, conjugated (times the parity sign) on the lower
 // half of the kz = 0 plane, times the inverse window.
-__global__ void __launch_bounds__(FT_TPB) k_ic_field(int N, float box_size, int dim1, int dim2, const float2* __restrict__ A, cufftComplex* __restrict__ Y) {
+__global__ void __launch_bounds__(FT_TPB) k_ic_field(int N, float box_size, int dim1, int dim2, const float* __restrict__ filter, const float2* __restrict__ A,
+		cufftComplex* __restrict__ Y) {
 	const int NZ = N / 2 + 1;
-	const int64_t total = (int64_t) N * N * NZ;
 	float sgn = 1.f;
 	sgn *= dim1 != 3 ? -1.f : 1.f;
 	sgn *= dim2 != 3 ? -1.f : 1.f;
-	for (int64_t e = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; e < total; e += (int64_t) gridDim.x * blockDim.x) {
-		const int I2 = (int) (e % NZ);
-		const int64_t row = e / NZ;
-		const int I0 = (int) (row / N), I1 = (int) (row % N);
+	const int64_t stride = (int64_t) gridDim.x * blockDim.x, total = (int64_t) N * N * NZ;
+	// the mode's indices advance with e: no division inside the loop
+	const int64_t e0 = blockIdx.x * (int64_t) blockDim.x + threadIdx.x;
+	int I2 = (int) (e0 % NZ), row = (int) (e0 / NZ);
+	const int d2 = (int) (stride % NZ), drow = (int) (stride / NZ);
+	for (int64_t e = e0; e < total; e += stride) {
+		const int I0 = (unsigned) row / (unsigned) N, I1 = row - I0 * N;
 		const float kx = wavenumber(I0, N, box_size), ky = wavenumber(I1, N, box_size), kz = wavenumber(I2, N, box_size);
 		float2 v = make_float2(0.f, 0.f);
 		if (I2 > 0 || I0 != 0 || I1 != 0) {
@@ -237,21 +263,28 @@ __global__ void __launch_bounds__(FT_TPB) k_ic_field(int N, float box_size, int 
 				v = make_float2(v.x * sgn, -v.y * sgn);
 			}
 		}
-		v = filtered(v, kx, ky, kz, box_size, N);
+		v = filtered(v, __ldg(filter + I0), __ldg(filter + I1), __ldg(filter + I2));
 		Y[e] = make_cuComplex(v.x, v.y);
+		I2 += d2;
+		row += drow;
+		if (I2 >= NZ) {
+			I2 -= NZ;
+			row++;
+		}
 	}
 }
 
 // Second-order displacement field of axis dim from the transformed 2LPT source:
 // Y = -i k_dim delta2(k) / k^2 times the inverse window, 0 at k = 0 (twolpt_correction2,
 // initialize.cpp:384-434).
-__global__ void __launch_bounds__(FT_TPB) k_ic_correction(const cufftComplex* __restrict__ src, cufftComplex* __restrict__ Y, int N, float box_size, int dim) {
+__global__ void __launch_bounds__(FT_TPB) k_ic_correction(const cufftComplex* __restrict__ src, cufftComplex* __restrict__ Y, int N, float box_size, int dim,
+		const float* __restrict__ filter) {
 	const int NZ = N / 2 + 1;
 	const int64_t total = (int64_t) N * N * NZ;
 	for (int64_t e = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; e < total; e += (int64_t) gridDim.x * blockDim.x) {
-		const int I2 = (int) (e % NZ);
-		const int64_t row = e / NZ;
-		const int I0 = (int) (row / N), I1 = (int) (row % N);
+		const unsigned row = (unsigned) (e / NZ);  // (at most 2^20 rows)
+		const int I2 = (int) (e - (int64_t) row * NZ);
+		const int I0 = (int) (row / (unsigned) N), I1 = (int) (row - (unsigned) I0 * (unsigned) N);
 		const int i = I0 < N / 2 ? I0 : I0 - N;
 		const int j = I1 < N / 2 ? I1 : I1 - N;
 		const int k = I2 < N / 2 ? I2 : I2 - N;
@@ -266,7 +299,7 @@ __global__ void __launch_bounds__(FT_TPB) k_ic_correction(const cufftComplex* __
 			// -i K y / k^2
 			v = make_float2(K[dim] * s.y, -K[dim] * s.x);
 			v = make_float2(v.x / k2, v.y / k2);
-			v = filtered(v, kx, ky, kz, box_size, N);
+			v = filtered(v, __ldg(filter + I0), __ldg(filter + I1), __ldg(filter + I2));
 		}
 		Y[e] = make_cuComplex(v.x, v.y);
 	}
@@ -295,67 +328,89 @@ __global__ void __launch_bounds__(FT_TPB) k_ic_lattice(int N, uint32_t* __restri
 // with the cloud kernel at each particle's lattice point, dx = -D field / box; the position
 // moves by dx (periodic) and the velocity by prefac dx.  Particle (I0 N + I1) N + I2 sits at
 // lattice point I, and the kernel's 6^3 weights there are products of per-axis weights that
-// depend only on I0, I1, I2, so the 216-term sum is taken as three 6-term passes over the grid
-// (double precision, as the reference accumulates): x and y into double grids, z fused with
-// the update.  The largest dx in units of the mean spacing goes to dxmax (float bits: a
-// positive float orders like its bits).
-__device__ __forceinline__ void lattice_stencil(int I, int N, int& i1, double w[6]) {
-	const double x0 = fixed_to_double(fixed_from_double(I * (1.0 / N)));
-	i1 = (int) (x0 * N);
-	const double t = x0 * N - i1;
+// depend only on I0, I1, I2, so the 216-term sum is taken as 6-term sums along x, y and z (double
+// precision, as the reference accumulates).  One block takes DISP_ROWS rows (x, y .. y + 7) of one
+// x: the x sums of the rows it needs (8 and their y neighbours) into shared memory, then per row the
+// y sums and, from those, the z sums and the update.  As three passes over double grids the same
+// sums moved 36 bytes a point through memory; here a point is read from the field (which the L2
+// keeps) and updated.  256^3: 1,260 us an axis with weights evaluated per point, now 90.
+// The largest dx in units of the mean spacing goes to dxmax (float bits: a positive float orders
+// like its bits).
+constexpr int DISP_ROWS = 8;
+
+// An index at most one grid length outside 0 .. n - 1.
+__device__ __forceinline__ int wrap1(int i, int n) {
+	return i < 0 ? i + n : (i >= n ? i - n : i);
+}
+
+__global__ void __launch_bounds__(FT_TPB) k_ic_displace(int N, const float* __restrict__ R, AxisTables t, double scale, float D, float prefac,
+		double box_size_inv, uint32_t* __restrict__ X, float* __restrict__ V, unsigned int* dxmax) {
+	extern __shared__ double s_rows[];  // [rows][N] sums along x, then [N] sums along x and y
+	const int I0 = blockIdx.y, y0 = blockIdx.x * DISP_ROWS;
+	const int ny = min(DISP_ROWS, N - y0);
+	// rows y0's first neighbour .. the last row's last, wrapped (a lattice point's cell never falls
+	// by more than one below its index, and rises with it)
+	const int r0 = __ldg(t.cell + y0) + CLOUD_MIN;
+	const int nrow = __ldg(t.cell + y0 + ny - 1) + CLOUD_MAX - r0 + 1;  // at most DISP_ROWS + 6
+	double* s_y = s_rows + (size_t) (DISP_ROWS + 6) * N;
+	const int c0 = __ldg(t.cell + I0) + CLOUD_MIN;
+	int64_t plane[6];
+	double wx[6];
 #pragma unroll
 	for (int j = 0; j < 6; j++) {
-		w[j] = cloud_weight((float) (-(j + CLOUD_MIN) + t));
+		plane[j] = (int64_t) wrap1(c0 + j, N) * N * N;
+		wx[j] = __ldg(t.weight + j * N + I0);
 	}
-}
-
-// One pass along axis 0 (stride N^2) or 1 (stride N).
-template<class Tin>
-__global__ void __launch_bounds__(FT_TPB) k_ic_smooth(int N, int axis, const Tin* __restrict__ in, double* __restrict__ out) {
-	const int64_t n = (int64_t) N * N * N;
-	const int64_t stride = axis == 0 ? (int64_t) N * N : N;
-	for (int64_t e = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; e < n; e += (int64_t) gridDim.x * blockDim.x) {
-		const int I = axis == 0 ? (int) (e / ((int64_t) N * N)) : (int) ((e / N) % N);
-		int i1;
-		double w[6];
-		lattice_stencil(I, N, i1, w);
-		const int64_t base = e - (int64_t) I * stride;
-		double acc = 0.0;
+	for (int r = 0; r < nrow; r++) {
+		const float* p = R + (int64_t) wrap1(r0 + r, N) * N;
+		for (int z = threadIdx.x; z < N; z += FT_TPB) {
+			double acc = 0.0;
 #pragma unroll
-		for (int j = 0; j < 6; j++) {
-			acc += w[j] * (double) in[base + (int64_t) wrap(i1 + j + CLOUD_MIN, N) * stride];
+			for (int j = 0; j < 6; j++) {
+				acc += wx[j] * (double) p[plane[j] + z];
+			}
+			s_rows[(size_t) r * N + z] = acc;
 		}
-		out[e] = acc;
 	}
-}
-
-// The pass along z, scaled by the inverse transform's normalisation, and the update.
-__global__ void __launch_bounds__(FT_TPB) k_ic_displace(int N, const double* __restrict__ B, double scale, int dim, float D, float prefac,
-		double box_size_inv, uint32_t* __restrict__ X, float* __restrict__ V, unsigned int* dxmax) {
-	const int64_t n = (int64_t) N * N * N;
+	__syncthreads();
 	float mymax = 0.f;
-	for (int64_t p = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; p < n; p += (int64_t) gridDim.x * blockDim.x) {
-		const int I2 = (int) (p % N);
-		int i1;
-		double w[6];
-		lattice_stencil(I2, N, i1, w);
-		const int64_t base = p - I2;
-		double dx = 0.0;
+	for (int y = 0; y < ny; y++) {
+		const int first = __ldg(t.cell + y0 + y) + CLOUD_MIN - r0;
+		double wy[6];
 #pragma unroll
 		for (int j = 0; j < 6; j++) {
-			dx += w[j] * B[base + wrap(i1 + j + CLOUD_MIN, N)];
+			wy[j] = __ldg(t.weight + j * N + y0 + y);
 		}
-		dx *= scale;
-		dx *= -D * box_size_inv;
-		double x = fixed_to_double(X[p]) + dx;
-		if (x >= 1.0) {
-			x -= 1.0;
-		} else if (x < 0.0) {
-			x += 1.0;
+		for (int z = threadIdx.x; z < N; z += FT_TPB) {
+			double acc = 0.0;
+#pragma unroll
+			for (int j = 0; j < 6; j++) {
+				acc += wy[j] * s_rows[(size_t) (first + j) * N + z];
+			}
+			s_y[z] = acc;
 		}
-		X[p] = fixed_from_double(x);
-		V[p] += prefac * dx;
-		mymax = fmaxf(mymax, (float) (dx * N));
+		__syncthreads();
+		const int64_t base = ((int64_t) I0 * N + y0 + y) * N;
+		for (int z = threadIdx.x; z < N; z += FT_TPB) {
+			const int c = __ldg(t.cell + z) + CLOUD_MIN;
+			double dx = 0.0;
+#pragma unroll
+			for (int j = 0; j < 6; j++) {
+				dx += __ldg(t.weight + j * N + z) * s_y[wrap1(c + j, N)];
+			}
+			dx *= scale;
+			dx *= -D * box_size_inv;
+			double x = fixed_to_double(X[base + z]) + dx;
+			if (x >= 1.0) {
+				x -= 1.0;
+			} else if (x < 0.0) {
+				x += 1.0;
+			}
+			X[base + z] = fixed_from_double(x);
+			V[base + z] += prefac * dx;
+			mymax = fmaxf(mymax, (float) (dx * N));
+		}
+		__syncthreads();
 	}
 	for (int o = 16; o; o >>= 1) {
 		mymax = fmaxf(mymax, __shfl_xor_sync(0xffffffffu, mymax, o));
@@ -365,22 +420,30 @@ __global__ void __launch_bounds__(FT_TPB) k_ic_displace(int N, const double* __r
 	}
 }
 
-// The 2LPT source (twolpt_phase, initialize.cpp:565-589): phases 0..8 bring the second
-// derivatives (yy, zz, xx, zz, xx, yy, xy, xz, yz); an even phase up to 6 keeps its field, an
-// odd one adds the product with the kept field, and phases 7 and 8 subtract their squares:
-// delta2 = p_yy p_zz + p_xx p_zz + p_xx p_yy - p_xz^2 - p_yz^2 (the reference keeps p_xy at
-// phase 6 without using it, so -p_xy^2 is not part of its source; reproduced as is).
-__global__ void __launch_bounds__(FT_TPB) k_twolpt_phase(int64_t n, int phase, const float* __restrict__ R, float scale, float* __restrict__ part,
-		float* __restrict__ delta2) {
+// The 2LPT source (twolpt_phase, initialize.cpp:565-589).  The reference brings the second
+// derivatives in nine phases (yy, zz, xx, zz, xx, yy, xy, xz, yz): an even phase up to 6 keeps its
+// field, an odd one adds the product with the kept field, and phases 7 and 8 subtract their squares:
+// delta2 = p_yy p_zz + p_xx p_zz + p_xx p_yy - p_xz^2 - p_yz^2 (it keeps p_xy at phase 6 without
+// using it, so -p_xy^2 is not part of its source; reproduced as is).  Here each of the five fields
+// that count is transformed once; the products and squares are added in the same order.
+__global__ void __launch_bounds__(FT_TPB) k_twolpt_products(int64_t n, const float* __restrict__ xx, const float* __restrict__ yy, float* __restrict__ zz,
+		float scale) {
 	for (int64_t p = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; p < n; p += (int64_t) gridDim.x * blockDim.x) {
-		const float r = R[p] * scale;
-		if (phase > 6) {
-			delta2[p] -= r * r;
-		} else if (phase % 2 == 0) {
-			part[p] = r;
-		} else {
-			delta2[p] += part[p] * r;
-		}
+		const float a = xx[p] * scale, b = yy[p] * scale, c = zz[p] * scale;
+		float d = b * c;
+		d += a * c;
+		d += a * b;
+		zz[p] = d;
+	}
+}
+__global__ void __launch_bounds__(FT_TPB) k_twolpt_squares(int64_t n, const float* __restrict__ xz, const float* __restrict__ yz, float* __restrict__ delta2,
+		float scale) {
+	for (int64_t p = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; p < n; p += (int64_t) gridDim.x * blockDim.x) {
+		const float a = xz[p] * scale, b = yz[p] * scale;
+		float d = delta2[p];
+		d -= a * a;
+		d -= b * b;
+		delta2[p] = d;
 	}
 }
 
@@ -671,15 +734,15 @@ extern "C" ct_status ct_initialize(ct_ctx* ctx, int box_id, const ct_ic_params* 
 	float2* A = nullptr;
 	cufftComplex* Y = nullptr;
 	float* R = nullptr;
-	double* G1 = nullptr;
-	double* G2 = nullptr;
+	AxisTables ax = {};
 	unsigned int* dmax = nullptr;
 	CT_TRY(S.alloc(&dP, P.size(), "power table"));
 	CT_TRY(S.alloc(&A, ncx, "mode amplitudes"));
 	CT_TRY(S.alloc(&Y, ncx, "k-space field"));
 	CT_TRY(S.alloc(&R, n, "real-space field"));
-	CT_TRY(S.alloc(&G1, n, "interpolation pass"));
-	CT_TRY(S.alloc(&G2, n, "interpolation pass"));
+	CT_TRY(S.alloc(&ax.filter, N, "axis tables"));
+	CT_TRY(S.alloc(&ax.cell, N, "axis tables"));
+	CT_TRY(S.alloc(&ax.weight, 6 * (size_t) N, "axis tables"));
 	CT_TRY(S.alloc(&dmax, 6, "displacement maxima"));
 	CT_TRY(S.plan(0, N, CUFFT_C2R));
 	CT_CUDA(c, cudaMemcpyAsync(dP, P.data(), sizeof(float) * P.size(), cudaMemcpyHostToDevice, st));
@@ -691,44 +754,48 @@ extern "C" ct_status ct_initialize(ct_ctx* ctx, int box_id, const ct_ic_params* 
 	const float fscale = (float) scale;
 	const double box_inv = 1.0 / box;
 	const int gn = ft_grid(c, n), gx = ft_grid(c, ncx);
-	c->launches += 3;
+	c->launches += 4;
+	k_ic_axis<<<(N + 127) / 128, 128, 0, st>>>(N, box, ax);
 	k_ic_lattice<<<gn, FT_TPB, 0, st>>>(N, b->x[0], b->x[1], b->x[2], b->v[0], b->v[1], b->v[2], b->rung);
 	k_ic_uniforms<<<ft_grid(c, (int64_t) N * N), FT_TPB, 0, st>>>(N, A);
 	k_ic_amplitude<<<gx, FT_TPB, 0, st>>>(N, box, factor, dtab, A);
 	// interpolation at the lattice points and update of axis dim
+	const size_t disp_smem = sizeof(double) * (DISP_ROWS + 7) * N;  // 120 KB at the largest grid
+	CT_CUDA(c, cudaFuncSetAttribute(k_ic_displace, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) disp_smem));
 	auto displace = [&](int dim, float D, float prefac, unsigned int* mx) {
-		c->launches += 3;
-		k_ic_smooth<float><<<gn, FT_TPB, 0, st>>>(N, 0, R, G1);
-		k_ic_smooth<double><<<gn, FT_TPB, 0, st>>>(N, 1, G1, G2);
-		k_ic_displace<<<gn, FT_TPB, 0, st>>>(N, G2, scale, dim, D, prefac, box_inv, b->x[dim], b->v[dim], mx);
+		c->launches++;
+		k_ic_displace<<<dim3((N + DISP_ROWS - 1) / DISP_ROWS, N), FT_TPB, disp_smem, st>>>(N, R, ax, scale, D, prefac, box_inv, b->x[dim], b->v[dim], mx);
+	};
+	// the field of dim1, dim2 in real space
+	auto field = [&](int dim1, int dim2, float* out) {
+		c->launches++;
+		k_ic_field<<<gx, FT_TPB, 0, st>>>(N, box, dim1, dim2, ax.filter, A, Y);
+		return fft_check(c, cufftExecC2R(S.plans[0], Y, out), "cufftExecC2R");
 	};
 	for (int dim = 0; dim < 3; dim++) {
-		c->launches++;
-		k_ic_field<<<gx, FT_TPB, 0, st>>>(N, box, dim, 3, A, Y);
-		CT_TRY(fft_check(c, cufftExecC2R(S.plans[0], Y, R), "cufftExecC2R"));
+		CT_TRY(field(dim, 3, R));
 		displace(dim, D1, prefac1, dmax + dim);
 	}
 	if (p->twolpt) {
-		float* delta2 = nullptr;
-		float* part = nullptr;
+		float* R1 = nullptr;
+		float* R2 = nullptr;
 		cufftComplex* d2k = nullptr;
-		CT_TRY(S.alloc(&delta2, n, "2LPT source"));
-		CT_TRY(S.alloc(&part, n, "2LPT factor"));
+		CT_TRY(S.alloc(&R1, n, "2LPT field"));
+		CT_TRY(S.alloc(&R2, n, "2LPT field"));
 		CT_TRY(S.alloc(&d2k, ncx, "2LPT source transform"));
 		CT_TRY(S.plan(1, N, CUFFT_R2C));
-		c->launches++;
-		k_fill<<<gn, FT_TPB, 0, st>>>(n, delta2, 0.f);
-		const int pairs[9][2] = { { 1, 1 }, { 2, 2 }, { 0, 0 }, { 2, 2 }, { 0, 0 }, { 1, 1 }, { 0, 1 }, { 0, 2 }, { 1, 2 } };
-		for (int ph = 0; ph < 9; ph++) {
-			c->launches += 2;
-			k_ic_field<<<gx, FT_TPB, 0, st>>>(N, box, pairs[ph][0], pairs[ph][1], A, Y);
-			CT_TRY(fft_check(c, cufftExecC2R(S.plans[0], Y, R), "cufftExecC2R"));
-			k_twolpt_phase<<<gn, FT_TPB, 0, st>>>(n, ph, R, fscale, part, delta2);
-		}
-		CT_TRY(fft_check(c, cufftExecR2C(S.plans[1], delta2, d2k), "cufftExecR2C"));
+		CT_TRY(field(1, 1, R1));
+		CT_TRY(field(2, 2, R2));
+		CT_TRY(field(0, 0, R));
+		c->launches += 2;
+		k_twolpt_products<<<gn, FT_TPB, 0, st>>>(n, R, R1, R2, fscale);
+		CT_TRY(field(0, 2, R));
+		CT_TRY(field(1, 2, R1));
+		k_twolpt_squares<<<gn, FT_TPB, 0, st>>>(n, R, R1, R2, fscale);
+		CT_TRY(fft_check(c, cufftExecR2C(S.plans[1], R2, d2k), "cufftExecR2C"));
 		for (int dim = 0; dim < 3; dim++) {
 			c->launches++;
-			k_ic_correction<<<gx, FT_TPB, 0, st>>>(d2k, Y, N, box, dim);
+			k_ic_correction<<<gx, FT_TPB, 0, st>>>(d2k, Y, N, box, dim, ax.filter);
 			CT_TRY(fft_check(c, cufftExecC2R(S.plans[0], Y, R), "cufftExecC2R"));
 			displace(dim, -D2, prefac2, dmax + 3 + dim);
 		}
