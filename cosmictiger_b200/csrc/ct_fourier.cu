@@ -11,6 +11,7 @@
 // (single precision, out of place); the reference's normalisations are applied around them.
 #include "ct_internal.cuh"
 
+#include <cub/cub.cuh>
 #include <cufft.h>
 
 #include <algorithm>
@@ -489,6 +490,160 @@ __global__ void __launch_bounds__(FT_TPB) k_density(int64_t n, const uint32_t* _
 	}
 }
 
+// The same deposit through shared memory.  216 float atomics a particle go to the L2 at about 390 G/s
+// whatever the particles' order (256^3 particles on 256^3 cells: 9.4 ms); here the particles are first
+// listed by tile of 8^3 cells, and a warp adds a tile's particles one after the other to its own copy
+// of the tile (13^3 cells with the kernel's reach), each lane one (x, y) row of the 6^3 cells, so that
+// no two lanes meet; the block's copies are summed and go to the grid with one atomic a cell and unit
+// of at most DEP_UNIT particles.  The row strides put the 32 rows of a warp on distinct banks.
+constexpr int DEP_TILE = 8;                // cells of a tile per axis
+constexpr int DEP_SPAN = DEP_TILE + 5;     // cells its particles reach
+constexpr int DEP_SY = 13, DEP_SX = 174;   // strides of y and x in the copy
+constexpr int DEP_CELLS = 12 * DEP_SX + 12 * DEP_SY + 13;
+constexpr int DEP_WARPS = 4;
+constexpr int DEP_UNIT = 1024;             // particles of a work unit
+constexpr int DEP_W = 20;                  // floats of a particle's weights: z, x, y, six each
+
+// Cell and fraction of a coordinate (the grid of accumulate_density_kernel, power.cu:32-61).
+__device__ __forceinline__ int deposit_cell(uint32_t X, int M, int N, float& frac) {
+	const float x = fmodf(M * (float(X) * (1.f / 4294967296.f)), 1.0f);
+	const int j = (int) (x * N);
+	frac = x * N - j;
+	return j < N ? j : j - N;  // (a product rounded up to N is cell 0's)
+}
+
+// Tile of every particle: counted, with the particle's rank among its tile's (in no order).
+__global__ void __launch_bounds__(FT_TPB) k_dep_count(int64_t n, const uint32_t* __restrict__ X, const uint32_t* __restrict__ Y, const uint32_t* __restrict__ Z,
+		int M, int N, int nt, uint32_t* __restrict__ count, uint32_t* __restrict__ rank) {
+	for (int64_t p0 = blockIdx.x * (int64_t) blockDim.x; p0 < n; p0 += (int64_t) gridDim.x * blockDim.x) {
+		const int64_t p = p0 + threadIdx.x;
+		uint32_t tile = 0xffffffffu;
+		if (p < n) {
+			float f;
+			const int j = deposit_cell(X[p], M, N, f) / DEP_TILE, k = deposit_cell(Y[p], M, N, f) / DEP_TILE, l = deposit_cell(Z[p], M, N, f) / DEP_TILE;
+			tile = (uint32_t) ((j * nt + k) * nt + l);
+		}
+		// one atomic for the lanes that share a tile (particles near in memory usually are near)
+		const unsigned same = __match_any_sync(0xffffffffu, tile);
+		const int lane = threadIdx.x & 31, leader = __ffs(same) - 1;
+		uint32_t base = 0;
+		if (lane == leader && p < n) {
+			base = atomicAdd(count + tile, (uint32_t) __popc(same));
+		}
+		base = __shfl_sync(0xffffffffu, base, leader);
+		if (p < n) {
+			rank[p] = base + (uint32_t) __popc(same & ((1u << lane) - 1u));
+		}
+	}
+}
+
+// The particles' indices by tile.
+__global__ void __launch_bounds__(FT_TPB) k_dep_order(int64_t n, const uint32_t* __restrict__ X, const uint32_t* __restrict__ Y, const uint32_t* __restrict__ Z,
+		int M, int N, int nt, const uint32_t* __restrict__ offset, const uint32_t* __restrict__ rank, uint32_t* __restrict__ order) {
+	for (int64_t p = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; p < n; p += (int64_t) gridDim.x * blockDim.x) {
+		float f;
+		const int j = deposit_cell(X[p], M, N, f) / DEP_TILE, k = deposit_cell(Y[p], M, N, f) / DEP_TILE, l = deposit_cell(Z[p], M, N, f) / DEP_TILE;
+		order[offset[(j * nt + k) * nt + l] + rank[p]] = (uint32_t) p;
+	}
+}
+
+// Work units (tile, first particle, particles) of the tiles that hold any.
+__global__ void __launch_bounds__(FT_TPB) k_dep_units(int ntile, const uint32_t* __restrict__ count, const uint32_t* __restrict__ offset, uint4* __restrict__ units,
+		unsigned int* __restrict__ nunits) {
+	const int t = blockIdx.x * blockDim.x + threadIdx.x;
+	if (t >= ntile || count[t] == 0) {
+		return;
+	}
+	const uint32_t c = count[t], nu = (c + DEP_UNIT - 1) / DEP_UNIT;
+	const unsigned int u = atomicAdd(nunits, nu);
+	for (uint32_t q = 0; q < nu; q++) {
+		units[u + q] = make_uint4((uint32_t) t, offset[t] + q * DEP_UNIT, min((uint32_t) DEP_UNIT, c - q * DEP_UNIT), 0u);
+	}
+}
+
+__global__ void __launch_bounds__(32 * DEP_WARPS) k_density_tiles(const uint32_t* __restrict__ X, const uint32_t* __restrict__ Y, const uint32_t* __restrict__ Z,
+		int M, int N, int nt, const uint32_t* __restrict__ order, const uint4* __restrict__ units, const unsigned int* __restrict__ nunits,
+		unsigned int* __restrict__ next, float* __restrict__ rho) {
+	__shared__ float s_rho[DEP_WARPS][DEP_CELLS];
+	__shared__ __align__(16) float s_w[DEP_WARPS][32][DEP_W];
+	__shared__ unsigned int s_unit;
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+	const unsigned int total = *nunits;
+	// this lane's rows of the 6 x 6 (x, y) rows: one of the first 32, and a quarter of one of the last
+	// four (24 lanes, one cell each)
+	const int a1 = lane / 6, b1 = lane % 6, o1 = a1 * DEP_SX + b1 * DEP_SY;
+	const int r2 = 32 + min(lane, 23) / 6, c2 = min(lane, 23) % 6, a2 = r2 / 6, b2 = r2 % 6, o2 = a2 * DEP_SX + b2 * DEP_SY + c2;
+	float* T = s_rho[w];
+	for (;;) {
+		if (threadIdx.x == 0) {
+			s_unit = atomicAdd(next, 1u);
+		}
+		__syncthreads();
+		const unsigned int u = s_unit;
+		if (u >= total) {
+			break;
+		}
+		const uint4 un = units[u];
+		const int tx = (int) (un.x / (uint32_t) (nt * nt)), ty = (int) (un.x / (uint32_t) nt % (uint32_t) nt), tz = (int) (un.x % (uint32_t) nt);
+		for (int i = lane; i < DEP_CELLS; i += 32) {
+			T[i] = 0.f;
+		}
+		__syncwarp();
+		for (uint32_t q0 = 32 * w; q0 < un.z; q0 += 32 * DEP_WARPS) {
+			// a particle a lane: its first cell in the tile and its 18 weights
+			const int cnt = min(32, (int) (un.z - q0));
+			int base = 0;
+			if (lane < cnt) {
+				const uint32_t p = order[un.y + q0 + lane];
+				float fx, fy, fz;
+				const int j = deposit_cell(X[p], M, N, fx), k = deposit_cell(Y[p], M, N, fy), l = deposit_cell(Z[p], M, N, fz);
+				base = (j - tx * DEP_TILE) * DEP_SX + (k - ty * DEP_TILE) * DEP_SY + (l - tz * DEP_TILE);
+				float* sw = s_w[w][lane];
+#pragma unroll
+				for (int q = 0; q < 6; q++) {
+					sw[q] = cloud_weight(fz - (q + CLOUD_MIN));
+					sw[6 + q] = cloud_weight(fx - (q + CLOUD_MIN));
+					sw[12 + q] = cloud_weight(fy - (q + CLOUD_MIN));
+				}
+			}
+			__syncwarp();
+			for (int i = 0; i < cnt; i++) {
+				const int bs = __shfl_sync(0xffffffffu, base, i);
+				const float* sw = s_w[w][i];
+				const float4 z0 = *reinterpret_cast<const float4*>(sw);
+				const float2 z1 = *reinterpret_cast<const float2*>(sw + 4);
+				const float wxy = sw[6 + a1] * sw[12 + b1];
+				float* r = T + bs + o1;
+				r[0] += wxy * z0.x;
+				r[1] += wxy * z0.y;
+				r[2] += wxy * z0.z;
+				r[3] += wxy * z0.w;
+				r[4] += wxy * z1.x;
+				r[5] += wxy * z1.y;
+				if (lane < 24) {
+					T[bs + o2] += sw[6 + a2] * sw[12 + b2] * sw[c2];
+				}
+				__syncwarp();  // the next particle's rows may be these
+			}
+		}
+		__syncthreads();
+		// the copies' sum to the grid (the reach wraps around the box)
+		for (int i = threadIdx.x; i < DEP_SPAN * DEP_SPAN * DEP_SPAN; i += 32 * DEP_WARPS) {
+			const int cz = i % DEP_SPAN, cy = i / DEP_SPAN % DEP_SPAN, cx = i / (DEP_SPAN * DEP_SPAN);
+			float v = 0.f;
+#pragma unroll
+			for (int q = 0; q < DEP_WARPS; q++) {
+				v += s_rho[q][cx * DEP_SX + cy * DEP_SY + cz];
+			}
+			if (v != 0.f) {
+				const int64_t gx = wrap(tx * DEP_TILE + cx + CLOUD_MIN, N), gy = wrap(ty * DEP_TILE + cy + CLOUD_MIN, N), gz = wrap(tz * DEP_TILE + cz + CLOUD_MIN, N);
+				atomicAdd(rho + (gx * N + gy) * N + gz, v);
+			}
+		}
+		__syncthreads();
+	}
+}
+
 // Bin of |k| (grid units) among the log-spaced edges (search_kbins, fft.cpp:219-237): -1 below
 // 0 or at / above the last edge.
 __device__ __forceinline__ int k_bin(const float* kb, int nb, double k) {
@@ -509,12 +664,22 @@ __device__ __forceinline__ int k_bin(const float* kb, int nb, double k) {
 
 constexpr int MAX_BINS = 1024;
 
+// Per-axis factors of the two passes by grid index: the inverse window, and sinc(pi i / N).
+__global__ void k_power_axis(int N, double* __restrict__ axis) {
+	const int I = blockIdx.x * blockDim.x + threadIdx.x;
+	if (I < N) {
+		const int64_t i = I < N / 2 ? I : I - N;
+		axis[I] = cloud_filter(2.0 * M_PI * i / N);
+		axis[N + I] = sinc(M_PI * i / N);
+	}
+}
+
 // Pass 1 (power_spectrum_compute, fft.cpp:240-304): each mode of the half-complex box,
 // deconvolved by the kernel's window (in place), adds |Y|^2, 1 and |k| to its bin.
 // Pass 2 (power_spectrum_compute2, :306-360): the mode is multiplied further by
 // (sinc(pi i/N) sinc(pi j/N) sinc(pi k/N))^-3 and adds (|Y|^2 - P_bin)^2 to its bin.
 __global__ void __launch_bounds__(FT_TPB) k_power_bins(cufftComplex* __restrict__ Y, int N, const float* __restrict__ kb, int nb, int pass,
-		const double* __restrict__ pmean, double* __restrict__ out) {
+		const double* __restrict__ axis, const double* __restrict__ pmean, double* __restrict__ out) {
 	__shared__ double s_p[MAX_BINS], s_c[MAX_BINS], s_k[MAX_BINS];
 	for (int b = threadIdx.x; b < nb; b += blockDim.x) {
 		s_p[b] = s_c[b] = s_k[b] = 0.0;
@@ -522,37 +687,60 @@ __global__ void __launch_bounds__(FT_TPB) k_power_bins(cufftComplex* __restrict_
 	__syncthreads();
 	const int NZ = N / 2 + 1;
 	const int64_t total = (int64_t) N * N * NZ;
-	for (int64_t e = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; e < total; e += (int64_t) gridDim.x * blockDim.x) {
-		const int I2 = (int) (e % NZ);
-		const int64_t row = e / NZ;
-		const int I0 = (int) (row / N), I1 = (int) (row % N);
-		const int64_t i = I0 < N / 2 ? I0 : I0 - N;
-		const int64_t j = I1 < N / 2 ? I1 : I1 - N;
-		const int64_t k = I2 < N / 2 ? I2 : I2 - N;
-		double c0;
-		if (pass == 1) {
-			c0 = cloud_filter(2.0 * M_PI * i / N) * cloud_filter(2.0 * M_PI * j / N) * cloud_filter(2.0 * M_PI * k / N);
-		} else {
-			c0 = pow(1.0 / (sinc(M_PI * i / N) * sinc(M_PI * j / N) * sinc(M_PI * k / N)), 3);
-		}
-		cufftComplex y = Y[e];
-		y.x *= c0;
-		y.y *= c0;
-		Y[e] = y;
-		const double kk = sqrt((double) (i * i + j * j + k * k));
-		if (kk > 0) {
-			const int bin = k_bin(kb, nb, kk);
-			if (bin >= 0) {
+	const double* f = axis + (pass == 1 ? 0 : N);
+	const int lane = threadIdx.x & 31;
+	// whole warps step together: the lanes' sums of a bin are added before they go to shared memory
+	// (the modes of a warp lie along a row and share few bins; an atomic each met in the same word)
+	for (int64_t e0 = blockIdx.x * (int64_t) blockDim.x; e0 < total; e0 += (int64_t) gridDim.x * blockDim.x) {
+		const int64_t e = e0 + threadIdx.x;
+		int bin = -1;
+		double vp = 0.0, vk = 0.0;
+		if (e < total) {
+			const unsigned row = (unsigned) (e / NZ);  // (at most 2^20 rows)
+			const int I2 = (int) (e - (int64_t) row * NZ);
+			const int I0 = (int) (row / (unsigned) N), I1 = (int) (row - (unsigned) I0 * (unsigned) N);
+			const int64_t i = I0 < N / 2 ? I0 : I0 - N;
+			const int64_t j = I1 < N / 2 ? I1 : I1 - N;
+			const int64_t k = I2 < N / 2 ? I2 : I2 - N;
+			double c0 = f[I0] * f[I1] * f[I2];
+			if (pass == 2) {
+				c0 = 1.0 / c0;
+				c0 = c0 * c0 * c0;
+			}
+			cufftComplex y = Y[e];
+			y.x *= c0;
+			y.y *= c0;
+			Y[e] = y;
+			const double kk = sqrt((double) (i * i + j * j + k * k));
+			if (kk > 0) {
+				bin = k_bin(kb, nb, kk);
 				const float pwr = y.x * y.x + y.y * y.y;
 				if (pass == 1) {
-					atomicAdd(&s_p[bin], (double) pwr);
-					atomicAdd(&s_c[bin], 1.0);
-					atomicAdd(&s_k[bin], kk);
-				} else {
+					vp = (double) pwr;
+					vk = kk;
+				} else if (bin >= 0) {
 					const double d = (double) (pwr - (float) pmean[bin]);
-					atomicAdd(&s_p[bin], d * d);
+					vp = d * d;
 				}
 			}
+		}
+		unsigned todo = __ballot_sync(0xffffffffu, bin >= 0);
+		while (todo) {
+			const int b = __shfl_sync(0xffffffffu, bin, __ffs(todo) - 1);
+			const unsigned mine = __ballot_sync(0xffffffffu, bin == b);
+			double p = bin == b ? vp : 0.0, q = bin == b ? vk : 0.0;
+			for (int o = 16; o; o >>= 1) {
+				p += __shfl_xor_sync(0xffffffffu, p, o);
+				q += __shfl_xor_sync(0xffffffffu, q, o);
+			}
+			if (lane == 0) {
+				atomicAdd(&s_p[b], p);
+				if (pass == 1) {
+					atomicAdd(&s_c[b], (double) __popc(mine));
+					atomicAdd(&s_k[b], q);
+				}
+			}
+			todo &= ~mine;
 		}
 	}
 	__syncthreads();
@@ -616,6 +804,42 @@ struct FtScope {
 		return fft_check(c, cufftSetStream(plans[which], c->stream), "cufftSetStream");
 	}
 };
+
+// The particles' mass on the grid.  By tiles where the tiles hold enough particles for their copies
+// to pay (DEP_MIN a tile on average) and the index arrays fit the budget, else particle by particle.
+constexpr int64_t DEP_MIN = 16;
+
+ct_status deposit(Ctx* c, FtScope& S, Box* b, int fold, int N, float* rho) {
+	cudaStream_t st = c->stream;
+	const int64_t np = b->n;
+	const int nt = (N + DEP_TILE - 1) / DEP_TILE;
+	const int64_t ntile = (int64_t) nt * nt * nt, max_units = np / DEP_UNIT + std::min(ntile, np) + 1;
+	size_t tmp_bytes = 0;
+	uint32_t *count = nullptr, *offset = nullptr, *rank = nullptr, *order = nullptr;
+	uint4* units = nullptr;
+	char* tmp = nullptr;
+	bool tiles = np >= DEP_MIN * ntile;
+	if (tiles) {
+		CT_CUDA(c, cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, count, offset, (int) ntile, st));
+		tiles = S.alloc(&count, ntile + 2, "tile counts") == CT_OK && S.alloc(&offset, ntile, "tile offsets") == CT_OK && S.alloc(&rank, np, "tile ranks") == CT_OK
+				&& S.alloc(&order, np, "tile order") == CT_OK && S.alloc(&units, max_units, "deposit units") == CT_OK && S.alloc(&tmp, tmp_bytes, "scan") == CT_OK;
+	}
+	if (!tiles) {
+		c->launches++;
+		k_density<<<ft_grid(c, np), FT_TPB, 0, st>>>(np, b->x[0], b->x[1], b->x[2], fold, N, rho);
+		return CT_OK;
+	}
+	unsigned int* ctr = (unsigned int*) (count + ntile);  // units made, units taken
+	CT_CUDA(c, cudaMemsetAsync(count, 0, sizeof(uint32_t) * (ntile + 2), st));
+	c->launches += 4;
+	k_dep_count<<<ft_grid(c, np), FT_TPB, 0, st>>>(np, b->x[0], b->x[1], b->x[2], fold, N, nt, count, rank);
+	CT_CUDA(c, cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, count, offset, (int) ntile, st));
+	k_dep_order<<<ft_grid(c, np), FT_TPB, 0, st>>>(np, b->x[0], b->x[1], b->x[2], fold, N, nt, offset, rank, order);
+	k_dep_units<<<(int) ((ntile + FT_TPB - 1) / FT_TPB), FT_TPB, 0, st>>>((int) ntile, count, offset, units, ctr);
+	const int nblk = (int) std::min<int64_t>(max_units, (int64_t) c->nsm * 4);
+	k_density_tiles<<<nblk, 32 * DEP_WARPS, 0, st>>>(b->x[0], b->x[1], b->x[2], fold, N, nt, order, units, ctr, ctr + 1, rho);
+	return CT_OK;
+}
 
 // cosmos_growth_factor (src/cosmology.cpp:80-87): the linear growth factor's fitting formula.
 double growth_factor(double omega_m, float a) {
@@ -865,19 +1089,21 @@ extern "C" ct_status ct_power_spectrum(ct_ctx* ctx, int box_id, int nfour, int f
 	CT_TRY(S.alloc(&dkb, kb.size(), "k bins"));
 	CT_TRY(S.alloc(&acc, 3 * nb, "bin sums"));
 	CT_TRY(S.alloc(&pmean, nb, "bin means"));
+	double* axis = nullptr;
+	CT_TRY(S.alloc(&axis, 2 * (size_t) N, "axis factors"));
 	CT_TRY(S.plan(1, N, CUFFT_R2C));
 	CT_CUDA(c, cudaMemcpyAsync(dkb, kb.data(), sizeof(float) * kb.size(), cudaMemcpyHostToDevice, st));
 	CT_CUDA(c, cudaMemsetAsync(acc, 0, sizeof(double) * 3 * nb, st));
 	// the grid starts at -1 (fft3d_init(N, -1), power.cpp:35) and gains the particles' weights
-	c->launches += 2;
+	c->launches += 3;
+	k_power_axis<<<(N + 127) / 128, 128, 0, st>>>(N, axis);
 	k_fill<<<ft_grid(c, ng), FT_TPB, 0, st>>>(ng, rho, -1.0f);
 	const int64_t np = b->n;
 	if (np > 0) {
-		c->launches++;
-		k_density<<<ft_grid(c, np), FT_TPB, 0, st>>>(np, b->x[0], b->x[1], b->x[2], fold, N, rho);
+		CT_TRY(deposit(c, S, b, fold, N, rho));
 	}
 	CT_TRY(fft_check(c, cufftExecR2C(S.plans[1], rho, Y), "cufftExecR2C"));
-	k_power_bins<<<ft_grid(c, ncx), FT_TPB, 0, st>>>(Y, N, dkb, nb, 1, nullptr, acc);
+	k_power_bins<<<ft_grid(c, ncx), FT_TPB, 0, st>>>(Y, N, dkb, nb, 1, axis, nullptr, acc);
 	std::vector<double> h(3 * nb);
 	CT_CUDA(c, cudaMemcpyAsync(h.data(), acc, sizeof(double) * 3 * nb, cudaMemcpyDeviceToHost, st));
 	CT_CUDA(c, cudaStreamSynchronize(st));
@@ -891,7 +1117,7 @@ extern "C" ct_status ct_power_spectrum(ct_ctx* ctx, int box_id, int nfour, int f
 	CT_CUDA(c, cudaMemcpyAsync(pmean, mean.data(), sizeof(double) * nb, cudaMemcpyHostToDevice, st));
 	CT_CUDA(c, cudaMemsetAsync(acc, 0, sizeof(double) * nb, st));
 	c->launches++;
-	k_power_bins<<<ft_grid(c, ncx), FT_TPB, 0, st>>>(Y, N, dkb, nb, 2, pmean, acc);
+	k_power_bins<<<ft_grid(c, ncx), FT_TPB, 0, st>>>(Y, N, dkb, nb, 2, axis, pmean, acc);
 	std::vector<double> dev(nb);
 	CT_CUDA(c, cudaMemcpyAsync(dev.data(), acc, sizeof(double) * nb, cudaMemcpyDeviceToHost, st));
 	CT_CUDA(c, cudaStreamSynchronize(st));
