@@ -703,12 +703,15 @@ __global__ void __launch_bounds__(128, 5) k_p2l(int64_t nn, const int32_t* __res
 // similar length, so that warps working at the same time read nearby source nodes.
 constexpr int ORDER_KEY_BITS = 6;  // bit lengths 0..32
 __global__ void k_order_keys(int64_t nn, const NodeW* __restrict__ nodes, const int2* __restrict__ ecc, const int2* __restrict__ dcc,
-		const int2* __restrict__ cp, uint32_t* __restrict__ key, int32_t* __restrict__ idx) {
+		const int2* __restrict__ cp, const int2* __restrict__ pp, uint32_t* __restrict__ key, int32_t* __restrict__ idx) {
 	for (int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < nn; i += (int64_t) gridDim.x * blockDim.x) {
 		const uint32_t le = (uint32_t) ecc[i].y, ld = (uint32_t) dcc[i].y, lp = (nodes[i].flags & 1) ? (uint32_t) cp[i].y : 0u;
 		key[i] = 32u - __clz(le);
 		key[nn + i] = 32u - __clz(ld);
 		key[2 * nn + i] = 32u - __clz(lp);
+		// leaves with particles by their source leaves times sinks (at least 1)
+		const uint32_t np = (uint32_t) (nodes[i].pend - nodes[i].pbeg);
+		key[3 * nn + i] = (nodes[i].flags & 1) && np ? 32u - __clz(max(1u, (uint32_t) min(0x7fffffffull, (unsigned long long) pp[i].y * np))) : 0u;
 		idx[i] = (int32_t) i;
 	}
 }
@@ -782,6 +785,8 @@ struct P2PArgs {
 	double* near_pairs;
 	unsigned long long* next;  // work counter: warps take tiles in list order
 	int tw;                    // sinks per tile (32, or 16: every tile through the SMALL path)
+	const int32_t* order;      // k_p2p_leaf: nodes, leaves with the most pairs first
+	int64_t nn;
 };
 
 // Approximate reciprocal square root (the MUFU unit), flushing denormals: pair separations
@@ -1156,6 +1161,183 @@ __global__ void __launch_bounds__(P2P_TPB, 3) k_p2p(P2PArgs a) {
 	}
 }
 
+// The same sums, a warp per leaf (up to 128 of its sinks at a time): each chunk of sources is staged
+// once and meets all of the leaf's tiles, instead of once a tile.  Staging (owner search, gathers,
+// conversions) and bookkeeping were 16 of k_p2p's 47 warp instructions a quad of pairs, and its waits
+// on the gathers and shuffles a fifth of its stalls.  The tiles' compensated sums and the sinks'
+// offsets stay in shared memory between chunks, which leaves 72 registers for seven blocks of four
+// warps an SM (28 warps against 24).  Every sink's sums are made from the same chunks in the same
+// order as k_p2p makes them, so the two give the same bits and either may run: this one where the
+// leaves keep its warps busy (see launch_p2p_any).
+constexpr int LEAF_TPB = 128;
+constexpr int LEAF_SINKS = 128;
+constexpr int64_t LEAF_WAVES = 2;  // leaves per resident warp from which a warp takes whole leaves
+template<int STAGE>
+struct LeafStage {
+	P2PStage<STAGE> src;
+	float4 s[LEAF_SINKS / 32][32];  // sums and compensations of (tile, lane)
+	float4 c[LEAF_SINKS / 32][32];
+	float k[3][LEAF_SINKS];         // the sinks' offsets from the leaf's centre
+	int2 leaf[32];                  // the source leaves of a class
+};
+
+template<int STAGE>
+__global__ void __launch_bounds__(LEAF_TPB, 7) k_p2p_leaf(P2PArgs a) {
+	extern __shared__ __align__(16) char leaf_smem[];
+	const int lane = threadIdx.x & 31;
+	LeafStage<STAGE>& my = reinterpret_cast<LeafStage<STAGE>*>(leaf_smem)[threadIdx.x >> 5];
+	double npairs = 0.0, nnear = 0.0;
+	for (;;) {
+		const int64_t si = next_node(a.next, a.order, a.nn);
+		if (si < 0) {
+			break;
+		}
+		const NodeW self = a.nodes[si];
+		const int nleaf = self.pend - self.pbeg;
+		if (!(self.flags & 1) || nleaf == 0) {
+			break;  // the rest of the order holds no leaf with particles
+		}
+		const float h = a.sub_h ? a.sub_h[box_of(a.sub_off, a.nsub, self.pbeg)] : a.h;
+		const float h2 = h * h, hinv = 1.f / h, h2inv = hinv * hinv, h3inv = h2inv * hinv;
+		const float near2 = h2 * 1.01f;  // (as in k_p2p)
+		const int2 ppl = a.pp[si];
+		for (int g0 = 0; g0 < nleaf; g0 += LEAF_SINKS) {
+			const int ns = min(LEAF_SINKS, nleaf - g0), nt = (ns + 31) / 32;
+			// the last tile, if at most 16 sinks: Sp lanes hold them, 32 / Sp replicas share the chunk
+			const int S = ns - 32 * (nt - 1);
+			const bool small = S <= 16;
+			const int Sp = S <= 1 ? 1 : 1 << (32 - __clz(S - 1));
+			__syncwarp();
+			for (int t = 0; t < nt; t++) {
+				const int q = 32 * t + lane;
+				if (q < ns) {
+					const int k = self.pbeg + g0 + q;
+					my.k[0][q] = fixed_dist(a.x[0][k], self.x);
+					my.k[1][q] = fixed_dist(a.x[1][k], self.y);
+					my.k[2][q] = fixed_dist(a.x[2][k], self.z);
+				}
+				my.s[t][lane] = my.c[t][lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+			}
+			int64_t np = 0, nn = 0;
+			for (int qb = 0; qb < ppl.y; qb += 32) {
+				int beg = 0, cnt = 0;
+				bool near = false;
+				if (qb + lane < ppl.y) {
+					const int sl = a.pp_list[ppl.x + qb + lane];
+					const int2 pr = *reinterpret_cast<const int2*>(&a.nodes[sl].pbeg);
+					beg = pr.x;
+					cnt = pr.y - pr.x;
+					near = box_gap2(a.nbox + 6 * si, a.nbox + 6 * (int64_t) sl) <= near2;
+				}
+				for (int cls = 0; cls < 2; cls++) {
+					const bool check = cls != 0;
+					const int c = near == check ? cnt : 0;
+					int inc = c;
+#pragma unroll
+					for (int o = 1; o < 32; o <<= 1) {
+						const int t = __shfl_up_sync(0xffffffffu, inc, o);
+						inc += lane >= o ? t : 0;
+					}
+					const int total = __shfl_sync(0xffffffffu, inc, 31);
+					// the class's leaves moved to the first lanes: flat indices [start, inc), particle
+					// index = first + flat index
+					const unsigned has = __ballot_sync(0xffffffffu, c > 0);
+					__syncwarp();
+					if (c > 0) {
+						my.leaf[__popc(has & ((1u << lane) - 1u))] = make_int2(inc, beg - (inc - c));
+					}
+					__syncwarp();
+					const int2 lf = lane < __popc(has) ? my.leaf[lane] : make_int2(0x7fffffff, 0);
+					inc = lf.x;
+					const int first = lf.y;
+					int start = __shfl_up_sync(0xffffffffu, inc, 1);
+					start = lane == 0 ? 0 : start;
+					for (int gb = 0; gb < total; gb += STAGE) {
+						const int n = min(STAGE, total - gb);
+						__syncwarp();  // the last chunk's readers are done
+#pragma unroll
+						for (int j = 0; j < STAGE; j += 32) {
+							// owner of flat index gb + j + lane: the leaves ending at or before gb + j, plus
+							// those starting after it up to the index
+							const int b = gb + j;
+							const int o0 = __popc(__ballot_sync(0xffffffffu, inc <= b));
+							const int rel = start - b;
+							const unsigned starts = __reduce_or_sync(0xffffffffu, rel > 0 && rel < 32 ? 1u << rel : 0u);
+							const int l = o0 + __popc(starts & ((2u << lane) - 1u));
+							const int pi = __shfl_sync(0xffffffffu, first, l & 31) + b + lane;
+							if (b + lane < total) {
+								stage_put(&my.src, j + lane, fixed_dist(a.x[0][pi], self.x), fixed_dist(a.x[1][pi], self.y), fixed_dist(a.x[2][pi], self.z));
+							}
+						}
+						__syncwarp();
+						for (int t = 0; t < nt; t++) {
+							int sl = lane, jb = 0, je = n;
+							if (t == nt - 1) {
+								sl = min(lane, S - 1);
+								if (small) {
+									sl = lane & (Sp - 1);
+									sl = sl < S ? sl : sl - S;
+									const int R = 32 / Sp, rep = lane / Sp;
+									const int sub = ((n + R - 1) / R + 3) & ~3;
+									jb = min(n, rep * sub);
+									je = min(n, jb + sub);
+								}
+							}
+							const float kx = my.k[0][32 * t + sl], ky = my.k[1][32 * t + sl], kz = my.k[2][32 * t + sl];
+							float fx = 0.f, fy = 0.f, fz = 0.f, pt = 0.f;
+							if (check) {
+								p2p_chunk<true, STAGE>(&my.src, jb, je, kx, ky, kz, h2, hinv, h2inv, h3inv, fx, fy, fz, pt);
+							} else {
+								p2p_chunk<false, STAGE>(&my.src, jb, je, kx, ky, kz, h2, hinv, h2inv, h3inv, fx, fy, fz, pt);
+							}
+							float4 sm = my.s[t][lane];
+							if (a.compensated) {
+								float4 cm = my.c[t][lane];
+								ksum(sm.x, cm.x, fx);
+								ksum(sm.y, cm.y, fy);
+								ksum(sm.z, cm.z, fz);
+								ksum(sm.w, cm.w, pt);
+								my.c[t][lane] = cm;
+							} else {
+								sm.x += fx;
+								sm.y += fy;
+								sm.z += fz;
+								sm.w += pt;
+							}
+							my.s[t][lane] = sm;
+						}
+						np += n;
+						nn += check ? n : 0;
+					}
+				}
+			}
+			for (int t = 0; t < nt; t++) {
+				const float4 sm = my.s[t][lane], cm = my.c[t][lane];
+				float tx = sm.x + cm.x, ty = sm.y + cm.y, tz = sm.z + cm.z, tp = sm.w + cm.w;
+				bool active = 32 * t + lane < ns;
+				if (t == nt - 1 && small) {
+					for (int o = Sp; o < 32; o <<= 1) {
+						tx += __shfl_xor_sync(0xffffffffu, tx, o);
+						ty += __shfl_xor_sync(0xffffffffu, ty, o);
+						tz += __shfl_xor_sync(0xffffffffu, tz, o);
+						tp += __shfl_xor_sync(0xffffffffu, tp, o);
+					}
+					active = lane < S;
+				}
+				if (active) {
+					a.F[self.pbeg + g0 + 32 * t + lane] = make_float4(tx, ty, tz, tp);
+				}
+			}
+			npairs += (double) np * ns;
+			nnear += (double) nn * ns;
+		}
+	}
+	if (lane == 0 && npairs > 0) {
+		atomicAdd(a.pairs, npairs);
+		atomicAdd(a.near_pairs, nnear);
+	}
+}
+
 // Tiles with more than 16 sinks to `big`, the others to `small` (order within each list is
 // immaterial: every tile computes its own sinks).
 __global__ void k_split_tiles(const int2* __restrict__ items, int64_t nitems, const NodeW* __restrict__ nodes, int tw, int2* big, int2* small,
@@ -1447,6 +1629,14 @@ void launch_p2p(const Ctx* c, const P2PArgs& pa, int64_t ntiles, cudaStream_t st
 	}
 }
 
+template<int STAGE>
+ct_status launch_p2p_leaf_t(Ctx* c, const P2PArgs& pa, cudaStream_t st) {
+	const size_t smem = sizeof(LeafStage<STAGE>) * (LEAF_TPB / 32);
+	CT_CUDA(c, cudaFuncSetAttribute(k_p2p_leaf<STAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem));
+	k_p2p_leaf<STAGE><<<resident_blocks(c, k_p2p_leaf<STAGE>, LEAF_TPB, smem), LEAF_TPB, smem, st>>>(pa);
+	return CT_OK;
+}
+
 struct KickBuffers {
 	int2* per_node = nullptr;  // 7 arrays of nnodes
 	size_t per_node_n = 0;
@@ -1586,26 +1776,26 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 		}
 		// ---- interactions
 		CT_CUDA(c, cudaMemsetAsync(counters, 0, 16 * sizeof(double), st));
-		// node orders of the three node-indexed kernels, longest lists first (radix sort of the
+		// node orders of the node-indexed kernels, longest lists first (radix sort of the
 		// list lengths' bit lengths; nodes without a list of a kind sort last)
 		ct_status s3 = CT_OK;
-		uint32_t* okey = (uint32_t*) scratch(c, 46, sizeof(uint32_t) * 6 * nn, &s3);
-		int32_t* oidx = (int32_t*) scratch(c, 47, sizeof(int32_t) * 4 * nn, &s3);
-		unsigned long long* onext = (unsigned long long*) scratch(c, 48, 3 * sizeof(unsigned long long), &s3);
+		uint32_t* okey = (uint32_t*) scratch(c, 46, sizeof(uint32_t) * 8 * nn, &s3);
+		int32_t* oidx = (int32_t*) scratch(c, 47, sizeof(int32_t) * 5 * nn, &s3);
+		unsigned long long* onext = (unsigned long long*) scratch(c, 48, 4 * sizeof(unsigned long long), &s3);
 		CT_TRY(s3);
 		size_t sort_bytes = 0;
-		CT_CUDA(c, cub::DeviceRadixSort::SortPairsDescending(nullptr, sort_bytes, okey, okey + 3 * nn, oidx, oidx + nn, (int) nn, 0, ORDER_KEY_BITS, st));
+		CT_CUDA(c, cub::DeviceRadixSort::SortPairsDescending(nullptr, sort_bytes, okey, okey + 4 * nn, oidx, oidx + nn, (int) nn, 0, ORDER_KEY_BITS, st));
 		void* sort_tmp = scratch(c, 49, sort_bytes + 256, &s3);
 		CT_TRY(s3);
 		c->launches++;
-		k_order_keys<<<(int) std::max<int64_t>(1, std::min<int64_t>((nn + 255) / 256, c->nsm * 8)), 256, 0, st>>>(nn, b->nodes, o.ecc, o.dcc, o.cp, okey,
+		k_order_keys<<<(int) std::max<int64_t>(1, std::min<int64_t>((nn + 255) / 256, c->nsm * 8)), 256, 0, st>>>(nn, b->nodes, o.ecc, o.dcc, o.cp, o.pp, okey,
 				oidx);
-		for (int k = 0; k < 3; k++) {
+		for (int k = 0; k < 4; k++) {
 			size_t tb = sort_bytes;
-			CT_CUDA(c, cub::DeviceRadixSort::SortPairsDescending(sort_tmp, tb, okey + k * nn, okey + (3 + k) * nn, oidx, oidx + (1 + k) * nn, (int) nn, 0,
+			CT_CUDA(c, cub::DeviceRadixSort::SortPairsDescending(sort_tmp, tb, okey + k * nn, okey + (4 + k) * nn, oidx, oidx + (1 + k) * nn, (int) nn, 0,
 					ORDER_KEY_BITS, st));
 		}
-		CT_CUDA(c, cudaMemsetAsync(onext, 0, 3 * sizeof(unsigned long long), st));
+		CT_CUDA(c, cudaMemsetAsync(onext, 0, 4 * sizeof(unsigned long long), st));
 		const size_t dl_bytes = sizeof(float) * NEXP_STRIDE * nn;
 		CT_CUDA(c, cudaMemsetAsync(K.dL, 0, dl_bytes, st));
 		// The three kernels run side by side on three streams, each into its own expansion
@@ -1695,34 +1885,45 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 			pa.pairs = counters + 4 + 7;
 			pa.near_pairs = counters + 13;
 			pa.tw = tw;
-			// full tiles and tiles of at most 16 sinks go to separate launches
-			int2* tiles2 = (int2*) scratch(c, 45, sizeof(int2) * 2 * (nitems + 1), &s2);
-			CT_TRY(s2);
-			unsigned long long* tcount = (unsigned long long*) (c->d_flags + 44);
-			CT_CUDA(c, cudaMemsetAsync(tcount, 0, 2 * sizeof(unsigned long long), st));
-			unsigned long long* wnext = (unsigned long long*) (c->d_flags + 52);  // work counters of the two launches
-			CT_CUDA(c, cudaMemsetAsync(wnext, 0, 2 * sizeof(unsigned long long), st));
+			const int64_t leaf_warps = (int64_t) c->nsm * 28;
+			if (c->tune.warps_per_tile == 1 && tw == 32 && nleaves >= LEAF_WAVES * leaf_warps) {
+				pa.order = oidx + 4 * nn;
+				pa.nn = nn;
+				pa.next = onext + 3;
+				cudaEventRecord(c->ev[4], st);
+				c->launches++;
+				const int stage = c->tune.p2p_stage;
+				CT_TRY(stage == 64 ? launch_p2p_leaf_t<64>(c, pa, st) : stage == 256 ? launch_p2p_leaf_t<256>(c, pa, st) : launch_p2p_leaf_t<128>(c, pa, st));
+			} else {
+				// full tiles and tiles of at most 16 sinks go to separate launches
+				int2* tiles2 = (int2*) scratch(c, 45, sizeof(int2) * 2 * (nitems + 1), &s2);
+				CT_TRY(s2);
+				unsigned long long* tcount = (unsigned long long*) (c->d_flags + 44);
+				CT_CUDA(c, cudaMemsetAsync(tcount, 0, 2 * sizeof(unsigned long long), st));
+				unsigned long long* wnext = (unsigned long long*) (c->d_flags + 52);  // work counters of the two launches
+				CT_CUDA(c, cudaMemsetAsync(wnext, 0, 2 * sizeof(unsigned long long), st));
 
-			c->launches++;
-			k_split_tiles<<<(int) std::max<int64_t>(1, std::min<int64_t>((nitems + 255) / 256, c->nsm * 8)), 256, 0, st>>>(items, nitems, b->nodes, tw,
-					tiles2, tiles2 + nitems + 1, tcount);
-			CT_CUDA(c, cudaMemcpyAsync(hf, tcount, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-			CT_CUDA(c, cudaStreamSynchronize(st));
-			const int64_t nbig = (int64_t) ((unsigned long long*) hf)[0], nsmall = (int64_t) ((unsigned long long*) hf)[1];
-			cudaEventRecord(c->ev[4], st);
-			if (nbig > 0) {
-				pa.items = tiles2;
-				pa.nitems = nbig;
-				pa.next = wnext;
 				c->launches++;
-				launch_p2p<false>(c, pa, nbig, st);
-			}
-			if (nsmall > 0) {
-				pa.items = tiles2 + nitems + 1;
-				pa.nitems = nsmall;
-				pa.next = wnext + 1;
-				c->launches++;
-				launch_p2p<true>(c, pa, nsmall, st);
+				k_split_tiles<<<(int) std::max<int64_t>(1, std::min<int64_t>((nitems + 255) / 256, c->nsm * 8)), 256, 0, st>>>(items, nitems, b->nodes, tw,
+						tiles2, tiles2 + nitems + 1, tcount);
+				CT_CUDA(c, cudaMemcpyAsync(hf, tcount, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+				CT_CUDA(c, cudaStreamSynchronize(st));
+				const int64_t nbig = (int64_t) ((unsigned long long*) hf)[0], nsmall = (int64_t) ((unsigned long long*) hf)[1];
+				cudaEventRecord(c->ev[4], st);
+				if (nbig > 0) {
+					pa.items = tiles2;
+					pa.nitems = nbig;
+					pa.next = wnext;
+					c->launches++;
+					launch_p2p<false>(c, pa, nbig, st);
+				}
+				if (nsmall > 0) {
+					pa.items = tiles2 + nitems + 1;
+					pa.nitems = nsmall;
+					pa.next = wnext + 1;
+					c->launches++;
+					launch_p2p<true>(c, pa, nsmall, st);
+				}
 			}
 			cudaEventRecord(c->ev[5], st);
 			KickTileArgs ka;
