@@ -573,6 +573,7 @@ void ct_ctx_destroy(ct_ctx* ctx) {
 		}
 	}
 	kick_buffers_release(c);
+	fourier_release(c);
 	for (auto& s : c->scratch) {
 		dfree(c, s.p, s.bytes);
 	}

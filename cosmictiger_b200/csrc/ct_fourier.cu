@@ -147,6 +147,50 @@ __device__ __forceinline__ float wavenumber(int I, int N, float box_size) {
 	return 2.f * (float) M_PI / box_size * float(i);
 }
 
+// sigma8 normalisation of the table (power_spectrum_function::normalize and
+// sigma8_integrand, initialize.cpp:141-172): Simpson's rule over 8192 log-k intervals of the
+// top-hat variance at R = 8 / h Mpc, the integrand in float as the reference takes it, the sum in
+// double; the table is scaled in place and the factor kept in norm.  One block: the host took 0.8 ms
+// for the same 8193 values.
+constexpr int SIGMA_TPB = 1024;
+constexpr int SIGMA_N = 8 * 1024;
+__global__ void __launch_bounds__(SIGMA_TPB) k_sigma8(PowerTable t, float* P, float logkmax_table, float hubble, double sigma8, float* norm) {
+	__shared__ double s_sum[SIGMA_TPB / 32];
+	const float logkmax = logkmax_table - 2.5 * t.dlogk;
+	const float logkmin = t.logkmin + 1.5 * t.dlogk;
+	const float dlogk = (logkmax - logkmin) / SIGMA_N;
+	const float R = 8 / hubble;
+	const float c0 = float(9) / (2. * float(M_PI) * float(M_PI)) / powf(R, 6);
+	double sum = 0.0;
+	for (int i = threadIdx.x; i <= SIGMA_N; i += SIGMA_TPB) {
+		const float x = i == SIGMA_N ? logkmax : logkmin + i * dlogk;
+		const float k = expf(x);
+		const float p = t(k);
+		const float tmp = (sinf(k * R) - k * R * cosf(k * R));
+		const float f = c0 * p * tmp * tmp * powf(k, -3.f);
+		const double w = i == 0 || i == SIGMA_N ? 1.0 / 3.0 : (i & 1) ? 4.0 / 3.0 : 2.0 / 3.0;
+		sum += w * f * dlogk;
+	}
+	for (int o = 16; o; o >>= 1) {
+		sum += __shfl_xor_sync(0xffffffffu, sum, o);
+	}
+	if ((threadIdx.x & 31) == 0) {
+		s_sum[threadIdx.x >> 5] = sum;
+	}
+	__syncthreads();
+	sum = 0.0;
+	for (int i = 0; i < SIGMA_TPB / 32; i++) {
+		sum += s_sum[i];
+	}
+	const float f = (float) ((sigma8 * sigma8) / sum);
+	for (int i = threadIdx.x; i < t.n; i += SIGMA_TPB) {
+		P[i] *= f;
+	}
+	if (threadIdx.x == 0) {
+		*norm = f;
+	}
+}
+
 // Per-axis values of one call, by grid index: the inverse window at the axis' wavenumber and the
 // lattice point's stencil (first cell and six weights).  Evaluated once an axis; every mode and
 // every point used to evaluate its own in double, which bounded the field and interpolation passes
@@ -346,7 +390,7 @@ __device__ __forceinline__ int wrap1(int i, int n) {
 
 __global__ void __launch_bounds__(FT_TPB) k_ic_displace(int N, const float* __restrict__ R, AxisTables t, double scale, float D, float prefac,
 		double box_size_inv, uint32_t* __restrict__ X, float* __restrict__ V, unsigned int* dxmax) {
-	extern __shared__ double s_rows[];  // [rows][N] sums along x, then [N] sums along x and y
+	extern __shared__ double s_rows[];  // [rows][N] sums along x, then [DISP_ROWS][N] sums along x and y
 	const int I0 = blockIdx.y, y0 = blockIdx.x * DISP_ROWS;
 	const int ny = min(DISP_ROWS, N - y0);
 	// rows y0's first neighbour .. the last row's last, wrapped (a lattice point's cell never falls
@@ -374,7 +418,6 @@ __global__ void __launch_bounds__(FT_TPB) k_ic_displace(int N, const float* __re
 		}
 	}
 	__syncthreads();
-	float mymax = 0.f;
 	for (int y = 0; y < ny; y++) {
 		const int first = __ldg(t.cell + y0 + y) + CLOUD_MIN - r0;
 		double wy[6];
@@ -388,30 +431,39 @@ __global__ void __launch_bounds__(FT_TPB) k_ic_displace(int N, const float* __re
 			for (int j = 0; j < 6; j++) {
 				acc += wy[j] * s_rows[(size_t) (first + j) * N + z];
 			}
-			s_y[z] = acc;
+			s_y[(size_t) y * N + z] = acc;
 		}
-		__syncthreads();
-		const int64_t base = ((int64_t) I0 * N + y0 + y) * N;
-		for (int z = threadIdx.x; z < N; z += FT_TPB) {
-			const int c = __ldg(t.cell + z) + CLOUD_MIN;
+	}
+	__syncthreads();
+	float mymax = 0.f;
+	for (int z = threadIdx.x; z < N; z += FT_TPB) {
+		const int c = __ldg(t.cell + z) + CLOUD_MIN;
+		int at[6];
+		double wz[6];
+#pragma unroll
+		for (int j = 0; j < 6; j++) {
+			at[j] = wrap1(c + j, N);
+			wz[j] = __ldg(t.weight + j * N + z);
+		}
+		for (int y = 0; y < ny; y++) {
+			const int64_t p = ((int64_t) I0 * N + y0 + y) * N + z;
 			double dx = 0.0;
 #pragma unroll
 			for (int j = 0; j < 6; j++) {
-				dx += __ldg(t.weight + j * N + z) * s_y[wrap1(c + j, N)];
+				dx += wz[j] * s_y[(size_t) y * N + at[j]];
 			}
 			dx *= scale;
 			dx *= -D * box_size_inv;
-			double x = fixed_to_double(X[base + z]) + dx;
+			double x = fixed_to_double(X[p]) + dx;
 			if (x >= 1.0) {
 				x -= 1.0;
 			} else if (x < 0.0) {
 				x += 1.0;
 			}
-			X[base + z] = fixed_from_double(x);
-			V[base + z] += prefac * dx;
+			X[p] = fixed_from_double(x);
+			V[p] += prefac * dx;
 			mymax = fmaxf(mymax, (float) (dx * N));
 		}
-		__syncthreads();
 	}
 	for (int o = 16; o; o >>= 1) {
 		mymax = fmaxf(mymax, __shfl_xor_sync(0xffffffffu, mymax, o));
@@ -772,24 +824,35 @@ ct_status fft_check(Ctx* c, cufftResult r, const char* what) {
 	return CT_OK;
 }
 
-// Device buffers and cuFFT plans of one call, released on every return path.
+}  // namespace
+
+// The context's cuFFT plans, one of each kind: kept from one call to the next of the same grid (a
+// plan's making took 0.3 to 0.8 ms, several times the transforms of a 64^3 grid), replaced for
+// another grid, freed with the context.  They hold no work area: each call lends one from the
+// context's pool.
+struct FtPlans {
+	cufftHandle plan[2] = { 0, 0 };
+	size_t work[2] = { 0, 0 };
+	int n[2] = { 0, 0 };
+};
+
+namespace {
+
+// Device buffers of one call, released on every return path.
 struct FtScope {
 	Ctx* c;
 	std::vector<std::pair<void*, size_t>> bufs;
+	std::vector<void*> work;
 	cufftHandle plans[2] = { 0, 0 };
-	bool have[2] = { false, false };
 
 	explicit FtScope(Ctx* c_) : c(c_) {
 	}
 	~FtScope() {
-		cudaStreamSynchronize(c->stream);
-		for (int i = 0; i < 2; i++) {
-			if (have[i]) {
-				cufftDestroy(plans[i]);
-			}
-		}
 		for (auto& b : bufs) {
 			dfree(c, b.first, b.second);
+		}
+		for (auto p : work) {
+			cudaFreeAsync(p, c->stream);
 		}
 	}
 	template<class T>
@@ -799,8 +862,38 @@ struct FtScope {
 		return CT_OK;
 	}
 	ct_status plan(int which, int N, cufftType type) {
-		CT_TRY(fft_check(c, cufftPlan3d(&plans[which], N, N, N, type), "cufftPlan3d"));
-		have[which] = true;
+		if (!c->ft) {
+			c->ft = new FtPlans();
+		}
+		FtPlans& F = *c->ft;
+		if (F.n[which] != N) {
+			if (F.n[which]) {
+				cufftDestroy(F.plan[which]);
+				F.n[which] = 0;
+			}
+			CT_TRY(fft_check(c, cufftCreate(&F.plan[which]), "cufftCreate"));
+			cufftResult r = cufftSetAutoAllocation(F.plan[which], 0);
+			if (r == CUFFT_SUCCESS) {
+				r = cufftMakePlan3d(F.plan[which], N, N, N, type, &F.work[which]);
+			}
+			if (r != CUFFT_SUCCESS) {
+				cufftDestroy(F.plan[which]);
+				return fft_check(c, r, "cufftMakePlan3d");
+			}
+			F.n[which] = N;
+		}
+		plans[which] = F.plan[which];
+		// the work area is cuFFT's own business and outside the budget, as when plans allocated it
+		void* w = nullptr;
+		if (F.work[which]) {
+			const cudaError_t e = cudaMallocFromPoolAsync(&w, F.work[which], c->pool, c->stream);
+			if (e != cudaSuccess) {
+				cudaGetLastError();
+				return fail(c, CT_ERR_MEMORY, std::string("device allocation failed for a transform's work area: ") + cudaGetErrorString(e));
+			}
+			work.push_back(w);
+			CT_TRY(fft_check(c, cufftSetWorkArea(plans[which], w), "cufftSetWorkArea"));
+		}
 		return fft_check(c, cufftSetStream(plans[which], c->stream), "cufftSetStream");
 	}
 };
@@ -851,41 +944,20 @@ double growth_factor(double omega_m, float a) {
 	return a * 2.5 * Om / (pow(Om, 4.f / 7.f) - Ol + (1.f + 0.5f * Om) * (1.f + 0.014285714f * Ol));
 }
 
-// sigma8 normalisation of the table (power_spectrum_function::normalize and
-// sigma8_integrand, initialize.cpp:141-172): Simpson's rule over 8192 log-k intervals of the
-// top-hat variance at R = 8 / h Mpc, in float; the table is scaled in place and the factor
-// returned.
-float sigma8_normalize(PowerTable& t, std::vector<float>& P, float logkmax_table, double hubble, double sigma8) {
-	auto integrand = [&](float x) -> float {
-		const float R = 8 / (float) hubble;
-		const float c0 = float(9) / (2. * float(M_PI) * float(M_PI)) / powf(R, 6);
-		const float k = std::exp(x);
-		const float p = t(k);
-		const float tmp = (std::sin(k * R) - k * R * std::cos(k * R));
-		return c0 * p * tmp * tmp * std::pow(k, -3);
-	};
-	const int N = 8 * 1024;
-	float sum = 0.0;
-	const float logkmax = logkmax_table - 2.5 * t.dlogk;
-	const float logkmin = t.logkmin + 1.5 * t.dlogk;
-	const float dlogk = (logkmax - logkmin) / N;
-	sum = (1.0 / 3.0) * (integrand(logkmax) + integrand(logkmin)) * dlogk;
-	for (int i = 1; i < N; i += 2) {
-		const float logk = logkmin + i * dlogk;
-		sum += (4.0 / 3.0) * integrand(logk) * dlogk;
+}  // namespace
+
+void fourier_release(Ctx* c) {
+	if (c->ft) {
+		for (int i = 0; i < 2; i++) {
+			if (c->ft->n[i]) {
+				cufftDestroy(c->ft->plan[i]);
+			}
+		}
+		delete c->ft;
+		c->ft = nullptr;
 	}
-	for (int i = 2; i < N; i += 2) {
-		const float logk = logkmin + i * dlogk;
-		sum += (2.0 / 3.0) * integrand(logk) * dlogk;
-	}
-	sum = (sigma8 * sigma8) / sum;
-	for (auto& q : P) {
-		q *= sum;
-	}
-	return sum;
 }
 
-}  // namespace
 }  // namespace ct
 
 using namespace ct;
@@ -936,7 +1008,6 @@ extern "C" ct_status ct_initialize(ct_ctx* ctx, int box_id, const ct_ic_params* 
 		return fail(c, CT_ERR_ARG, "ct_initialize: the power table does not cover the grid's wavenumbers " + std::to_string(kf) + " .. " +
 				std::to_string(kN) + " / Mpc");
 	}
-	const float norm = sigma8_normalize(tab, P, logkmax, p->hubble, p->sigma8);
 	// growth and velocity factors (initialize(), initialize.cpp:262-275)
 	const float omega_m = (float) p->omega_m;
 	const float a0 = 1.0 / (p->z0 + 1.0);
@@ -959,7 +1030,7 @@ extern "C" ct_status ct_initialize(ct_ctx* ctx, int box_id, const ct_ic_params* 
 	cufftComplex* Y = nullptr;
 	float* R = nullptr;
 	AxisTables ax = {};
-	unsigned int* dmax = nullptr;
+	unsigned int* dmax = nullptr;  // six displacement maxima, then the table's factor
 	CT_TRY(S.alloc(&dP, P.size(), "power table"));
 	CT_TRY(S.alloc(&A, ncx, "mode amplitudes"));
 	CT_TRY(S.alloc(&Y, ncx, "k-space field"));
@@ -967,7 +1038,7 @@ extern "C" ct_status ct_initialize(ct_ctx* ctx, int box_id, const ct_ic_params* 
 	CT_TRY(S.alloc(&ax.filter, N, "axis tables"));
 	CT_TRY(S.alloc(&ax.cell, N, "axis tables"));
 	CT_TRY(S.alloc(&ax.weight, 6 * (size_t) N, "axis tables"));
-	CT_TRY(S.alloc(&dmax, 6, "displacement maxima"));
+	CT_TRY(S.alloc(&dmax, 7, "displacement maxima"));
 	CT_TRY(S.plan(0, N, CUFFT_C2R));
 	CT_CUDA(c, cudaMemcpyAsync(dP, P.data(), sizeof(float) * P.size(), cudaMemcpyHostToDevice, st));
 	CT_CUDA(c, cudaMemsetAsync(dmax, 0, 6 * sizeof(unsigned int), st));
@@ -978,13 +1049,14 @@ extern "C" ct_status ct_initialize(ct_ctx* ctx, int box_id, const ct_ic_params* 
 	const float fscale = (float) scale;
 	const double box_inv = 1.0 / box;
 	const int gn = ft_grid(c, n), gx = ft_grid(c, ncx);
-	c->launches += 4;
+	c->launches += 5;
+	k_sigma8<<<1, SIGMA_TPB, 0, st>>>(dtab, dP, logkmax, (float) p->hubble, p->sigma8, (float*) (dmax + 6));
 	k_ic_axis<<<(N + 127) / 128, 128, 0, st>>>(N, box, ax);
 	k_ic_lattice<<<gn, FT_TPB, 0, st>>>(N, b->x[0], b->x[1], b->x[2], b->v[0], b->v[1], b->v[2], b->rung);
 	k_ic_uniforms<<<ft_grid(c, (int64_t) N * N), FT_TPB, 0, st>>>(N, A);
 	k_ic_amplitude<<<gx, FT_TPB, 0, st>>>(N, box, factor, dtab, A);
 	// interpolation at the lattice points and update of axis dim
-	const size_t disp_smem = sizeof(double) * (DISP_ROWS + 7) * N;  // 120 KB at the largest grid
+	const size_t disp_smem = sizeof(double) * (2 * DISP_ROWS + 6) * N;  // 176 KB at the largest grid
 	CT_CUDA(c, cudaFuncSetAttribute(k_ic_displace, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) disp_smem));
 	auto displace = [&](int dim, float D, float prefac, unsigned int* mx) {
 		c->launches++;
@@ -1025,7 +1097,7 @@ extern "C" ct_status ct_initialize(ct_ctx* ctx, int box_id, const ct_ic_params* 
 		}
 	}
 	CT_CUDA(c, cudaGetLastError());
-	unsigned int hm[6];
+	unsigned int hm[7];
 	CT_CUDA(c, cudaMemcpyAsync(hm, dmax, sizeof(hm), cudaMemcpyDeviceToHost, st));
 	CT_CUDA(c, cudaStreamSynchronize(st));
 	b->rung_begin = 0;
@@ -1036,6 +1108,8 @@ extern "C" ct_status ct_initialize(ct_ctx* ctx, int box_id, const ct_ic_params* 
 		ret->D2 = D2;
 		ret->prefac1 = prefac1;
 		ret->prefac2 = prefac2;
+		float norm;
+		memcpy(&norm, hm + 6, 4);
 		ret->norm = norm;
 		for (int d = 0; d < 3; d++) {
 			float a, q;

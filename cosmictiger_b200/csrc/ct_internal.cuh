@@ -129,6 +129,9 @@ struct Box {
 // Frees a box's lightcone buffers (ct_lightcone.cu).
 void lightcone_release(Ctx* c, Box* b);
 
+struct FtPlans;  // cuFFT plans kept between calls (ct_fourier.cu)
+void fourier_release(Ctx* c);  // frees them (called by ct_ctx_destroy)
+
 struct KickBuffers;  // interaction lists and expansions of the kick (ct_kick.cu)
 
 // Host-visible error state and stream.
@@ -162,6 +165,7 @@ struct Ctx {
 	int compensated = 1;              // Neumaier-compensated P2P batch sums
 	int priority = 0;                 // CUDA stream priority of stream and side[] (0: default)
 	KickBuffers* kick = nullptr;      // owned; grown by the kick, freed with the context
+	FtPlans* ft = nullptr;            // owned; freed with the context
 };
 
 // Device time between two recorded events, 0 if it is not available.  A failed query sets the
