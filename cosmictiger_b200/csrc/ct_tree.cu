@@ -20,23 +20,32 @@
 
 #include "ct_internal.cuh"
 #include "ct_ops.cuh"
+#include "ct_partition.cuh"
 
 namespace ct {
 namespace {
 
 // ---------------------------------------------------------------- the levels
 // One cooperative launch builds every level: a resident grid whose blocks meet at grid barriers
-// between the phases of a level.  What bounded the build before was the level's structure, not its
-// data: twelve launches, two scans and a host round trip a level (16^3 particles: 0.87 ms for 11
-// levels and 64 KB of positions; 10^6 clustered particles: 2.7 ms for 28 levels).  A level whose
-// split nodes all hold at most WARP_NODE particles takes two barriers, others five.
+// (1.2 us from the last arrival) between the phases of a level.  What bounded the build before was the
+// level's structure, not its data: twelve launches, two scans and a host round trip a level (16^3
+// particles: 0.87 ms for 11 levels and 64 KB of positions; 10^6 clustered particles: 2.7 ms for 28
+// levels).  By the number of nodes on the level:
+//   few (at most 4 a block): a block partitions the nodes of its own share, by a warp up to WARP_FEW
+//   particles and by the whole block up to BLOCK_LINE, which is quickest for one node.  A child is
+//   counted by the block that makes it, so that the level takes one barrier.
+//   many: a warp partitions up to WARP_FEW particles (WARP_MANY where there are two nodes a warp), and
+//   warps take nodes from all shares, since the shares' work is uneven in a clustered box; three
+//   barriers.
+// Larger nodes go tile by tile over the whole grid, three barriers more.
 constexpr int LTPB = 512;             // threads of a level block
 constexpr int LWARPS = LTPB / 32;
-constexpr int TILE_ROWS = 8;
-constexpr int TILE = LTPB * TILE_ROWS;  // particles of a tile
-constexpr int WARP_NODE = 1024;       // nodes up to this size are partitioned by one warp: its lanes
-                                      // hold the 32 ballots of the node's particles
-constexpr int NODE_SPLIT = 2, NODE_TILES = 4;  // NodeW.flags while a level is built
+constexpr int SUB = 1024;             // particles whose ballots a warp's lanes hold, one each
+constexpr int BLOCK_SUB = 256;        // particles a warp takes of a node partitioned by its block
+constexpr int BLOCK_LINE = BLOCK_SUB * LWARPS;
+constexpr int WARP_FEW = SUB, WARP_MANY = 4 * SUB;
+constexpr int NODE_SPLIT = 2;         // NodeW.flags besides bit 0 (leaf)
+constexpr int TAKE = 4;               // nodes a warp takes at a time
 
 // A node partitioned in tiles by the whole grid.
 struct TileNode {
@@ -51,6 +60,7 @@ struct LevelCtl {
 	unsigned int arrived;  // barrier arrivals of this launch
 	int error;             // a barrier gave up
 	int status;            // 0 done, 1 the node arrays are full before `level`
+	unsigned int take[2];  // nodes taken of an even and an odd level
 	int level;
 	int64_t lb, le;        // nodes of `level`
 	int64_t need;          // nodes the arrays must hold
@@ -70,12 +80,16 @@ struct LevelArgs {
 	TileNode* tnode;
 	int32_t* tile_of;  // tile -> entry of tnode
 	int32_t* tile_lt;  // tile -> particles below the midpoint
-	int4* blk;         // per block: split nodes, tile nodes, tiles of its share of a level
+	uint32_t* tile_mask;  // the tile nodes' ballots, 32 words a SUB (see mask_row)
+	int4* blk;         // two levels' worth, per block: split nodes, tile nodes, tiles of a range of
+	                   // consecutive nodes, and the range's first node
 	LevelCtl* ctl;
 	int* flags;
 	const int64_t* off;
 	int64_t pb, n, node_cap;
 	int nroot, bucket, resume;
+	int sub;        // particles a warp takes of a tile: SUB, or BLOCK_SUB while tiles of 16 SUB would
+	                // leave blocks without one
 	double theta, hsoft;
 };
 
@@ -106,6 +120,12 @@ __device__ __forceinline__ bool grid_meet(LevelCtl* ctl, unsigned int& round) {
 	return !__syncthreads_or(bad);
 }
 
+// Row of the ballots of SUB s of tile node ti, which starts at particle pbeg: the tile nodes come in
+// particle order, so rows counted by particles, one spare a node, do not meet.
+__device__ __forceinline__ int64_t mask_row(const LevelArgs& a, int pbeg, int ti, int s) {
+	return ((int64_t) pbeg - a.pb) / a.sub + ti + s;
+}
+
 // Longest side of a node's box and its midpoint (tree.cpp:336-348).
 __device__ __forceinline__ int split_dim(const double* gb, double& xm) {
 	int xdim = 0;
@@ -121,25 +141,83 @@ __device__ __forceinline__ int split_dim(const double* gb, double& xm) {
 	return xdim;
 }
 
-// The two children of node ni, split at particle `mid`, by the lanes of a warp.
-__device__ __forceinline__ void make_children(const LevelArgs& a, int64_t ni, const NodeW& nd, int mid, int xd, double xm, int level, int lane) {
+// Leaf or split (tree.cpp:314-348): the flags of a node of box gb with nparts particles.
+__device__ __forceinline__ int classify(const LevelArgs& a, const double* gb, int nparts, int level) {
+	float box_r = 0.0f;
+#pragma unroll
+	for (int dim = 0; dim < 3; dim++) {
+		const double h = 0.5 * (gb[3 + dim] - gb[dim]);
+		box_r += h * h;
+	}
+	box_r = sqrtf(box_r);
+	const bool ewald_satisfied = (box_r < 0.25 * (a.theta / (1.0 + a.theta)) && box_r < 0.125 - 0.25 * a.hsoft);
+	if (!(nparts > a.bucket || (!ewald_satisfied && nparts > 0))) {
+		return 1;
+	}
+	if (level >= MAX_DEPTH - 1) {
+		atomicOr(a.flags + 2, 1);
+		return 1;
+	}
+	return NODE_SPLIT;
+}
+// A level of many nodes, and the size above which its nodes go tile by tile.
+__device__ __forceinline__ bool many_nodes(int64_t nl) {
+	return nl > 4 * (int64_t) gridDim.x;
+}
+// (on a level of many nodes a warp takes the larger ones too once there are two nodes a warp)
+__device__ __forceinline__ int warp_line_of(int64_t nl) {
+	return nl > 2 * LWARPS * (int64_t) gridDim.x ? WARP_MANY : WARP_FEW;
+}
+__device__ __forceinline__ int tile_line(int64_t nl) {
+	return many_nodes(nl) ? warp_line_of(nl) : BLOCK_LINE;
+}
+// What a node adds to its range's counts: split nodes, tile nodes, tiles.
+__device__ __forceinline__ int3 counted(const LevelArgs& a, int flags, int nparts, int line) {
+	const bool sp = flags & NODE_SPLIT, t = sp && nparts > line;
+	const int tile = a.sub * LWARPS;
+	return make_int3(sp, t, t ? (nparts + tile - 1) / tile : 0);
+}
+
+// The two children of node ni, split at particle `mid`, by the lanes of a warp; their counts (with the
+// next level's tile line) are added to sum (shared memory).
+__device__ __forceinline__ void make_children(const LevelArgs& a, int64_t ni, const NodeW& nd, int mid, int xd, double xm, int level, int lane, int line,
+		int* sum) {
 	const int64_t l = nd.child;
+	double gb[6];
+#pragma unroll
+	for (int d = 0; d < 6; d++) {
+		gb[d] = a.gbox[6 * ni + d];
+	}
+	const int side = lane & 1;
+#pragma unroll
+	for (int d = 0; d < 3; d++) {
+		gb[3 + d] = side == 0 && d == xd ? xm : gb[3 + d];
+		gb[d] = side == 1 && d == xd ? xm : gb[d];
+	}
 	if (lane < 2) {
 		NodeW c;
 		c.x = c.y = c.z = 0;
 		c.radius = 0.f;
 		c.child = -1;
-		c.flags = 1;
 		c.pbeg = lane == 0 ? nd.pbeg : mid;
 		c.pend = lane == 0 ? mid : nd.pend;
+		c.flags = classify(a, gb, c.pend - c.pbeg, level + 1);
 		a.nodes[l + lane] = c;
 		a.key[l + lane] = (a.key[ni] << 1) + lane;
 		a.depth[l + lane] = level + 1;
 		a.parent[l + lane] = (int32_t) ni;
-	}
-	if (lane < 12) {
-		const int side = lane / 6, d = lane % 6;
-		a.gbox[6 * (l + side) + d] = d == (side == 0 ? 3 + xd : xd) ? xm : a.gbox[6 * ni + d];
+#pragma unroll
+		for (int d = 0; d < 6; d++) {
+			a.gbox[6 * (l + lane) + d] = gb[d];
+		}
+		const int3 k = counted(a, c.flags, c.pend - c.pbeg, line);
+		if (k.x) {
+			atomicAdd(sum, k.x);
+		}
+		if (k.y) {
+			atomicAdd(sum + 1, k.y);
+			atomicAdd(sum + 2, k.z);
+		}
 	}
 }
 
@@ -155,13 +233,9 @@ __device__ __forceinline__ void swap_particles(const LevelArgs& a, int p, int q)
 	a.idx[q] = t;
 }
 
-// The partition of a node of at most WARP_NODE particles by one warp: lane c keeps the ballot of
-// particles 32 c .. 32 c + 31.  With m of them below the midpoint, the k-th particle at or above it
-// in the first m (from the left) changes places with the k-th below it in the rest (from the
-// right), which is the reference's two-pointer loop.  pos: WARP_NODE offsets in shared memory.
-__device__ __forceinline__ int warp_partition(const LevelArgs& a, const NodeW& nd, const uint32_t* xd, uint32_t xm, uint16_t* pos, int lane) {
-	const int n = nd.pend - nd.pbeg;
-	const uint32_t* xp = xd + nd.pbeg;
+// Ballots of up to SUB particles from xp on: lane c's has bit j set when particle 32 c + j lies below
+// the midpoint.
+__device__ __forceinline__ unsigned sub_below(const uint32_t* xp, int n, uint32_t xm, int lane) {
 	unsigned mine = 0;
 	for (int c0 = 0; c0 * 32 < n; c0 += 8) {
 		uint32_t v[8];
@@ -176,53 +250,136 @@ __device__ __forceinline__ int warp_partition(const LevelArgs& a, const NodeW& n
 			mine = lane == c0 + j ? lt : mine;
 		}
 	}
-	int m = __popc(mine);
-	for (int o = 16; o; o >>= 1) {
-		m += __shfl_xor_sync(0xffffffffu, m, o);
+	return mine;
+}
+// The partition of a node of at most WARP_MANY particles by one warp.  With m particles below the
+// midpoint, the k-th particle at or above it in the first m (from the left) changes places with the
+// k-th below it in the rest (from the right), which is the reference's two-pointer loop.  pos: SUB
+// offsets in shared memory; longer swaps go through the global scratch.
+__device__ __forceinline__ int warp_partition(const LevelArgs& a, const NodeW& nd, const uint32_t* xd, uint32_t xm, uint16_t* pos, int lane) {
+	constexpr int NS = WARP_MANY / SUB;
+	const int n = nd.pend - nd.pbeg;
+	unsigned mine[NS];
+	int m = 0;
+#pragma unroll
+	for (int q = 0; q < NS; q++) {
+		mine[q] = SUB * q < n ? sub_below(xd + nd.pbeg + SUB * q, min(SUB, n - SUB * q), xm, lane) : 0u;
+		m += __popc(mine[q]);
 	}
-	// this lane's 32 particles: those before the split point that are not below, and below after it
-	const int first = 32 * lane;
-	const unsigned valid = first >= n ? 0u : (n - first >= 32 ? 0xffffffffu : (1u << (n - first)) - 1u);
-	const unsigned before = first >= m ? 0u : (m - first >= 32 ? 0xffffffffu : (1u << (m - first)) - 1u);
-	unsigned L = before & ~mine & valid, R = mine & ~before;
-	int cl = __popc(L), cr = __popc(R);
-	int il = cl, ir = cr;
-	for (int o = 1; o < 32; o <<= 1) {
-		const int tl = __shfl_up_sync(0xffffffffu, il, o), tr = __shfl_up_sync(0xffffffffu, ir, o);
-		il += lane >= o ? tl : 0;
-		ir += lane >= o ? tr : 0;
+	m = __reduce_add_sync(0xffffffffu, m);
+	int ns = 0;
+#pragma unroll
+	for (int q = 0; q < NS; q++) {
+		ns += __popc(mine[q] & ~first_bits(m - SUB * q, 32 * lane));
 	}
-	const int ns = __shfl_sync(0xffffffffu, il, 31);  // as many on the right
-	if (ns > 0) {
-		uint16_t* pl = pos;
-		uint16_t* pr = pos + WARP_NODE / 2;
-		int k = il - cl;
-		while (L) {
-			pl[k++] = (uint16_t) (first + __ffs(L) - 1);
-			L &= L - 1;
-		}
-		k = ns - 1 - (ir - cr);
-		while (R) {
-			pr[k--] = (uint16_t) (first + __ffs(R) - 1);
-			R &= R - 1;
-		}
-		__syncwarp();
-		for (int q = lane; q < ns; q += 32) {
-			swap_particles(a, nd.pbeg + pl[q], nd.pbeg + pr[q]);
-		}
-		__syncwarp();
+	ns = __reduce_add_sync(0xffffffffu, ns);
+	if (ns == 0) {
+		return m;
 	}
+	const bool few = ns <= SUB / 2;
+	uint16_t* pl = pos;
+	uint16_t* pr = pos + SUB / 2;
+	int lt = 0;  // below the midpoint in earlier SUBs
+#pragma unroll
+	for (int q = 0; q < NS; q++) {
+		if (SUB * q < n) {
+			const int here = __reduce_add_sync(0xffffffffu, __popc(mine[q]));
+			const int l0 = SUB * q - lt, r0 = m - lt - here;
+			sub_wrong(mine[q], min(SUB, n - SUB * q), max(0, min(SUB, m - SUB * q)), lane,
+					[&](int k, int o) {
+						if (few) {
+							pl[l0 + k] = (uint16_t) (SUB * q + o);
+						} else {
+							a.posL[nd.pbeg + l0 + k] = SUB * q + o;
+						}
+					},
+					[&](int k, int o) {
+						if (few) {
+							pr[r0 + k] = (uint16_t) (SUB * q + o);
+						} else {
+							a.posR[nd.pbeg + r0 + k] = SUB * q + o;
+						}
+					});
+			lt += here;
+		}
+	}
+	__syncwarp();
+	for (int q = lane; q < ns; q += 32) {
+		swap_particles(a, nd.pbeg + (few ? pl[q] : a.posL[nd.pbeg + q]), nd.pbeg + (few ? pr[q] : a.posR[nd.pbeg + q]));
+	}
+	__syncwarp();
 	return m;
 }
 
+// Shared memory of a level block.
+struct LevelShared {
+	uint16_t pos[LWARPS][SUB];
+	int scan[3][LWARPS];
+	int sum[2][LWARPS];
+	int totals[7][LWARPS];
+	unsigned mask[LWARPS];
+	int tot[3];
+	int next, ns;
+};
+
+// Block sums of three values (all threads get them).
+__device__ __forceinline__ int3 block_total3(int x, int y, int z, int (*s)[LWARPS], int lane, int w) {
+	x = __reduce_add_sync(0xffffffffu, x);
+	y = __reduce_add_sync(0xffffffffu, y);
+	z = __reduce_add_sync(0xffffffffu, z);
+	__syncthreads();
+	if (lane == 0) {
+		s[0][w] = x;
+		s[1][w] = y;
+		s[2][w] = z;
+	}
+	__syncthreads();
+	int3 t = make_int3(0, 0, 0);
+#pragma unroll
+	for (int i = 0; i < LWARPS; i++) {
+		t.x += s[0][i];
+		t.y += s[1][i];
+		t.z += s[2][i];
+	}
+	return t;
+}
+
+// Positions of a tile's particles on the wrong side of the split point, by the block: warp w has the
+// ballots of its w-th sub particles, with lt_prev particles of the node below the midpoint in earlier tiles.  Before the
+// split point they are ranked from the node's left, after it from its right.  The warp that holds the
+// split point puts the node's number of swaps in *ns.
+__device__ __forceinline__ void tile_positions(const LevelArgs& a, LevelShared& sh, unsigned mine, int pbeg, int pend, int tb, int sub, int m, int lt_prev, int* ns, int lane,
+		int w) {
+	const int here = __reduce_add_sync(0xffffffffu, __popc(mine));
+	__syncthreads();
+	if (lane == 0) {
+		sh.sum[0][w] = here;
+	}
+	__syncthreads();
+	int lt = lt_prev;
+	for (int i = 0; i < w; i++) {
+		lt += sh.sum[0][i];
+	}
+	const int sb = tb + sub * w, n = min(sub, pend - sb);
+	if (n > 0) {
+		const int sp = pbeg + m, before = max(0, min(n, sp - sb));
+		const int l0 = pbeg + (sb - pbeg) - lt, after = m - lt - here, r0 = pbeg + after;
+		sub_wrong(mine, n, before, lane, [&](int k, int o) { a.posL[l0 + k] = sb + o; }, [&](int k, int o) { a.posR[r0 + k] = sb + o; });
+		// (the last warp, when nothing lies after the split point)
+		if ((sb <= sp && sp < sb + n) || (sp == pend && sb + n == pend)) {
+			const int right = __reduce_add_sync(0xffffffffu, __popc(mine & ~first_bits(before, 32 * lane)));
+			if (lane == 0) {
+				*ns = after + right;
+			}
+		}
+	}
+}
+
 __global__ void __launch_bounds__(LTPB, 2) k_tree_levels(const LevelArgs a) {
-	__shared__ uint16_t s_pos[LWARPS][WARP_NODE];
-	__shared__ int s_cnt[TILE_ROWS * LWARPS];
-	__shared__ int s_scan[3][LWARPS];
-	__shared__ int s_sum[2][LWARPS];
-	__shared__ int s_next;
+	__shared__ LevelShared sh;
 	const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
 	const unsigned lt_lane = (1u << lane) - 1u;
+	const int nblk = gridDim.x;
 	LevelCtl* ctl = a.ctl;
 	unsigned int round = 0;
 	int level = 0;
@@ -232,24 +389,24 @@ __global__ void __launch_bounds__(LTPB, 2) k_tree_levels(const LevelArgs a) {
 		lb = ctl->lb;
 		le = ctl->le;
 	} else {
-		const int64_t gt = blockIdx.x * (int64_t) LTPB + tid, gs = gridDim.x * (int64_t) LTPB;
+		const int64_t gt = blockIdx.x * (int64_t) LTPB + tid, gs = nblk * (int64_t) LTPB;
 		for (int64_t i = gt; i < a.n; i += gs) {
 			a.idx[i] = (int32_t) i;
 		}
 		// one root per box: node s covers the unit box and particles [off[s], off[s+1]), except that
 		// a single box starts at the active range
 		for (int64_t s = gt; s < a.nroot; s += gs) {
+			const double gb[6] = { 0.0, 0.0, 0.0, 1.0, 1.0, 1.0 };
 			NodeW r;
 			r.x = r.y = r.z = 0;
 			r.radius = 0.f;
 			r.pbeg = a.nroot == 1 ? (int32_t) a.pb : (int32_t) a.off[s];
 			r.pend = a.nroot == 1 ? (int32_t) a.n : (int32_t) a.off[s + 1];
 			r.child = -1;
-			r.flags = 1;
+			r.flags = classify(a, gb, r.pend - r.pbeg, 0);
 			a.nodes[s] = r;
-			for (int d = 0; d < 3; d++) {
-				a.gbox[6 * s + d] = 0.0;
-				a.gbox[6 * s + 3 + d] = 1.0;
+			for (int d = 0; d < 6; d++) {
+				a.gbox[6 * s + d] = gb[d];
 			}
 			a.key[s] = 1;
 			a.depth[s] = 0;
@@ -259,74 +416,82 @@ __global__ void __launch_bounds__(LTPB, 2) k_tree_levels(const LevelArgs a) {
 			return;
 		}
 	}
+	bool counts = false;  // the blocks' counts of this level's nodes are there
 	for (;; level++) {
 		const int64_t nl = le - lb;
-		const int64_t share = (nl + gridDim.x - 1) / gridDim.x;  // consecutive nodes of a block
+		const int64_t share = (nl + nblk - 1) / nblk;  // consecutive nodes of a block
 		const int64_t cb = lb + min(nl, share * blockIdx.x), ce = lb + min(nl, share * (blockIdx.x + 1));
-		// ---- leaf or split (tree.cpp:314-348), counted per block
-		int nsplit = 0, ntn = 0, ntile = 0;
-		for (int64_t ni = cb + tid; ni < ce; ni += LTPB) {
-			const int2 pr = *reinterpret_cast<const int2*>(&a.nodes[ni].pbeg);
-			const int nparts = pr.y - pr.x;
-			const double* gb = a.gbox + 6 * ni;
-			float box_r = 0.0f;
-			for (int dim = 0; dim < 3; dim++) {
-				const double h = 0.5 * (gb[3 + dim] - gb[dim]);
-				box_r += h * h;
+		const bool many = many_nodes(nl);
+		const int line = tile_line(nl), warp_line = warp_line_of(nl);
+		int4* blk = a.blk + (level & 1) * nblk;
+		int4* blk_next = a.blk + ((level + 1) & 1) * nblk;
+		if (!counts) {
+			int k0 = 0, k1 = 0, k2 = 0;
+			for (int64_t ni = cb + tid; ni < ce; ni += LTPB) {
+				const NodeW nd = a.nodes[ni];
+				const int3 k = counted(a, nd.flags, nd.pend - nd.pbeg, line);
+				k0 += k.x;
+				k1 += k.y;
+				k2 += k.z;
 			}
-			box_r = sqrtf(box_r);
-			const bool ewald_satisfied = (box_r < 0.25 * (a.theta / (1.0 + a.theta)) && box_r < 0.125 - 0.25 * a.hsoft);
-			bool split = nparts > a.bucket || (!ewald_satisfied && nparts > 0);
-			if (split && level >= MAX_DEPTH - 1) {
-				atomicOr(a.flags + 2, 1);
-				split = false;
+			const int3 t = block_total3(k0, k1, k2, sh.scan, lane, w);
+			if (tid == 0) {
+				blk[blockIdx.x] = make_int4(t.x, t.y, t.z, (int) cb);
 			}
-			const bool tiles = split && nparts > WARP_NODE;
-			a.nodes[ni].flags = split ? (tiles ? NODE_SPLIT | NODE_TILES : NODE_SPLIT) : 1;
-			nsplit += split;
-			ntn += tiles;
-			ntile += tiles ? (nparts + TILE - 1) / TILE : 0;
-		}
-		for (int o = 16; o; o >>= 1) {
-			nsplit += __shfl_xor_sync(0xffffffffu, nsplit, o);
-			ntn += __shfl_xor_sync(0xffffffffu, ntn, o);
-			ntile += __shfl_xor_sync(0xffffffffu, ntile, o);
-		}
-		if (lane == 0) {
-			s_scan[0][w] = nsplit;
-			s_scan[1][w] = ntn;
-			s_scan[2][w] = ntile;
-		}
-		__syncthreads();
-		if (tid == 0) {
-			int4 t = make_int4(0, 0, 0, 0);
-			for (int i = 0; i < LWARPS; i++) {
-				t.x += s_scan[0][i];
-				t.y += s_scan[1][i];
-				t.z += s_scan[2][i];
+			if (!grid_meet(ctl, round)) {
+				return;
 			}
-			a.blk[blockIdx.x] = t;
 		}
-		if (!grid_meet(ctl, round)) {
-			return;
-		}
-		// ---- totals of the level and of the blocks before this one (a warp: at most a few hundred)
+		// ---- totals of the level and of the nodes before this block's share: the ranges before it,
+		// and the part of the range the share begins in (nblk is at most the block's threads)
 		int base[3] = { 0, 0, 0 }, tot[3] = { 0, 0, 0 };
-		for (int i = lane; i < (int) gridDim.x; i += 32) {
-			const int4 t = __ldcg(a.blk + i);
-			const bool prev = i < (int) blockIdx.x;
-			tot[0] += t.x;
-			tot[1] += t.y;
-			tot[2] += t.z;
-			base[0] += prev ? t.x : 0;
-			base[1] += prev ? t.y : 0;
-			base[2] += prev ? t.z : 0;
-		}
-		for (int o = 16; o; o >>= 1) {
-			for (int q = 0; q < 3; q++) {
-				tot[q] += __shfl_xor_sync(0xffffffffu, tot[q], o);
-				base[q] += __shfl_xor_sync(0xffffffffu, base[q], o);
+		int part = 0x7fffffff;  // first node of the range that holds cb
+		{
+			int4 t = make_int4(0, 0, 0, 0x7fffffff);
+			int end = 0x7fffffff;
+			if (tid < nblk) {
+				t = __ldcg(blk + tid);
+				end = tid + 1 < nblk ? __ldcg(&blk[tid + 1].w) : (int) le;
 			}
+			const bool prev = end <= (int) cb;
+			int v[7] = { t.x, t.y, t.z, prev ? t.x : 0, prev ? t.y : 0, prev ? t.z : 0, t.w < (int) cb && end > (int) cb ? t.w : 0x7fffffff };
+			const int nw = (nblk + 31) / 32;
+			if (w < nw) {
+#pragma unroll
+				for (int q = 0; q < 7; q++) {
+					v[q] = q < 6 ? __reduce_add_sync(0xffffffffu, v[q]) : __reduce_min_sync(0xffffffffu, v[q]);
+				}
+			}
+			__syncthreads();
+			if (lane == 0 && w < nw) {
+#pragma unroll
+				for (int q = 0; q < 7; q++) {
+					sh.totals[q][w] = v[q];
+				}
+			}
+			__syncthreads();
+			for (int i = 0; i < nw; i++) {
+#pragma unroll
+				for (int q = 0; q < 3; q++) {
+					tot[q] += sh.totals[q][i];
+					base[q] += sh.totals[3 + q][i];
+				}
+				part = min(part, sh.totals[6][i]);
+			}
+		}
+		if (part < (int) cb) {
+			int k0 = 0, k1 = 0, k2 = 0;
+			for (int ni = part + tid; ni < (int) cb; ni += LTPB) {
+				const NodeW nd = a.nodes[ni];
+				const int3 k = counted(a, nd.flags, nd.pend - nd.pbeg, line);
+				k0 += k.x;
+				k1 += k.y;
+				k2 += k.z;
+			}
+			const int3 t = block_total3(k0, k1, k2, sh.scan, lane, w);
+			base[0] += t.x;
+			base[1] += t.y;
+			base[2] += t.z;
 		}
 		const int64_t next_le = le + 2 * (int64_t) tot[0];
 		if (next_le > a.node_cap) {
@@ -344,33 +509,55 @@ __global__ void __launch_bounds__(LTPB, 2) k_tree_levels(const LevelArgs a) {
 			ctl->start[level] = lb;
 			ctl->start[level + 1] = le;
 			ctl->level = level;
+			ctl->take[(level + 1) & 1] = 0;  // (the last level's takers are done)
 		}
-		// ---- children's indices in node order, tile nodes listed
+		if (tot[0] == 0) {
+			break;
+		}
+		const int first_child = (int) le + 2 * base[0];
+		const int next_line = tile_line(2 * (int64_t) tot[0]);
+		__syncthreads();
+		if (tid < 3) {
+			sh.tot[tid] = 0;
+		}
+		// one node by this warp
+		auto by_warp = [&](int64_t ni) {
+			const NodeW nd = a.nodes[ni];
+			if (nd.child < 0 || nd.pend - nd.pbeg > warp_line) {
+				return;
+			}
+			double xm;
+			const int xd = split_dim(a.gbox + 6 * ni, xm);
+			const int m = warp_partition(a, nd, xd == 0 ? a.x[0] : xd == 1 ? a.x[1] : a.x[2], fixed_from_double(xm), sh.pos[w], lane);
+			make_children(a, ni, nd, nd.pbeg + m, xd, xm, level, lane, next_line, sh.tot);
+		};
+		// ---- LTPB nodes at a time: children numbered in node order, then (few nodes) the partitions
 		for (int64_t n0 = cb; n0 < ce; n0 += LTPB) {
 			const int64_t ni = n0 + tid;
-			const int f = ni < ce ? a.nodes[ni].flags : 1;
-			const int sp = (f & NODE_SPLIT) != 0, tn = (f & NODE_TILES) != 0;
-			int nt = 0;
-			if (tn) {
-				const int2 pr = *reinterpret_cast<const int2*>(&a.nodes[ni].pbeg);
-				nt = (pr.y - pr.x + TILE - 1) / TILE;
+			int f = 1, nparts = 0;
+			if (ni < ce) {
+				const NodeW nd = a.nodes[ni];
+				f = nd.flags;
+				nparts = nd.pend - nd.pbeg;
 			}
-			int inc = nt;
-			for (int o = 1; o < 32; o <<= 1) {
-				const int t = __shfl_up_sync(0xffffffffu, inc, o);
-				inc += lane >= o ? t : 0;
-			}
-			const unsigned ms = __ballot_sync(0xffffffffu, sp), mt = __ballot_sync(0xffffffffu, tn);
+			const int3 k = counted(a, f, nparts, line);
+			const int inc = lane_scan(k.z, lane);
+			const unsigned ms = __ballot_sync(0xffffffffu, k.x), mt = __ballot_sync(0xffffffffu, k.y);
+			const unsigned mb = __ballot_sync(0xffffffffu, k.x && !k.y && nparts > warp_line);
 			__syncthreads();
 			if (lane == 31) {
-				s_scan[0][w] = __popc(ms);
-				s_scan[1][w] = __popc(mt);
-				s_scan[2][w] = inc;
+				sh.scan[0][w] = __popc(ms);
+				sh.scan[1][w] = __popc(mt);
+				sh.scan[2][w] = inc;
+				sh.mask[w] = mb;
+			}
+			if (tid == 0) {
+				sh.next = 0;
 			}
 			__syncthreads();
 			int e0 = base[0], e1 = base[1], e2 = base[2];
 			for (int i = 0; i < LWARPS; i++) {
-				const int q0 = s_scan[0][i], q1 = s_scan[1][i], q2 = s_scan[2][i];
+				const int q0 = sh.scan[0][i], q1 = sh.scan[1][i], q2 = sh.scan[2][i];
 				e0 += i < w ? q0 : 0;
 				e1 += i < w ? q1 : 0;
 				e2 += i < w ? q2 : 0;
@@ -378,224 +565,152 @@ __global__ void __launch_bounds__(LTPB, 2) k_tree_levels(const LevelArgs a) {
 				base[1] += q1;
 				base[2] += q2;
 			}
-			if (sp) {
+			if (k.x) {
+				// (the flags stay: another block may still be counting up to its share)
 				a.nodes[ni].child = (int32_t) (le + 2 * (int64_t) (e0 + __popc(ms & lt_lane)));
-				a.nodes[ni].flags = 0;
 			}
-			if (tn) {
+			if (k.y) {
 				TileNode t;
 				t.node = (int32_t) ni;
-				t.t0 = e2 + inc - nt;
-				t.nt = nt;
+				t.t0 = e2 + inc - k.z;
+				t.nt = k.z;
 				t.m = t.nswap = 0;
 				a.tnode[e1 + __popc(mt & lt_lane)] = t;
-				for (int q = 0; q < nt; q++) {
-					a.tile_of[t.t0 + q] = e1 + __popc(mt & lt_lane);
+			}
+			for (unsigned q = mt; q; q &= q - 1) {
+				const int src = __ffs(q) - 1;
+				const int t0 = __shfl_sync(0xffffffffu, e2 + inc - k.z, src), nt = __shfl_sync(0xffffffffu, k.z, src);
+				for (int i = lane; i < nt; i += 32) {
+					a.tile_of[t0 + i] = e1 + __popc(mt & ((1u << src) - 1u));
 				}
 			}
-		}
-		// ---- nodes of at most WARP_NODE particles: a warp each, taken from the block's share
-		if (tid == 0) {
-			s_next = 0;
-		}
-		__syncthreads();
-		for (;;) {
-			int k = 0;
-			if (lane == 0) {
-				k = atomicAdd(&s_next, 1);
-			}
-			const int64_t ni = cb + __shfl_sync(0xffffffffu, k, 0);
-			if (ni >= ce) {
-				break;
-			}
-			const NodeW nd = a.nodes[ni];
-			if (nd.child < 0 || nd.pend - nd.pbeg > WARP_NODE) {
+			if (many) {
 				continue;
 			}
-			double xm;
-			const int xd = split_dim(a.gbox + 6 * ni, xm);
-			const int m = warp_partition(a, nd, xd == 0 ? a.x[0] : xd == 1 ? a.x[1] : a.x[2], fixed_from_double(xm), s_pos[w], lane);
-			make_children(a, ni, nd, nd.pbeg + m, xd, xm, level, lane);
-		}
-		if (tot[2] > 0) {
-			if (!grid_meet(ctl, round)) {
-				return;
-			}
-			// ---- larger nodes, tile by tile: particles below the midpoint
-			for (int t = blockIdx.x; t < tot[2]; t += gridDim.x) {
-				const TileNode tn = a.tnode[a.tile_of[t]];
-				const int2 pr = *reinterpret_cast<const int2*>(&a.nodes[tn.node].pbeg);
-				double xm;
-				const int xd = split_dim(a.gbox + 6 * (int64_t) tn.node, xm);
-				const uint32_t* x = xd == 0 ? a.x[0] : xd == 1 ? a.x[1] : a.x[2];
-				const uint32_t xf = fixed_from_double(xm);
-				const int p0 = pr.x + (t - tn.t0) * TILE + tid;
-				int c = 0;
-#pragma unroll
-				for (int j = 0; j < TILE_ROWS; j++) {
-					const int p = p0 + j * LTPB;
-					c += p < pr.y && x[min(p, pr.y - 1)] < xf;
-				}
-				c = __reduce_add_sync(0xffffffffu, c);
-				if (lane == 0) {
-					s_sum[0][w] = c;
-				}
-				__syncthreads();
-				if (tid == 0) {
-					int s = 0;
-					for (int i = 0; i < LWARPS; i++) {
-						s += s_sum[0][i];
+			__syncthreads();
+			// nodes of at most BLOCK_LINE particles, one after the other by the block
+			for (int i = 0; i < LWARPS; i++) {
+				for (unsigned q = sh.mask[i]; q; q &= q - 1) {
+					const int64_t bi = n0 + 32 * i + __ffs(q) - 1;
+					const NodeW nd = a.nodes[bi];
+					double xm;
+					const int xd = split_dim(a.gbox + 6 * bi, xm);
+					const uint32_t* x = xd == 0 ? a.x[0] : xd == 1 ? a.x[1] : a.x[2];
+					const int sb = nd.pbeg + BLOCK_SUB * w;
+					const unsigned mine = sb < nd.pend ? sub_below(x + sb, min(BLOCK_SUB, nd.pend - sb), fixed_from_double(xm), lane) : 0u;
+					const int m = block_total3(__popc(mine), 0, 0, sh.scan, lane, w).x;
+					tile_positions(a, sh, mine, nd.pbeg, nd.pend, nd.pbeg, BLOCK_SUB, m, 0, &sh.ns, lane, w);
+					__syncthreads();
+					const int ns = sh.ns;
+					for (int p = tid; p < ns; p += LTPB) {
+						swap_particles(a, a.posL[nd.pbeg + p], a.posR[nd.pbeg + p]);
 					}
-					a.tile_lt[t] = s;
+					if (w == 0) {
+						make_children(a, bi, nd, nd.pbeg + m, xd, xm, level, lane, next_line, sh.tot);
+					}
 				}
-				__syncthreads();
 			}
+			// the others: a warp each, taken from the block's
+			const int have = (int) min((int64_t) LTPB, ce - n0);
+			for (;;) {
+				int j = 0;
+				if (lane == 0) {
+					j = atomicAdd(&sh.next, 1);
+				}
+				j = __shfl_sync(0xffffffffu, j, 0);
+				if (j >= have) {
+					break;
+				}
+				by_warp(n0 + j);
+			}
+		}
+		counts = !many && tot[2] == 0;
+		if (counts) {
+			// the children this block made are consecutive: their counts are the next level's
+			__syncthreads();
+			if (tid == 0) {
+				blk_next[blockIdx.x] = make_int4(sh.tot[0], sh.tot[1], sh.tot[2], first_child);
+			}
+		} else {
 			if (!grid_meet(ctl, round)) {
 				return;
 			}
-			// positions of the particles on the wrong side of the split point: before it ranked from the
-			// node's left, after it from the node's right.  Earlier tiles hold only particles before a
-			// particle on the left, later ones only particles after one on the right, so the counts
-			// below the midpoint of whole tiles give both ranks.
-			for (int t = blockIdx.x; t < tot[2]; t += gridDim.x) {
+			// ---- larger nodes, tile by tile: ballots and counts of the particles below the midpoint
+			for (int t = blockIdx.x; t < tot[2]; t += nblk) {
 				const int ti = a.tile_of[t];
 				const TileNode tn = a.tnode[ti];
 				const int2 pr = *reinterpret_cast<const int2*>(&a.nodes[tn.node].pbeg);
 				double xm;
 				const int xd = split_dim(a.gbox + 6 * (int64_t) tn.node, xm);
 				const uint32_t* x = xd == 0 ? a.x[0] : xd == 1 ? a.x[1] : a.x[2];
-				const uint32_t xf = fixed_from_double(xm);
-				const int tb = pr.x + (t - tn.t0) * TILE, te = min(tb + TILE, pr.y);
-				unsigned below = 0;  // bit j: row j's particle of this thread
-#pragma unroll
-				for (int j = 0; j < TILE_ROWS; j++) {
-					const int p = tb + j * LTPB + tid;
-					below |= (unsigned) (p < te && x[min(p, te - 1)] < xf) << j;
+				const int sb = pr.x + ((t - tn.t0) * LWARPS + w) * a.sub;
+				const unsigned mine = sb < pr.y ? sub_below(x + sb, min(a.sub, pr.y - sb), fixed_from_double(xm), lane) : 0u;
+				if (sb < pr.y) {
+					a.tile_mask[32 * mask_row(a, pr.x, ti, (t - tn.t0) * LWARPS + w) + lane] = mine;
 				}
-				int all = 0, prev = 0;
-				for (int q = tid; q < tn.nt; q += LTPB) {
-					const int c = __ldcg(a.tile_lt + tn.t0 + q);
-					all += c;
-					prev += q < t - tn.t0 ? c : 0;
-				}
-				all = __reduce_add_sync(0xffffffffu, all);
-				prev = __reduce_add_sync(0xffffffffu, prev);
-				if (lane == 0) {
-					s_sum[0][w] = all;
-					s_sum[1][w] = prev;
-				}
-				__syncthreads();
-				int m = 0, lt_prev = 0;
-				for (int i = 0; i < LWARPS; i++) {
-					m += s_sum[0][i];
-					lt_prev += s_sum[1][i];
-				}
-				const int sp = pr.x + m;
-				unsigned wrong = 0;
-				int right = 0;  // wrong ones after the split point
-#pragma unroll
-				for (int j = 0; j < TILE_ROWS; j++) {
-					const int p = tb + j * LTPB + tid;
-					const bool lt = below >> j & 1u;
-					const bool bad = p < te && (p < sp ? !lt : lt);
-					const unsigned mk = __ballot_sync(0xffffffffu, bad);
-					wrong |= (unsigned) bad << j;
-					right += bad && p >= sp;
-					if (lane == 0) {
-						s_cnt[j * LWARPS + w] = __popc(mk);
-					}
-				}
-				__syncthreads();
-				// prefix of the rows' warps in particle order, by every warp for itself
-				int mybase[TILE_ROWS], run = 0;
-				{
-					constexpr int PER = TILE_ROWS * LWARPS / 32;
-					int c[PER], s = 0;
-					for (int i = 0; i < PER; i++) {
-						c[i] = s_cnt[lane * PER + i];
-						s += c[i];
-					}
-					int inc = s;
-					for (int o = 1; o < 32; o <<= 1) {
-						const int v = __shfl_up_sync(0xffffffffu, inc, o);
-						inc += lane >= o ? v : 0;
-					}
-					run = __shfl_sync(0xffffffffu, inc, 31);
-					int ex[PER];
-					int e = inc - s;
-					for (int i = 0; i < PER; i++) {
-						ex[i] = e;
-						e += c[i];
-					}
-#pragma unroll
-					for (int j = 0; j < TILE_ROWS; j++) {
-						const int q = j * LWARPS + w;
-						int v = 0;
-						for (int i = 0; i < PER; i++) {
-							const int u = __shfl_sync(0xffffffffu, ex[i], q / PER);
-							v = q % PER == i ? u : v;
-						}
-						mybase[j] = v;
-					}
-				}
-				right = __reduce_add_sync(0xffffffffu, right);
-				__syncthreads();
-				if (lane == 0) {
-					s_sum[0][w] = right;
-				}
-				__syncthreads();
-				int nright = 0;
-				for (int i = 0; i < LWARPS; i++) {
-					nright += s_sum[0][i];
-				}
-				const int lt_tile = __ldcg(a.tile_lt + t);
-				const int after = m - lt_prev - lt_tile;  // below the midpoint in later tiles
-				const int leftbase = (tb - pr.x) - lt_prev;
-#pragma unroll
-				for (int j = 0; j < TILE_ROWS; j++) {
-					const bool bad = wrong >> j & 1u;
-					const unsigned mk = __ballot_sync(0xffffffffu, bad);
-					if (bad) {
-						const int p = tb + j * LTPB + tid;
-						const int e = mybase[j] + __popc(mk & lt_lane);
-						if (p < sp) {
-							a.posL[pr.x + leftbase + e] = p;
-						} else {
-							a.posR[pr.x + after + (run - e - 1)] = p;
-						}
-					}
-				}
+				const int c = block_total3(__popc(mine), 0, 0, sh.scan, lane, w).x;
 				if (tid == 0) {
-					if (t == tn.t0) {
-						a.tnode[ti].m = m;
+					a.tile_lt[t] = c;
+				}
+			}
+			if (many) {
+				for (;;) {
+					unsigned int j = 0;
+					if (lane == 0) {
+						j = atomicAdd(&ctl->take[level & 1], (unsigned int) TAKE);
 					}
-					// the tile that holds the split point (or the last one, when nothing lies after it)
-					if ((tb <= sp && sp < te) || (sp == pr.y && te == pr.y)) {
-						a.tnode[ti].nswap = after + nright;
+					j = __shfl_sync(0xffffffffu, j, 0);
+					if ((int64_t) j >= nl) {
+						break;
+					}
+					for (int64_t q = j; q < min(nl, (int64_t) j + TAKE); q++) {
+						by_warp(lb + q);
 					}
 				}
-				__syncthreads();
 			}
-			if (!grid_meet(ctl, round)) {
-				return;
-			}
-			for (int t = blockIdx.x; t < tot[2]; t += gridDim.x) {
-				const TileNode* tp = a.tnode + a.tile_of[t];
-				const int node = tp->node, t0 = tp->t0;
-				const int m = __ldcg(&tp->m), ns = __ldcg(&tp->nswap);
-				const int pbeg = a.nodes[node].pbeg;
-				for (int k = (t - t0) * TILE + tid; k < min(ns, (t - t0 + 1) * TILE); k += LTPB) {
-					swap_particles(a, __ldcg(a.posL + pbeg + k), __ldcg(a.posR + pbeg + k));
+			if (tot[2] > 0) {
+				if (!grid_meet(ctl, round)) {
+					return;
 				}
-				if (t == t0 && w == 0) {
-					double xm;
-					const int xd = split_dim(a.gbox + 6 * (int64_t) node, xm);
-					make_children(a, node, a.nodes[node], pbeg + m, xd, xm, level, lane);
+				// positions of the particles on the wrong side of the split point.  Earlier tiles hold only
+				// particles before a particle on the left, later ones only particles after one on the right,
+				// so the counts below the midpoint of whole tiles give both ranks.
+				for (int t = blockIdx.x; t < tot[2]; t += nblk) {
+					const int ti = a.tile_of[t];
+					const TileNode tn = a.tnode[ti];
+					const int2 pr = *reinterpret_cast<const int2*>(&a.nodes[tn.node].pbeg);
+					const int sub = (t - tn.t0) * LWARPS + w;
+					const unsigned mine = pr.x + a.sub * sub < pr.y ? __ldcg(a.tile_mask + 32 * mask_row(a, pr.x, ti, sub) + lane) : 0u;
+					int all = 0, prev = 0;
+					for (int q = tid; q < tn.nt; q += LTPB) {
+						const int c = __ldcg(a.tile_lt + tn.t0 + q);
+						all += c;
+						prev += q < t - tn.t0 ? c : 0;
+					}
+					const int3 s = block_total3(all, prev, 0, sh.scan, lane, w);
+					tile_positions(a, sh, mine, pr.x, pr.y, pr.x + (t - tn.t0) * LWARPS * a.sub, a.sub, s.x, s.y, &a.tnode[ti].nswap, lane, w);
+					if (tid == 0 && t == tn.t0) {
+						a.tnode[ti].m = s.x;
+					}
+				}
+				if (!grid_meet(ctl, round)) {
+					return;
+				}
+				for (int t = blockIdx.x; t < tot[2]; t += nblk) {
+					const TileNode* tp = a.tnode + a.tile_of[t];
+					const int node = tp->node, t0 = tp->t0;
+					const int m = __ldcg(&tp->m), ns = __ldcg(&tp->nswap);
+					const int pbeg = a.nodes[node].pbeg, tile = a.sub * LWARPS;
+					for (int k = (t - t0) * tile + tid; k < min(ns, (t - t0 + 1) * tile); k += LTPB) {
+						swap_particles(a, __ldcg(a.posL + pbeg + k), __ldcg(a.posR + pbeg + k));
+					}
+					if (t == t0 && w == 0) {
+						double xm;
+						const int xd = split_dim(a.gbox + 6 * (int64_t) node, xm);
+						make_children(a, node, a.nodes[node], pbeg + m, xd, xm, level, lane, next_line, sh.tot);
+					}
 				}
 			}
-		}
-		if (tot[0] == 0) {
-			break;
 		}
 		lb = le;
 		le = next_le;
@@ -644,8 +759,141 @@ __device__ __forceinline__ T warp_sum(T v) {
 
 constexpr int UTPB = 128;
 
-// A warp per node (tree.cpp:351-571): tight box, expansion centre and radius, multipole (P2M of
-// the particles for a leaf, M2M of the two children in double for an interior node).
+// Sums of N doubles per lane over the warp: afterwards lane l has the sums of entries k with
+// k % 32 == l in out[k / 32].  Halves of the entries change places at each step, so that the warp
+// moves N values instead of 5 N; the pairs added are those of a butterfly over lane distances
+// 16, 8, 4, 2, 1.
+template<int N, int O>
+struct WarpScatterSum {
+	static constexpr int HALF = (N + 1) / 2;
+	static __device__ __forceinline__ void run(double* v, int lane) {
+		const bool hi = lane & O;
+		double w[HALF];
+#pragma unroll
+		for (int i = 0; i < HALF; i++) {
+			const double up = HALF + i < N ? v[HALF + i] : 0.0;
+			w[i] = (hi ? up : v[i]) + __shfl_xor_sync(0xffffffffu, hi ? v[i] : up, O);
+		}
+#pragma unroll
+		for (int i = 0; i < HALF; i++) {
+			v[i] = w[i];
+		}
+		if constexpr (O > 1) {
+			WarpScatterSum<HALF, O / 2>::run(v, lane);
+		}
+	}
+	// entry that slot `i` of a lane holds after the steps from distance O down
+	static __device__ __forceinline__ int entry(int i, int lane) {
+		int k = i;
+		if constexpr (O > 1) {
+			k = WarpScatterSum<HALF, O / 2>::entry(i, lane);
+		}
+		return k >= HALF || k < 0 ? -1 : ((lane & O) ? (HALF + k < N ? HALF + k : -1) : k);
+	}
+	static constexpr int slots() {
+		if constexpr (O > 1) {
+			return WarpScatterSum<HALF, O / 2>::slots();
+		} else {
+			return HALF;
+		}
+	}
+};
+
+// All leaves of the tree, a warp each (tree.cpp:498-571): tight box, centre, radius and the
+// particles' multipole, summed in double.  The leaves need nothing of one another, so they run in one
+// launch and not level by level; the warp's 37 sums are scattered over its lanes instead of made by
+// every lane (370 shuffles before).
+template<class Ops>
+__global__ void __launch_bounds__(UTPB) k_leaf_moments(int64_t nn, NodeW* nodes, int32_t* nbox, float* multi, double* tbox, const double* gbox, const uint32_t* x0,
+		const uint32_t* x1, const uint32_t* x2) {
+	constexpr int NM = Ops::NMULT;
+	using Sum = WarpScatterSum<NM, 16>;
+	const uint32_t* xs[3] = { x0, x1, x2 };
+	const int lane = threadIdx.x & 31;
+	const int64_t gw = (blockIdx.x * (int64_t) blockDim.x + threadIdx.x) >> 5;
+	const int64_t nw = ((int64_t) gridDim.x * blockDim.x) >> 5;
+	for (int64_t ni = gw; ni < nn; ni += nw) {
+		const NodeW nd = nodes[ni];
+		if (nd.child >= 0) {
+			continue;
+		}
+		const double* gb = gbox + 6 * ni;
+		double mn[3], mx[3];
+		for (int d = 0; d < 3; d++) {
+			mn[d] = gb[3 + d];
+			mx[d] = gb[d];
+		}
+		for (int p = nd.pbeg + lane; p < nd.pend; p += 32) {
+			for (int d = 0; d < 3; d++) {
+				const double xx = fixed_to_double(xs[d][p]);
+				mx[d] = fmax(mx[d], xx);
+				mn[d] = fmin(mn[d], xx);
+			}
+		}
+		for (int d = 0; d < 3; d++) {
+			mn[d] = warp_min(mn[d]);
+			mx[d] = warp_max(mx[d]);
+		}
+		double Xc[3];
+		for (int d = 0; d < 3; d++) {
+			Xc[d] = (mx[d] + mn[d]) * 0.5;
+		}
+		double r = 0.0;
+		for (int p = nd.pbeg + lane; p < nd.pend; p += 32) {
+			double this_radius = 0.0;
+			for (int d = 0; d < 3; d++) {
+				const double dx = fixed_to_double(xs[d][p]) - Xc[d];
+				this_radius += dx * dx;
+			}
+			r = fmax(r, this_radius);
+		}
+		r = warp_max(r);
+		// P2M about fixed32(Xc), summed in double
+		uint32_t Y[3];
+		for (int d = 0; d < 3; d++) {
+			Y[d] = fixed_from_double(Xc[d]);
+		}
+		double M[NM];
+#pragma unroll
+		for (int k = 0; k < NM; k++) {
+			M[k] = 0.0;
+		}
+		for (int p = nd.pbeg + lane; p < nd.pend; p += 32) {
+			float m[NM];
+			Ops::p2m(m, fixed_dist(x0[p], Y[0]), fixed_dist(x1[p], Y[1]), fixed_dist(x2[p], Y[2]));
+#pragma unroll
+			for (int k = 0; k < NM; k++) {
+				M[k] += (double) m[k];
+			}
+		}
+		Sum::run(M, lane);
+		if (lane == 0) {
+			NodeW o = nd;
+			o.x = Y[0];
+			o.y = Y[1];
+			o.z = Y[2];
+			o.radius = (float) sqrt(r);
+			nodes[ni] = o;
+		}
+		if (lane < 3) {
+			const double lo = lane == 0 ? mn[0] : lane == 1 ? mn[1] : mn[2], hi = lane == 0 ? mx[0] : lane == 1 ? mx[1] : mx[2];
+			tbox[6 * ni + lane] = lo;
+			tbox[6 * ni + 3 + lane] = hi;
+			nbox[6 * ni + lane] = range_fixed_from_double(lo);
+			nbox[6 * ni + 3 + lane] = range_fixed_from_double(hi);
+		}
+#pragma unroll
+		for (int i = 0; i < Sum::slots(); i++) {
+			const int k = Sum::entry(i, lane);
+			if (k >= 0) {
+				multi[NMULT_STRIDE * ni + k] = (float) M[i];
+			}
+		}
+	}
+}
+
+// The interior nodes of one level, a warp each (tree.cpp:351-497): union of the children's tight boxes,
+// expansion centre and radius, M2M of the two children in double.
 template<class Ops>
 __global__ void __launch_bounds__(UTPB) k_upsweep(int64_t lb, int64_t le, NodeW* nodes, int32_t* nbox, float* multi, double* tbox, const double* gbox,
 		const uint32_t* x0, const uint32_t* x1, const uint32_t* x2, int bucket) {
@@ -659,77 +907,9 @@ __global__ void __launch_bounds__(UTPB) k_upsweep(int64_t lb, int64_t le, NodeW*
 		const int nparts = nd.pend - nd.pbeg;
 		const double* gb = gbox + 6 * ni;
 		if (nd.child < 0) {
-			// ---- leaf (tree.cpp:498-571)
-			double mn[3], mx[3];
-			for (int d = 0; d < 3; d++) {
-				mn[d] = gb[3 + d];
-				mx[d] = gb[d];
-			}
-			for (int p = nd.pbeg + lane; p < nd.pend; p += 32) {
-				for (int d = 0; d < 3; d++) {
-					const double xx = fixed_to_double(xs[d][p]);
-					mx[d] = fmax(mx[d], xx);
-					mn[d] = fmin(mn[d], xx);
-				}
-			}
-			for (int d = 0; d < 3; d++) {
-				mn[d] = warp_min(mn[d]);
-				mx[d] = warp_max(mx[d]);
-			}
-			double Xc[3];
-			for (int d = 0; d < 3; d++) {
-				Xc[d] = (mx[d] + mn[d]) * 0.5;
-			}
-			double r = 0.0;
-			for (int p = nd.pbeg + lane; p < nd.pend; p += 32) {
-				double this_radius = 0.0;
-				for (int d = 0; d < 3; d++) {
-					const double dx = fixed_to_double(xs[d][p]) - Xc[d];
-					this_radius += dx * dx;
-				}
-				r = fmax(r, this_radius);
-			}
-			r = warp_max(r);
-			// P2M about fixed32(Xc), summed in double
-			uint32_t Y[3];
-			for (int d = 0; d < 3; d++) {
-				Y[d] = fixed_from_double(Xc[d]);
-			}
-			double M[NM];
-			for (int k = 0; k < NM; k++) {
-				M[k] = 0.0;
-			}
-			for (int p = nd.pbeg + lane; p < nd.pend; p += 32) {
-				float m[NM];
-				Ops::p2m(m, fixed_dist(x0[p], Y[0]), fixed_dist(x1[p], Y[1]), fixed_dist(x2[p], Y[2]));
-				for (int k = 0; k < NM; k++) {
-					M[k] += (double) m[k];
-				}
-			}
-			for (int k = 0; k < NM; k++) {
-				M[k] = warp_sum(M[k]);
-			}
-			if (lane == 0) {
-				NodeW o = nd;
-				o.x = Y[0];
-				o.y = Y[1];
-				o.z = Y[2];
-				o.radius = (float) sqrt(r);
-				nodes[ni] = o;
-				for (int d = 0; d < 3; d++) {
-					tbox[6 * ni + d] = mn[d];
-					tbox[6 * ni + 3 + d] = mx[d];
-					nbox[6 * ni + d] = range_fixed_from_double(mn[d]);
-					nbox[6 * ni + 3 + d] = range_fixed_from_double(mx[d]);
-				}
-			}
-#pragma unroll
-			for (int k = 0; k < NM; k++) {
-				if (lane == (k & 31)) {
-					multi[NMULT_STRIDE * ni + k] = (float) M[k];
-				}
-			}
-		} else {
+			continue;
+		}
+		{
 			// ---- interior node (tree.cpp:351-497)
 			const int64_t L = nd.child, R = nd.child + 1;
 			const NodeW nl = nodes[L], nr = nodes[R];
@@ -769,6 +949,7 @@ __global__ void __launch_bounds__(UTPB) k_upsweep(int64_t lb, int64_t le, NodeW*
 					Xc1[d] = 0.5 * (bb[d] + be[d]);
 					xc[d] = fixed_from_double(Xc1[d]);
 				}
+#pragma unroll 4
 				for (int p = nd.pbeg + lane; p < nd.pend; p += 32) {
 					const float dx = fixed_dist(x0[p], xc[0]);
 					const float dy = fixed_dist(x1[p], xc[1]);
@@ -947,12 +1128,14 @@ ct_status tree_build_t(Ctx* c, Box* b, const ct_tree_params* p) {
 	la.idx = (int32_t*) scratch(c, 0, sizeof(int32_t) * n, &s1);
 	la.posL = (int32_t*) scratch(c, 1, sizeof(int32_t) * n, &s1);
 	la.posR = (int32_t*) scratch(c, 2, sizeof(int32_t) * n, &s1);
-	// nodes in tiles hold more than WARP_NODE particles each
-	const int64_t max_tn = np / WARP_NODE + 1, max_tiles = np / TILE + max_tn + 1;
+	la.sub = np > 2 * (int64_t) c->nsm * SUB * LWARPS ? SUB : BLOCK_SUB;
+	// nodes in tiles hold more than WARP_FEW particles each
+	const int64_t max_tn = np / WARP_FEW + 1, max_tiles = np / (la.sub * LWARPS) + max_tn + 1;
 	la.tnode = (TileNode*) scratch(c, 3, sizeof(TileNode) * max_tn, &s1);
 	la.tile_of = (int32_t*) scratch(c, 4, sizeof(int32_t) * max_tiles, &s1);
 	la.tile_lt = (int32_t*) scratch(c, 5, sizeof(int32_t) * max_tiles, &s1);
-	la.blk = (int4*) scratch(c, 6, sizeof(int4) * c->nsm, &s1);
+	la.tile_mask = (uint32_t*) scratch(c, 8, sizeof(uint32_t) * 32 * (np / la.sub + max_tn + 2), &s1);
+	la.blk = (int4*) scratch(c, 6, sizeof(int4) * 2 * nblk, &s1);
 	la.ctl = (LevelCtl*) scratch(c, 7, sizeof(LevelCtl), &s1);
 	CT_TRY(s1);
 	for (int d = 0; d < 3; d++) {
@@ -1013,15 +1196,18 @@ ct_status tree_build_t(Ctx* c, Box* b, const ct_tree_params* p) {
 			k_gather_particles<<<grid_for(c, np, 256), 256, 0, st>>>(pb, n, perm, t0, t1, t2, tr, b->v[0], b->v[1], b->v[2], b->rung);
 		}
 	}
-	// upsweep, deepest level first
+	// upsweep: the leaves at once, then the interior nodes, deepest level first
+	c->launches++;
+	k_leaf_moments<Ops><<<grid_for(c, 32 * b->nnodes, UTPB, 16), UTPB, 0, st>>>(b->nnodes, b->nodes, b->nbox, b->multi, b->tbox, b->gbox, b->x[0], b->x[1],
+			b->x[2]);
 	for (int k = (int) levels.size() - 2; k >= 0; k--) {
 		const int64_t a = levels[k], e = levels[k + 1];
-		if (e > a) {
-			c->launches++;
-			k_upsweep<Ops><<<(int) std::min<int64_t>((e - a + UTPB / 32 - 1) / (UTPB / 32), (int64_t) c->nsm * 16), UTPB, 0, st>>>(a, e, b->nodes, b->nbox,
-					b->multi, b->tbox, b->gbox,
-					b->x[0], b->x[1], b->x[2], p->bucket);
+		if (k + 1 == (int) levels.size() - 1) {
+			continue;  // the deepest level is all leaves
 		}
+		c->launches++;
+		k_upsweep<Ops><<<(int) std::min<int64_t>((e - a + UTPB / 32 - 1) / (UTPB / 32), (int64_t) c->nsm * 16), UTPB, 0, st>>>(a, e, b->nodes, b->nbox, b->multi,
+				b->tbox, b->gbox, b->x[0], b->x[1], b->x[2], p->bucket);
 	}
 	CT_CUDA(c, cudaGetLastError());
 	CT_CUDA(c, cudaMemcpyAsync(h_tot, c->d_flags, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
