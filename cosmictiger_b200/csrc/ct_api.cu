@@ -8,6 +8,7 @@
 #include <new>
 
 #include "ct_internal.cuh"
+#include "ct_partition.cuh"
 #include "fmm_p7.h"
 
 namespace ct {
@@ -131,29 +132,91 @@ __global__ void __launch_bounds__(256) k_drift(int64_t b, int64_t n, uint32_t* _
 }
 
 // ---- rung partition (src/particles.cpp:1029-1076): same exact permutation rule as the tree
-// partition, with predicate rung < minrung on the left.
-__global__ void k_rung_flags(int64_t b, int64_t e, const int8_t* rung, int minrung, int* lt) {
-	for (int64_t i = b + blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < e; i += (int64_t) gridDim.x * blockDim.x) {
-		lt[i - b] = rung[i] < minrung;
+// partition, with predicate rung < minrung on the left.  Three passes over the rungs' ballots: a warp
+// takes 1,024 particles (one word a lane), a block 8,192.  Seven integer arrays a particle and six
+// library scans and sums took 0.33 ms of the 0.57 ms for 16.8M particles, and 15 launches.
+constexpr int RUNG_TPB = 256;
+constexpr int RUNG_SUB = 1024;
+constexpr int RUNG_TILE = RUNG_SUB * RUNG_TPB / 32;
+
+__device__ __forceinline__ int rung_block_sum(int v, int* s) {
+	v = __reduce_add_sync(0xffffffffu, v);
+	__syncthreads();
+	if ((threadIdx.x & 31) == 0) {
+		s[threadIdx.x >> 5] = v;
 	}
-}
-__global__ void k_rung_mis(int64_t b, int64_t e, const int* lt, const int* m, int* misL, int* misR) {
-	const int64_t s = b + *m;
-	for (int64_t i = b + blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < e; i += (int64_t) gridDim.x * blockDim.x) {
-		const int f = lt[i - b];
-		misL[i - b] = (i < s) && !f;
-		misR[i - b] = (i >= s) && f;
+	__syncthreads();
+	int t = 0;
+	for (int i = 0; i < RUNG_TPB / 32; i++) {
+		t += s[i];
 	}
+	return t;
 }
-__global__ void k_rung_pos(int64_t b, int64_t e, const int* misL, const int* misR, const int* exL, const int* exR, const int* totR, int* posL,
-		int* posR) {
-	for (int64_t i = b + blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < e; i += (int64_t) gridDim.x * blockDim.x) {
-		const int64_t k = i - b;
-		if (misL[k]) {
-			posL[exL[k]] = (int) i;
+
+// Ballots of rung < minrung (word c of a SUB: particles 32 c ..) and their number per tile.
+__global__ void __launch_bounds__(RUNG_TPB) k_rung_ballots(int64_t b, int64_t e, const int8_t* __restrict__ rung, int minrung, uint32_t* __restrict__ mask,
+		int* __restrict__ lt) {
+	__shared__ int s_sum[RUNG_TPB / 32];
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+	const int64_t sb = b + blockIdx.x * (int64_t) RUNG_TILE + w * RUNG_SUB;
+	unsigned mine = 0;
+	for (int c0 = 0; c0 < 32 && sb + 32 * c0 < e; c0 += 8) {
+		int v[8];
+#pragma unroll
+		for (int j = 0; j < 8; j++) {
+			const int64_t p = sb + 32 * (c0 + j) + lane;
+			v[j] = p < e ? rung[p] : 127;
 		}
-		if (misR[k]) {
-			posR[*totR - 1 - exR[k]] = (int) i;
+#pragma unroll
+		for (int j = 0; j < 8; j++) {
+			const unsigned m = __ballot_sync(0xffffffffu, sb + 32 * (c0 + j) + lane < e && v[j] < minrung);
+			mine = lane == c0 + j ? m : mine;
+		}
+	}
+	mask[(blockIdx.x * (RUNG_TPB / 32) + w) * 32 + lane] = mine;
+	const int t = rung_block_sum(__popc(mine), s_sum);
+	if (threadIdx.x == 0) {
+		lt[blockIdx.x] = t;
+	}
+}
+
+// Positions of the particles on the wrong side, ranked from the left before the split point and from
+// the right after it; tot[0]: particles below minrung, tot[1]: swaps.
+__global__ void __launch_bounds__(RUNG_TPB) k_rung_pos(int64_t b, int64_t e, const uint32_t* __restrict__ mask, const int* __restrict__ lt, int* __restrict__ tot,
+		int* __restrict__ posL, int* __restrict__ posR) {
+	__shared__ int s_sum[RUNG_TPB / 32], s_sub[RUNG_TPB / 32];
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+	int all = 0, prev = 0;
+	for (int q = threadIdx.x; q < (int) gridDim.x; q += RUNG_TPB) {
+		const int c = lt[q];
+		all += c;
+		prev += q < (int) blockIdx.x ? c : 0;
+	}
+	const int m = rung_block_sum(all, s_sum);
+	int before = rung_block_sum(prev, s_sum);
+	const unsigned mine = mask[(blockIdx.x * (RUNG_TPB / 32) + w) * 32 + lane];
+	const int here = __reduce_add_sync(0xffffffffu, __popc(mine));
+	if (lane == 0) {
+		s_sub[w] = here;
+	}
+	__syncthreads();
+	for (int i = 0; i < w; i++) {
+		before += s_sub[i];
+	}
+	const int64_t off = blockIdx.x * (int64_t) RUNG_TILE + w * RUNG_SUB;  // from b
+	const int n = (int) max((int64_t) 0, min((int64_t) RUNG_SUB, e - b - off));
+	if (n > 0) {
+		const int cut = (int) max((int64_t) 0, min((int64_t) n, m - off));
+		const int l0 = (int) off - before, after = m - before - here;
+		const int base = (int) (b + off);
+		sub_wrong(mine, n, cut, lane, [&](int k, int o) { posL[l0 + k] = base + o; }, [&](int k, int o) { posR[after + k] = base + o; });
+		// the warp that holds the split point (or the last one, when nothing lies after it)
+		if ((off <= m && m < off + n) || (m == e - b && off + n == e - b)) {
+			const int right = __reduce_add_sync(0xffffffffu, __popc(mine & ~first_bits(cut, 32 * lane)));
+			if (lane == 0) {
+				tot[0] = m;
+				tot[1] = after + right;
+			}
 		}
 	}
 }
@@ -402,34 +465,19 @@ ct_status sort_by_rung_run(Ctx* c, Box* b, int minrung) {
 		return CT_OK;
 	}
 	ct_status s = CT_OK;
-	int* lt = (int*) scratch(c, 21, sizeof(int) * n, &s);
-	int* misL = (int*) scratch(c, 22, sizeof(int) * n, &s);
-	int* misR = (int*) scratch(c, 23, sizeof(int) * n, &s);
-	int* exL = (int*) scratch(c, 24, sizeof(int) * n, &s);
-	int* exR = (int*) scratch(c, 25, sizeof(int) * n, &s);
-	int* posL = (int*) scratch(c, 26, sizeof(int) * n, &s);
-	int* posR = (int*) scratch(c, 27, sizeof(int) * n, &s);
+	const int nt = (int) ((n + RUNG_TILE - 1) / RUNG_TILE);
+	int* lt = (int*) scratch(c, 21, sizeof(int) * nt, &s);
+	uint32_t* mask = (uint32_t*) scratch(c, 22, sizeof(uint32_t) * (RUNG_TILE / 32) * nt, &s);
+	// (at most half of the particles change places)
+	int* posL = (int*) scratch(c, 26, sizeof(int) * (n / 2 + 1), &s);
+	int* posR = (int*) scratch(c, 27, sizeof(int) * (n / 2 + 1), &s);
 	int* tot = (int*) scratch(c, 28, sizeof(int) * 4, &s);
 	CT_TRY(s);
-	size_t need = 0, need2 = 0;
-	cub::DeviceReduce::Sum(nullptr, need, lt, tot, (int) n, st);
-	cub::DeviceScan::ExclusiveSum(nullptr, need2, misL, exL, (int) n, st);
-	void* tmp = scratch(c, 29, std::max(need, need2) + 256, &s);
-	CT_TRY(s);
-	need = std::max(need, need2);
-	c->launches++;
-	k_rung_flags<<<grid(c, n, 256), 256, 0, st>>>(beg, e, b->rung, minrung, lt);
-	CT_CUDA(c, cub::DeviceReduce::Sum(tmp, need, lt, tot, (int) n, st));
-	c->launches++;
-	k_rung_mis<<<grid(c, n, 256), 256, 0, st>>>(beg, e, lt, tot, misL, misR);
-	CT_CUDA(c, cub::DeviceScan::ExclusiveSum(tmp, need, misL, exL, (int) n, st));
-	CT_CUDA(c, cub::DeviceReduce::Sum(tmp, need, misL, tot + 1, (int) n, st));
-	CT_CUDA(c, cub::DeviceScan::ExclusiveSum(tmp, need, misR, exR, (int) n, st));
-	CT_CUDA(c, cub::DeviceReduce::Sum(tmp, need, misR, tot + 2, (int) n, st));
-	c->launches++;
-	k_rung_pos<<<grid(c, n, 256), 256, 0, st>>>(beg, e, misL, misR, exL, exR, tot + 2, posL, posR);
-	c->launches++;
+	c->launches += 3;
+	k_rung_ballots<<<nt, RUNG_TPB, 0, st>>>(beg, e, b->rung, minrung, mask, lt);
+	k_rung_pos<<<nt, RUNG_TPB, 0, st>>>(beg, e, mask, lt, tot, posL, posR);
 	k_rung_swap<<<grid(c, n, 256), 256, 0, st>>>(posL, posR, tot + 1, b->x[0], b->x[1], b->x[2], b->v[0], b->v[1], b->v[2], b->rung);
+	CT_CUDA(c, cudaGetLastError());
 	int* h = (int*) c->pinned;
 	CT_CUDA(c, cudaMemcpyAsync(h, tot, sizeof(int), cudaMemcpyDeviceToHost, st));
 	CT_CUDA(c, cudaStreamSynchronize(st));
