@@ -388,9 +388,9 @@ __device__ __forceinline__ int wrap1(int i, int n) {
 	return i < 0 ? i + n : (i >= n ? i - n : i);
 }
 
-__global__ void __launch_bounds__(FT_TPB) k_ic_displace(int N, const float* __restrict__ R, AxisTables t, double scale, float D, float prefac,
+__global__ void __launch_bounds__(FT_TPB, 5) k_ic_displace(int N, const float* __restrict__ R, AxisTables t, double scale, float D, float prefac,
 		double box_size_inv, uint32_t* __restrict__ X, float* __restrict__ V, unsigned int* dxmax) {
-	extern __shared__ double s_rows[];  // [rows][N] sums along x, then [DISP_ROWS][N] sums along x and y
+	extern __shared__ double s_rows[];  // [rows][N] sums along x, then [N] sums along x and y
 	const int I0 = blockIdx.y, y0 = blockIdx.x * DISP_ROWS;
 	const int ny = min(DISP_ROWS, N - y0);
 	// rows y0's first neighbour .. the last row's last, wrapped (a lattice point's cell never falls
@@ -399,25 +399,26 @@ __global__ void __launch_bounds__(FT_TPB) k_ic_displace(int N, const float* __re
 	const int nrow = __ldg(t.cell + y0 + ny - 1) + CLOUD_MAX - r0 + 1;  // at most DISP_ROWS + 6
 	double* s_y = s_rows + (size_t) (DISP_ROWS + 6) * N;
 	const int c0 = __ldg(t.cell + I0) + CLOUD_MIN;
-	int64_t plane[6];
+	int plane[6];  // (a grid has at most 2^30 points)
 	double wx[6];
 #pragma unroll
 	for (int j = 0; j < 6; j++) {
-		plane[j] = (int64_t) wrap1(c0 + j, N) * N * N;
+		plane[j] = wrap1(c0 + j, N) * N * N;
 		wx[j] = __ldg(t.weight + j * N + I0);
 	}
 	for (int r = 0; r < nrow; r++) {
-		const float* p = R + (int64_t) wrap1(r0 + r, N) * N;
+		const int p = wrap1(r0 + r, N) * N;
 		for (int z = threadIdx.x; z < N; z += FT_TPB) {
 			double acc = 0.0;
 #pragma unroll
 			for (int j = 0; j < 6; j++) {
-				acc += wx[j] * (double) p[plane[j] + z];
+				acc += wx[j] * (double) R[plane[j] + p + z];
 			}
-			s_rows[(size_t) r * N + z] = acc;
+			s_rows[r * N + z] = acc;
 		}
 	}
 	__syncthreads();
+	float mymax = 0.f;
 	for (int y = 0; y < ny; y++) {
 		const int first = __ldg(t.cell + y0 + y) + CLOUD_MIN - r0;
 		double wy[6];
@@ -429,41 +430,32 @@ __global__ void __launch_bounds__(FT_TPB) k_ic_displace(int N, const float* __re
 			double acc = 0.0;
 #pragma unroll
 			for (int j = 0; j < 6; j++) {
-				acc += wy[j] * s_rows[(size_t) (first + j) * N + z];
+				acc += wy[j] * s_rows[(first + j) * N + z];
 			}
-			s_y[(size_t) y * N + z] = acc;
+			s_y[z] = acc;
 		}
-	}
-	__syncthreads();
-	float mymax = 0.f;
-	for (int z = threadIdx.x; z < N; z += FT_TPB) {
-		const int c = __ldg(t.cell + z) + CLOUD_MIN;
-		int at[6];
-		double wz[6];
-#pragma unroll
-		for (int j = 0; j < 6; j++) {
-			at[j] = wrap1(c + j, N);
-			wz[j] = __ldg(t.weight + j * N + z);
-		}
-		for (int y = 0; y < ny; y++) {
-			const int64_t p = ((int64_t) I0 * N + y0 + y) * N + z;
+		__syncthreads();
+		const int base = (I0 * N + y0 + y) * N;
+		for (int z = threadIdx.x; z < N; z += FT_TPB) {
+			const int c = __ldg(t.cell + z) + CLOUD_MIN;
 			double dx = 0.0;
 #pragma unroll
 			for (int j = 0; j < 6; j++) {
-				dx += wz[j] * s_y[(size_t) y * N + at[j]];
+				dx += __ldg(t.weight + j * N + z) * s_y[wrap1(c + j, N)];
 			}
 			dx *= scale;
 			dx *= -D * box_size_inv;
-			double x = fixed_to_double(X[p]) + dx;
+			double x = fixed_to_double(X[base + z]) + dx;
 			if (x >= 1.0) {
 				x -= 1.0;
 			} else if (x < 0.0) {
 				x += 1.0;
 			}
-			X[p] = fixed_from_double(x);
-			V[p] += prefac * dx;
+			X[base + z] = fixed_from_double(x);
+			V[base + z] += prefac * dx;
 			mymax = fmaxf(mymax, (float) (dx * N));
 		}
+		__syncthreads();
 	}
 	for (int o = 16; o; o >>= 1) {
 		mymax = fmaxf(mymax, __shfl_xor_sync(0xffffffffu, mymax, o));
@@ -641,14 +633,21 @@ __global__ void __launch_bounds__(32 * DEP_WARPS) k_density_tiles(const uint32_t
 			T[i] = 0.f;
 		}
 		__syncwarp();
+		// (the next particles' positions are on their way while these are added)
+		uint32_t px = 0, py = 0, pz = 0;
+		if (32u * w + lane < un.z) {
+			const uint32_t p = order[un.y + 32 * w + lane];
+			px = X[p];
+			py = Y[p];
+			pz = Z[p];
+		}
 		for (uint32_t q0 = 32 * w; q0 < un.z; q0 += 32 * DEP_WARPS) {
 			// a particle a lane: its first cell in the tile and its 18 weights
 			const int cnt = min(32, (int) (un.z - q0));
 			int base = 0;
 			if (lane < cnt) {
-				const uint32_t p = order[un.y + q0 + lane];
 				float fx, fy, fz;
-				const int j = deposit_cell(X[p], M, N, fx), k = deposit_cell(Y[p], M, N, fy), l = deposit_cell(Z[p], M, N, fz);
+				const int j = deposit_cell(px, M, N, fx), k = deposit_cell(py, M, N, fy), l = deposit_cell(pz, M, N, fz);
 				base = (j - tx * DEP_TILE) * DEP_SX + (k - ty * DEP_TILE) * DEP_SY + (l - tz * DEP_TILE);
 				float* sw = s_w[w][lane];
 #pragma unroll
@@ -657,6 +656,12 @@ __global__ void __launch_bounds__(32 * DEP_WARPS) k_density_tiles(const uint32_t
 					sw[6 + q] = cloud_weight(fx - (q + CLOUD_MIN));
 					sw[12 + q] = cloud_weight(fy - (q + CLOUD_MIN));
 				}
+			}
+			if (q0 + 32 * DEP_WARPS + lane < un.z) {
+				const uint32_t p = order[un.y + q0 + 32 * DEP_WARPS + lane];
+				px = X[p];
+				py = Y[p];
+				pz = Z[p];
 			}
 			__syncwarp();
 			for (int i = 0; i < cnt; i++) {
@@ -688,8 +693,15 @@ __global__ void __launch_bounds__(32 * DEP_WARPS) k_density_tiles(const uint32_t
 				v += s_rho[q][cx * DEP_SX + cy * DEP_SY + cz];
 			}
 			if (v != 0.f) {
-				const int64_t gx = wrap(tx * DEP_TILE + cx + CLOUD_MIN, N), gy = wrap(ty * DEP_TILE + cy + CLOUD_MIN, N), gz = wrap(tz * DEP_TILE + cz + CLOUD_MIN, N);
-				atomicAdd(rho + (gx * N + gy) * N + gz, v);
+				auto cell = [&](int t, int c) {
+					int g = t * DEP_TILE + c + CLOUD_MIN;
+					g = g < 0 ? g + N : g;
+					while (g >= N) {
+						g -= N;
+					}
+					return (int64_t) g;
+				};
+				atomicAdd(rho + (cell(tx, cx) * N + cell(ty, cy)) * N + cell(tz, cz), v);
 			}
 		}
 		__syncthreads();
@@ -1056,7 +1068,7 @@ extern "C" ct_status ct_initialize(ct_ctx* ctx, int box_id, const ct_ic_params* 
 	k_ic_uniforms<<<ft_grid(c, (int64_t) N * N), FT_TPB, 0, st>>>(N, A);
 	k_ic_amplitude<<<gx, FT_TPB, 0, st>>>(N, box, factor, dtab, A);
 	// interpolation at the lattice points and update of axis dim
-	const size_t disp_smem = sizeof(double) * (2 * DISP_ROWS + 6) * N;  // 176 KB at the largest grid
+	const size_t disp_smem = sizeof(double) * (DISP_ROWS + 7) * N;  // 120 KB at the largest grid
 	CT_CUDA(c, cudaFuncSetAttribute(k_ic_displace, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) disp_smem));
 	auto displace = [&](int dim, float D, float prefac, unsigned int* mx) {
 		c->launches++;
