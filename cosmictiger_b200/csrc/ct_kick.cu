@@ -191,6 +191,37 @@ __device__ __forceinline__ int2 flush(const int* src, int cnt, int cap, int* dst
 	return make_int2((int) off, cnt);
 }
 
+// A check list read ahead: the node of the next 32 entries and the indices of the 32 after them are on
+// their way while a batch is tested (an entry's index and its node are two dependent gathers of about
+// half a microsecond each, and a warp's batches used to wait for both in turn).
+struct CheckStream {
+	const int* list;
+	int n;
+	int c1, c2;  // this lane's entry of the next batch and of the one after
+	NodeW ahead;
+	__device__ __forceinline__ void start(const int* l, int count, const NodeW* __restrict__ nodes, int lane) {
+		list = l;
+		n = count;
+		c1 = lane < n ? list[lane] : -1;
+		c2 = lane + 32 < n ? list[lane + 32] : -1;
+		if (c1 >= 0) {
+			ahead = nodes[c1];
+		}
+	}
+	// entry j0 + lane (-1 past the end) and its node; j0 rises by 32 from call to call
+	__device__ __forceinline__ int next(int j0, NodeW& ot, const NodeW* __restrict__ nodes, int lane) {
+		const int c = c1;
+		ot = ahead;
+		c1 = c2;
+		const int j = j0 + 64 + lane;
+		c2 = j < n ? list[j] : -1;
+		if (c1 >= 0) {
+			ahead = nodes[c1];
+		}
+		return c;
+	}
+};
+
 __global__ void __launch_bounds__(WALK_TPB) k_walk(int64_t lb, int64_t le, const NodeW* __restrict__ nodes, const int32_t* __restrict__ nbox,
 		const int32_t* __restrict__ parent, WalkOut o, WalkParams p) {
 	const int lane = threadIdx.x & 31;
@@ -250,12 +281,13 @@ __global__ void __launch_bounds__(WALK_TPB) k_walk(int64_t lb, int64_t le, const
 		const float rs = self.radius;
 		// ---- Ewald list: one pass
 		int n_ecc = 0, n_eout = 0;
+		CheckStream cs;
+		cs.start(ein, ne, nodes, lane);
 		for (int j0 = 0; j0 < ne; j0 += 32) {
-			const int j = j0 + lane;
-			int cc = 0, nx = 0, c = 0, c0 = 0;
-			if (j < ne) {
-				c = ein[j];
-				const NodeW ot = nodes[c];
+			int cc = 0, nx = 0, c0 = 0;
+			NodeW ot;
+			const int c = cs.next(j0, ot, nodes, lane);
+			if (c >= 0) {
 				if (ot.pend > ot.pbeg) {
 					const float dx = fixed_dist(self.x, ot.x), dy = fixed_dist(self.y, ot.y), dz = fixed_dist(self.z, ot.z);
 					float R2 = sqrf3(dx, dy, dz);
@@ -284,13 +316,13 @@ __global__ void __launch_bounds__(WALK_TPB) k_walk(int64_t lb, int64_t le, const
 		while (true) {
 			int* nxt = sl[S_NEXT0 + which];
 			n_next = 0;
+			cs.start(cur, ncur, nodes, lane);
 			for (int j0 = 0; j0 < ncur; j0 += 32) {
-				const int j = j0 + lane;
-				int kind = -1, c = 0;  // 0 cc 1 cp 2 pc 3 leaf 4 next
+				int kind = -1;  // 0 cc 1 cp 2 pc 3 leaf 4 next
 				int c0 = 0;
-				if (j < ncur) {
-					c = cur[j];
-					const NodeW ot = nodes[c];
+				NodeW ot;
+				const int c = cs.next(j0, ot, nodes, lane);
+				if (c >= 0) {
 					const int onp = ot.pend - ot.pbeg;
 					if (onp) {
 						const float dx = fixed_dist(self.x, ot.x), dy = fixed_dist(self.y, ot.y), dz = fixed_dist(self.z, ot.z);
