@@ -799,14 +799,28 @@ __device__ __forceinline__ void ksum(float& s, float& comp, float v) {
 // warp in shared memory as offsets from the leaf centre), then M2P + L2P + kick per tile.
 constexpr int P2P_TPB = 256;
 
+// The sink tiles of the leaves that hold particles, made on the device and never counted on the host
+// (each count read back cost a kick of a small box 15-20 us): full tiles from the front of the array,
+// tiles of at most 16 sinks from its back.
+struct TileList {
+	const int2* items;
+	int64_t cap;
+	const unsigned long long* count;  // full tiles, small tiles, leaves
+	__device__ __forceinline__ int64_t big() const {
+		return (int64_t) count[0];
+	}
+	__device__ __forceinline__ int64_t small() const {
+		return (int64_t) count[1];
+	}
+};
+
 struct P2PArgs {
 	int nsub;
 	const int64_t* sub_off;
 	const float* sub_h;
 	const NodeW* nodes;
 	const int32_t* nbox;  // tight boxes of the nodes
-	const int2* items;  // (leaf node, tile)
-	int64_t nitems;
+	TileList tiles;     // (leaf node, tile)
 	const int2* pp;
 	const int* pp_list;
 	const uint32_t* x[3];
@@ -1036,6 +1050,7 @@ __global__ void __launch_bounds__(P2P_TPB, 3) k_p2p(P2PArgs a) {
 	const int pw = WPT > 1 ? (w & 1) : 0, pair = w >> 1;
 	P2PStage<STAGE>* my = &stage[w];
 	double npairs = 0.0, nnear = 0.0;
+	const int64_t nitems = SMALL ? a.tiles.small() : a.tiles.big();
 	// a resident grid; each warp (pair of warps) takes the next tile when it is done with one
 	for (;;) {
 		int64_t it;
@@ -1051,10 +1066,10 @@ __global__ void __launch_bounds__(P2P_TPB, 3) k_p2p(P2PArgs a) {
 			pair_sync(pair);
 			it = pair_tile[pair];
 		}
-		if (it >= a.nitems) {
+		if (it >= nitems) {
 			break;
 		}
-		const int2 item = a.items[it];
+		const int2 item = a.tiles.items[SMALL ? a.tiles.cap - 1 - it : it];
 		const NodeW self = a.nodes[item.x];
 		const float h = a.sub_h ? a.sub_h[box_of(a.sub_off, a.nsub, self.pbeg)] : a.h;
 		const float h2 = h * h, hinv = 1.f / h, h2inv = hinv * hinv, h3inv = h2inv * hinv;
@@ -1197,8 +1212,8 @@ __global__ void __launch_bounds__(P2P_TPB, 3) k_p2p(P2PArgs a) {
 // once and meets all of the leaf's tiles, instead of once a tile.  Staging (owner search, gathers,
 // conversions) and bookkeeping were 16 of k_p2p's 47 warp instructions a quad of pairs, and its waits
 // on the gathers and shuffles a fifth of its stalls.  The tiles' compensated sums and the sinks'
-// offsets stay in shared memory between chunks, which leaves 72 registers for seven blocks of four
-// warps an SM (28 warps against 24).  Every sink's sums are made from the same chunks in the same
+// offsets stay in shared memory between chunks, which leaves 80 registers, without spills, for six
+// blocks of four warps an SM (seven at 72 registers and eight at 64 measured 1% slower).  Every sink's sums are made from the same chunks in the same
 // order as k_p2p makes them, so the two give the same bits and either may run: this one where the
 // leaves keep its warps busy (see launch_p2p_any).
 constexpr int LEAF_TPB = 128;
@@ -1214,7 +1229,7 @@ struct LeafStage {
 };
 
 template<int STAGE>
-__global__ void __launch_bounds__(LEAF_TPB, 7) k_p2p_leaf(P2PArgs a) {
+__global__ void __launch_bounds__(LEAF_TPB, 6) k_p2p_leaf(P2PArgs a) {
 	extern __shared__ __align__(16) char leaf_smem[];
 	const int lane = threadIdx.x & 31;
 	LeafStage<STAGE>& my = reinterpret_cast<LeafStage<STAGE>*>(leaf_smem)[threadIdx.x >> 5];
@@ -1370,18 +1385,40 @@ __global__ void __launch_bounds__(LEAF_TPB, 7) k_p2p_leaf(P2PArgs a) {
 	}
 }
 
-// Tiles with more than 16 sinks to `big`, the others to `small` (order within each list is
-// immaterial: every tile computes its own sinks).
-__global__ void k_split_tiles(const int2* __restrict__ items, int64_t nitems, const NodeW* __restrict__ nodes, int tw, int2* big, int2* small,
-		unsigned long long* counts) {
-	for (int64_t it = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; it < nitems; it += (int64_t) gridDim.x * blockDim.x) {
-		const int2 item = items[it];
-		const NodeW nd = nodes[item.x];
-		const int S = min(tw, nd.pend - (nd.pbeg + tw * item.y));
-		if (S > 16) {
-			big[atomicAdd(counts, 1ull)] = item;
-		} else {
-			small[atomicAdd(counts + 1, 1ull)] = item;
+// The tile list: tw sinks a tile (order within each kind is immaterial: every tile computes its own
+// sinks), one atomic a warp and kind.
+__global__ void __launch_bounds__(256) k_leaf_tiles(int64_t nn, const NodeW* __restrict__ nodes, int tw, int64_t cap, int2* __restrict__ items, unsigned long long* count) {
+	const int lane = threadIdx.x & 31;
+	for (int64_t i0 = blockIdx.x * (int64_t) blockDim.x + (threadIdx.x - lane); i0 < nn; i0 += (int64_t) gridDim.x * blockDim.x) {
+		const int64_t i = i0 + lane;
+		int n = 0;
+		if (i < nn) {
+			const NodeW nd = nodes[i];
+			n = nd.flags & 1 ? nd.pend - nd.pbeg : 0;
+		}
+		const int nt = (n + tw - 1) / tw;
+		// tiles of more than 16 sinks come first; the rest are small (the last, or all at width 16)
+		const int nb = tw <= 16 ? 0 : nt - (n > 0 && n - tw * (nt - 1) <= 16), ns = nt - nb;
+		int ib = nb, is = ns;
+		for (int o = 1; o < 32; o <<= 1) {
+			const int tb = __shfl_up_sync(0xffffffffu, ib, o), ts = __shfl_up_sync(0xffffffffu, is, o);
+			ib += lane >= o ? tb : 0;
+			is += lane >= o ? ts : 0;
+		}
+		const unsigned have = __ballot_sync(0xffffffffu, n > 0);
+		unsigned long long b0 = 0, s0 = 0;
+		if (lane == 31 && have) {
+			b0 = ib ? atomicAdd(count, (unsigned long long) ib) : 0ull;
+			s0 = is ? atomicAdd(count + 1, (unsigned long long) is) : 0ull;
+			atomicAdd(count + 2, (unsigned long long) __popc(have));
+		}
+		b0 = __shfl_sync(0xffffffffu, b0, 31) + (unsigned long long) (ib - nb);
+		s0 = __shfl_sync(0xffffffffu, s0, 31) + (unsigned long long) (is - ns);
+		for (int t = 0; t < nb; t++) {
+			items[b0 + t] = make_int2((int) i, t);
+		}
+		for (int t = 0; t < ns; t++) {
+			items[cap - 1 - (int64_t) (s0 + t)] = make_int2((int) i, nb + t);
 		}
 	}
 }
@@ -1397,8 +1434,8 @@ struct KickTileArgs {
 	const NodeW* nodes;
 	const float* multi;
 	const float* Lx;
-	const int2* items;
-	int64_t nitems;
+	TileList tiles;
+	const int* bad;  // the walk's flags: nothing is kicked when its lists did not fit
 	const int2* pc;
 	const int* pc_list;
 	const float4* F;
@@ -1428,8 +1465,9 @@ __global__ void __launch_bounds__(128, 3) k_leaf_kick(KickTileArgs a) {
 		acc[q] = 0.0;
 	}
 	int maxr = 0;
-	for (int64_t it = warp_take(a.next, 1); it < a.nitems; it = warp_take(a.next, 1)) {
-		const int2 item = a.items[it];
+	const int64_t nbig = a.tiles.big(), nitems = (a.bad[0] | a.bad[1]) ? 0 : nbig + a.tiles.small();
+	for (int64_t it = warp_take(a.next, 1); it < nitems; it = warp_take(a.next, 1)) {
+		const int2 item = a.tiles.items[it < nbig ? it : a.tiles.cap - 1 - (it - nbig)];
 		const NodeW self = a.nodes[item.x];
 		const int bx = a.nsub > 1 ? box_of(a.sub_off, a.nsub, self.pbeg) : 0;
 		const float hh = a.sub_h ? a.sub_h[bx] : kp.h;
@@ -1600,32 +1638,6 @@ __global__ void __launch_bounds__(128, 3) k_leaf_kick(KickTileArgs a) {
 	}
 }
 
-// Tiles of tw sinks of every leaf: counts, then (leaf, tile) items at the scanned offsets.
-__global__ void k_tile_count(int64_t nleaves, const int64_t* leaves, const NodeW* nodes, int tw, int* ntiles) {
-	for (int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < nleaves; i += (int64_t) gridDim.x * blockDim.x) {
-		const NodeW nd = nodes[leaves[i]];
-		ntiles[i] = (nd.pend - nd.pbeg + tw - 1) / tw;
-	}
-}
-__global__ void k_tile_fill(int64_t nleaves, const int64_t* leaves, const int* ntiles, const int* off, int2* items) {
-	for (int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < nleaves; i += (int64_t) gridDim.x * blockDim.x) {
-		const int o = off[i];
-		for (int t = 0; t < ntiles[i]; t++) {
-			items[o + t] = make_int2((int) leaves[i], t);
-		}
-	}
-}
-
-__global__ void k_collect_leaves(int64_t nn, const NodeW* nodes, int64_t* leaves, unsigned long long* count) {
-	for (int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < nn; i += (int64_t) gridDim.x * blockDim.x) {
-		const NodeW nd = nodes[i];
-		if ((nd.flags & 1) && nd.pend > nd.pbeg) {
-			const unsigned long long p = atomicAdd(count, 1ull);
-			leaves[p] = i;
-		}
-	}
-}
-
 // ---------------------------------------------------------------- host driver
 }  // namespace
 
@@ -1693,8 +1705,6 @@ struct KickBuffers {
 	size_t dL3_n = 0;
 	float* Lx = nullptr;
 	size_t Lx_n = 0;
-	int64_t* leaves = nullptr;
-	size_t leaves_n = 0;
 };
 
 namespace {
@@ -1734,7 +1744,6 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 	CT_TRY(ensure(c, &K.dL2, K.dL2_n, (size_t) NEXP_STRIDE * nn, "expansion deltas (direct M2L)"));
 	CT_TRY(ensure(c, &K.dL3, K.dL3_n, (size_t) NEXP_STRIDE * nn, "expansion deltas (P2L)"));
 	CT_TRY(ensure(c, &K.Lx, K.Lx_n, (size_t) NEXP_STRIDE * nn, "local expansions"));
-	CT_TRY(ensure(c, &K.leaves, K.leaves_n, (size_t) nn, "leaf index"));
 	K.nwarps = c->nsm * 16 * (WALK_TPB / 32) / 4;  // 4 blocks of 4 warps per SM
 	if (K.stage_cap == 0) {
 		K.stage_cap = 4096;
@@ -1792,20 +1801,8 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 		}
 		CT_CUDA(c, cudaGetLastError());
 		cudaEventRecord(c->ev[1], st);
-		int* hf = (int*) c->pinned;
-		CT_CUDA(c, cudaMemcpyAsync(hf, c->d_flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
-		CT_CUDA(c, cudaStreamSynchronize(st));
-		if (hf[1]) {
-			return fail(c, CT_ERR_STATE, "an Ewald check failed the opening test against a leaf; the tree was built with a different theta");
-		}
-		if (hf[0]) {
-			// overflow: grow everything and retry
-			K.stage_cap *= 2;
-			K.cap_cc *= 2;
-			K.cap_leaf *= 2;
-			K.cap_pass *= 2;
-			continue;
-		}
+		// (whether the lists fitted is read with the results: the kernels that follow run on what fitted,
+		// and the leaf kick changes nothing if something did not)
 		// ---- interactions
 		CT_CUDA(c, cudaMemsetAsync(counters, 0, 16 * sizeof(double), st));
 		// node orders of the node-indexed kernels, longest lists first (radix sort of the
@@ -1863,49 +1860,30 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 					K.Lx, kp->do_phi);
 		}
 		cudaEventRecord(c->ev[3], st);
-		// leaves
-		unsigned long long* lcount = (unsigned long long*) (c->d_flags + 40);
-		CT_CUDA(c, cudaMemsetAsync(lcount, 0, sizeof(unsigned long long), st));
-		c->launches++;
-		k_collect_leaves<<<(int) std::max<int64_t>(1, std::min<int64_t>((nn + 255) / 256, c->nsm * 8)), 256, 0, st>>>(nn, b->nodes, K.leaves, lcount);
-		CT_CUDA(c, cudaMemcpyAsync(hf, lcount, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-		CT_CUDA(c, cudaStreamSynchronize(st));
-		const int64_t nleaves = (int64_t) * (unsigned long long*) hf;
+		// leaves' tiles; a binary tree of nn nodes and nsub roots has (nn + nsub) / 2 leaves
+		const int64_t nleaf = (nn + b->nsub) / 2;
+		const int tw = c->tune.tile_width;
+		unsigned long long* tcount = (unsigned long long*) (c->d_flags + 40);  // full tiles, small tiles, leaves
+		CT_CUDA(c, cudaMemsetAsync(tcount, 0, 3 * sizeof(unsigned long long), st));
 		cudaEventRecord(c->ev[4], st);
 		cudaEventRecord(c->ev[5], st);
-		cudaEventRecord(c->ev[12], st);  // no leaves: zero P2P and leaf-kick times
-		if (nleaves > 0) {
-			// 32-sink tiles of the leaves
+		cudaEventRecord(c->ev[12], st);  // no particles: zero P2P and leaf-kick times
+		if (np > 0) {
 			ct_status s2 = CT_OK;
-			int* ntl = (int*) scratch(c, 40, sizeof(int) * (nleaves + 1), &s2);
-			int* off = (int*) scratch(c, 41, sizeof(int) * (nleaves + 1), &s2);
-			CT_TRY(s2);
-			size_t need = 0;
-			cub::DeviceScan::ExclusiveSum(nullptr, need, ntl, off, (int) nleaves + 1, st);
-			void* tmp = scratch(c, 42, need + 256, &s2);
-			CT_TRY(s2);
-			c->launches++;
-			const int tw = c->tune.tile_width;
-			k_tile_count<<<(int) std::max<int64_t>(1, std::min<int64_t>((nleaves + 255) / 256, c->nsm * 8)), 256, 0, st>>>(nleaves, K.leaves, b->nodes, tw,
-					ntl);
-			CT_CUDA(c, cudaMemsetAsync(ntl + nleaves, 0, sizeof(int), st));
-			CT_CUDA(c, cub::DeviceScan::ExclusiveSum(tmp, need, ntl, off, (int) nleaves + 1, st));
-			CT_CUDA(c, cudaMemcpyAsync(hf, off + nleaves, sizeof(int), cudaMemcpyDeviceToHost, st));
-			CT_CUDA(c, cudaStreamSynchronize(st));
-			const int64_t nitems = hf[0];
-			int2* items = (int2*) scratch(c, 43, sizeof(int2) * (nitems + 1), &s2);
+			const int64_t tile_cap = np / tw + nleaf + 1;
+			int2* items = (int2*) scratch(c, 43, sizeof(int2) * tile_cap, &s2);
 			float4* F = (float4*) scratch(c, 44, sizeof(float4) * b->n, &s2);
 			CT_TRY(s2);
 			c->launches++;
-			k_tile_fill<<<(int) std::max<int64_t>(1, std::min<int64_t>((nleaves + 255) / 256, c->nsm * 8)), 256, 0, st>>>(nleaves, K.leaves, ntl, off, items);
+			k_leaf_tiles<<<(int) std::max<int64_t>(1, std::min<int64_t>((nn + 255) / 256, c->nsm * 8)), 256, 0, st>>>(nn, b->nodes, tw, tile_cap, items, tcount);
+			const TileList tiles { items, tile_cap, tcount };
 			P2PArgs pa;
 			pa.nsub = b->nsub;
 			pa.sub_off = b->d_sub_off;
 			pa.sub_h = b->d_sub_h;
 			pa.nodes = b->nodes;
 			pa.nbox = b->nbox;
-			pa.items = items;
-			pa.nitems = nitems;
+			pa.tiles = tiles;
 			pa.pp = o.pp;
 			pa.pp_list = o.pp_list;
 			for (int d = 0; d < 3; d++) {
@@ -1917,45 +1895,27 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 			pa.pairs = counters + 4 + 7;
 			pa.near_pairs = counters + 13;
 			pa.tw = tw;
-			const int64_t leaf_warps = (int64_t) c->nsm * 28;
-			if (c->tune.warps_per_tile == 1 && tw == 32 && nleaves >= LEAF_WAVES * leaf_warps) {
+			cudaEventRecord(c->ev[4], st);
+			const int64_t leaf_warps = (int64_t) c->nsm * 24;
+			if (c->tune.warps_per_tile == 1 && tw == 32 && nleaf >= LEAF_WAVES * leaf_warps) {
 				pa.order = oidx + 4 * nn;
 				pa.nn = nn;
 				pa.next = onext + 3;
-				cudaEventRecord(c->ev[4], st);
 				c->launches++;
 				const int stage = c->tune.p2p_stage;
 				CT_TRY(stage == 64 ? launch_p2p_leaf_t<64>(c, pa, st) : stage == 256 ? launch_p2p_leaf_t<256>(c, pa, st) : launch_p2p_leaf_t<128>(c, pa, st));
 			} else {
-				// full tiles and tiles of at most 16 sinks go to separate launches
-				int2* tiles2 = (int2*) scratch(c, 45, sizeof(int2) * 2 * (nitems + 1), &s2);
-				CT_TRY(s2);
-				unsigned long long* tcount = (unsigned long long*) (c->d_flags + 44);
-				CT_CUDA(c, cudaMemsetAsync(tcount, 0, 2 * sizeof(unsigned long long), st));
-				unsigned long long* wnext = (unsigned long long*) (c->d_flags + 52);  // work counters of the two launches
+				// full tiles and tiles of at most 16 sinks in launches of their own
+				unsigned long long* wnext = (unsigned long long*) (c->d_flags + 52);  // their work counters
 				CT_CUDA(c, cudaMemsetAsync(wnext, 0, 2 * sizeof(unsigned long long), st));
-
-				c->launches++;
-				k_split_tiles<<<(int) std::max<int64_t>(1, std::min<int64_t>((nitems + 255) / 256, c->nsm * 8)), 256, 0, st>>>(items, nitems, b->nodes, tw,
-						tiles2, tiles2 + nitems + 1, tcount);
-				CT_CUDA(c, cudaMemcpyAsync(hf, tcount, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-				CT_CUDA(c, cudaStreamSynchronize(st));
-				const int64_t nbig = (int64_t) ((unsigned long long*) hf)[0], nsmall = (int64_t) ((unsigned long long*) hf)[1];
-				cudaEventRecord(c->ev[4], st);
-				if (nbig > 0) {
-					pa.items = tiles2;
-					pa.nitems = nbig;
+				if (tw > 16) {
 					pa.next = wnext;
 					c->launches++;
-					launch_p2p<false>(c, pa, nbig, st);
+					launch_p2p<false>(c, pa, np / tw + nleaf, st);
 				}
-				if (nsmall > 0) {
-					pa.items = tiles2 + nitems + 1;
-					pa.nitems = nsmall;
-					pa.next = wnext + 1;
-					c->launches++;
-					launch_p2p<true>(c, pa, nsmall, st);
-				}
+				pa.next = wnext + 1;
+				c->launches++;
+				launch_p2p<true>(c, pa, tw > 16 ? nleaf : np / tw + nleaf, st);
 			}
 			cudaEventRecord(c->ev[5], st);
 			KickTileArgs ka;
@@ -1973,8 +1933,8 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 			ka.nodes = b->nodes;
 			ka.multi = b->multi;
 			ka.Lx = K.Lx;
-			ka.items = items;
-			ka.nitems = nitems;
+			ka.tiles = tiles;
+			ka.bad = c->d_flags;
 			ka.pc = o.pc;
 			ka.pc_list = o.pc_list;
 			ka.F = F;
@@ -1992,7 +1952,7 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 			ka.tw = tw;
 			CT_CUDA(c, cudaMemsetAsync(ka.next, 0, sizeof(unsigned long long), st));
 			c->launches++;
-			k_leaf_kick<Ops><<<(int) std::max<int64_t>(1, std::min<int64_t>((nitems + 3) / 4, (int64_t) resident_blocks(c, k_leaf_kick<Ops>, 128))), 128, 0,
+			k_leaf_kick<Ops><<<(int) std::max<int64_t>(1, std::min<int64_t>((tile_cap + 3) / 4, (int64_t) resident_blocks(c, k_leaf_kick<Ops>, 128))), 128, 0,
 					st>>>(ka);
 			cudaEventRecord(c->ev[12], st);
 		}
@@ -2002,7 +1962,21 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 		CT_CUDA(c, cudaMemcpyAsync(hd + 16, c->d_flags + 48, sizeof(int), cudaMemcpyDeviceToHost, st));
 		unsigned long long* hcur = (unsigned long long*) (hd + 20);
 		CT_CUDA(c, cudaMemcpyAsync(hcur, o.cursor, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+		CT_CUDA(c, cudaMemcpyAsync(hcur + 5, tcount + 2, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+		int* hf = (int*) (hcur + 6);
+		CT_CUDA(c, cudaMemcpyAsync(hf, c->d_flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
 		CT_CUDA(c, cudaStreamSynchronize(st));
+		if (hf[1]) {
+			return fail(c, CT_ERR_STATE, "an Ewald check failed the opening test against a leaf; the tree was built with a different theta");
+		}
+		if (hf[0]) {
+			// overflow: grow everything and retry
+			K.stage_cap *= 2;
+			K.cap_cc *= 2;
+			K.cap_leaf *= 2;
+			K.cap_pass *= 2;
+			continue;
+		}
 		ct_kick_return r;
 		r.pot = hd[4];
 		r.kin = hd[5];
@@ -2023,7 +1997,7 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 		C.pp_near = hd[13];
 		C.cp_pairs = hd[1];
 		C.nodes = (double) nn;
-		C.leaves = (double) nleaves;
+		C.leaves = (double) hcur[5];
 		const double icnt = hd[0];
 		const bool phi = kp->do_phi != 0;
 		C.flops_pp = FLOP_PP * C.pp_pairs;
@@ -2037,7 +2011,7 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 		C.ms_m2l = elapsed_ms(c->ev[1], c->ev[2]);
 		C.ms_l2l = elapsed_ms(c->ev[2], c->ev[3]);
 		C.ms_leaf = elapsed_ms(c->ev[4], c->ev[5]);  // the P2P kernels
-		if (nleaves > 0) {
+		if (np > 0) {
 			C.ms_leafkick = elapsed_ms(c->ev[5], c->ev[12]);
 		}
 		b->have_force = kp->save_force != 0;
@@ -2101,7 +2075,6 @@ void kick_buffers_release(Ctx* c) {
 	dfree(c, K->dL2, sizeof(float) * K->dL2_n);
 	dfree(c, K->dL3, sizeof(float) * K->dL3_n);
 	dfree(c, K->Lx, sizeof(float) * K->Lx_n);
-	dfree(c, K->leaves, sizeof(int64_t) * K->leaves_n);
 	delete K;
 	c->kick = nullptr;
 }
