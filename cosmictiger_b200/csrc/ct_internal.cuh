@@ -4,6 +4,7 @@
 #include <stdint.h>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/ct_gravity.h"
@@ -63,6 +64,15 @@ __host__ __device__ inline int32_t range_fixed_from_double(double x) {
 #else
 	return (int32_t) (x * 536870912.0);
 #endif
+}
+
+// f(0), f(1), ..., f(N - 1) with the index a compile-time constant (std::integral_constant).
+template<int K, int N, class F>
+__host__ __device__ __forceinline__ void static_for(F&& f) {
+	if constexpr (K < N) {
+		f(std::integral_constant<int, K>());
+		static_for<K + 1, N>(f);
+	}
 }
 
 struct DevBuf {

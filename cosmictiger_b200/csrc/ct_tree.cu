@@ -892,178 +892,252 @@ __global__ void __launch_bounds__(UTPB) k_leaf_moments(int64_t nn, NodeW* nodes,
 	}
 }
 
-// The interior nodes of one level, a warp each (tree.cpp:351-497): union of the children's tight boxes,
-// expansion centre and radius, M2M of the two children in double.
-template<class Ops>
-__global__ void __launch_bounds__(UTPB) k_upsweep(int64_t lb, int64_t le, NodeW* nodes, int32_t* nbox, float* multi, double* tbox, const double* gbox,
-		const uint32_t* x0, const uint32_t* x1, const uint32_t* x2, int bucket) {
-	constexpr int NM = Ops::NMULT;
-	const uint32_t* xs[3] = { x0, x1, x2 };
-	const int lane = threadIdx.x & 31;
-	const int64_t gw = (blockIdx.x * (int64_t) blockDim.x + threadIdx.x) >> 5;
-	const int64_t nw = ((int64_t) gridDim.x * blockDim.x) >> 5;
-	for (int64_t ni = lb + gw; ni < le; ni += nw) {
-		const NodeW nd = nodes[ni];
-		const int nparts = nd.pend - nd.pbeg;
-		const double* gb = gbox + 6 * ni;
-		if (nd.child < 0) {
-			continue;
+// Component k of a stored multipole of orders < Q belongs to part 0..3 by the parities of its exponents:
+// the projection of a shifted multipole onto its traceless part mixes components of equal parities only,
+// so that a warp evaluating one part needs a quarter of the operator.
+template<int Q>
+__host__ __device__ constexpr int m2m_part(int k) {
+	if (k == Q * Q) {
+		return 3;  // (0, 0, 2)
+	}
+	const int c = k >= Q * (Q + 1) / 2;
+	int r = c ? k - Q * (Q + 1) / 2 : k, s = 0;
+	while (r >= s + 1) {
+		r -= s + 1;
+		s++;
+	}
+	const int a = (s - r) & 1, b = r & 1;  // (l, m, n) = (s - r, r, c)
+	return a == b && b == c ? 3 : a + b + c == 1 ? (a ? 0 : b ? 1 : 2) : (!a ? 0 : !b ? 1 : 2);
+}
+// One part of the shift of a child's multipole to the centre of its parent: lanes 2 i and 2 i + 1 take
+// the left and right child of a node, and the left one's stores the sum.
+template<class Ops, int PART>
+__device__ __forceinline__ void m2m_store(float* out, const float* Ma_, double x, double y, double z, bool on, bool left) {
+	constexpr int NM = Ops::NMULT, Q = Ops::ORDER - 1;
+	// the operator's other outputs are never formed (the compiler drops what nothing reads)
+	double Mo[NM];
+#pragma unroll
+	for (int k = 0; k < NM; k++) {
+		Mo[k] = 0.0;
+	}
+	if (on) {
+		double Ma[NM];
+#pragma unroll
+		for (int k = 0; k < NM; k++) {
+			Ma[k] = (double) Ma_[k];
 		}
-		{
-			// ---- interior node (tree.cpp:351-497)
-			const int64_t L = nd.child, R = nd.child + 1;
-			const NodeW nl = nodes[L], nr = nodes[R];
-			const float ml0 = multi[NMULT_STRIDE * L], mr0 = multi[NMULT_STRIDE * R];
-			double bb[3], be[3];
-			for (int d = 0; d < 3; d++) {
-				const double lb_ = tbox[6 * L + d], le_ = tbox[6 * L + 3 + d];
-				const double rb_ = tbox[6 * R + d], re_ = tbox[6 * R + 3 + d];
-				if (ml0 != 0.0f && mr0 != 0.0f) {
-					bb[d] = fmin(lb_, rb_);
-					be[d] = fmax(le_, re_);
-				} else if (ml0 != 0.0f) {
-					bb[d] = lb_;
-					be[d] = le_;
-				} else {
-					bb[d] = rb_;
-					be[d] = re_;
-				}
+		Ops::m2m(Mo, Ma, x, y, z);
+	}
+	static_for<0, NM>([&](auto c) {
+		constexpr int k = decltype(c)::value;
+		if constexpr (m2m_part<Q>(k) == PART) {
+			const double right = __shfl_down_sync(0xffffffffu, Mo[k], 1);
+			if (on && left) {
+				out[k] = (float) (Mo[k] + right);
 			}
-			int xdim = 0;
-			{
-				double max_span = -1.0;
+		}
+	});
+}
+
+constexpr int UPS_TPB = 256;
+constexpr int UPS_NODES = 32;    // nodes of a block, at most
+constexpr int UPS_ALONE = 256;   // particles that one warp goes through by itself
+
+// The interior nodes of one level (tree.cpp:351-497): union of the children's tight boxes, expansion
+// centre and radius, M2M of the two children in double.  A block takes `group` nodes: a thread each
+// for the boxes and centres, a warp each for the pass over the particles (or all eight, where a node
+// has more than UPS_ALONE), and for the shifts 32 lanes for 16 nodes' 32 children, in four warps of a
+// part of the components each.  With a warp a node, two of whose lanes shifted, levels of many nodes
+// were bound by the issue of double operations (430 us at 33,000 nodes) and a large node's pass by 256
+// dependent reads.  All levels, order 7: 256^3 particles 2,275 us -> 1,580; 64 boxes of 64^3 930 -> 610; a
+// 64^3 box's upper rungs 575 -> 230; 16^3 81 -> 77 (5 to 8 us a level: one chain of reads, roots and the shift).
+template<class Ops>
+__global__ void __launch_bounds__(UPS_TPB, 2) k_upsweep(int64_t lb, int64_t le, int group, NodeW* nodes, int32_t* nbox, float* multi, double* tbox, const double* gbox,
+		const uint32_t* x0, const uint32_t* x1, const uint32_t* x2, int bucket) {
+	__shared__ uint32_t s_xc[UPS_NODES][3];
+	__shared__ int s_beg[UPS_NODES], s_end[UPS_NODES];  // particles to go through
+	__shared__ unsigned int s_r2[UPS_NODES];            // largest squared distance (a positive float orders like its bits)
+	__shared__ int s_child[UPS_NODES];
+	__shared__ double s_X[UPS_NODES][3];
+	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+	const int64_t ngroups = (le - lb + group - 1) / group;
+	for (int64_t gi = blockIdx.x; gi < ngroups; gi += gridDim.x) {
+		const int64_t first = lb + gi * group;
+		const int cnt = (int) (le - first < group ? le - first : group);
+		const int64_t ni = first + threadIdx.x;  // the node of threads 0 .. cnt - 1
+		const bool own = (int) threadIdx.x < cnt;
+		NodeW nd, nl, nr;
+		float ml0 = 0.f, mr0 = 0.f;
+		double bb[3], be[3], Xc1[3];
+		bool inner = false, tried1 = false;
+		__syncthreads();
+		if (own) {
+			nd = nodes[ni];
+			inner = nd.child >= 0;
+			if (inner) {
+				const int64_t L = nd.child, R = nd.child + 1;
+				nl = nodes[L];
+				nr = nodes[R];
+				ml0 = multi[NMULT_STRIDE * L];
+				mr0 = multi[NMULT_STRIDE * R];
+				for (int d = 0; d < 3; d++) {
+					const double lb_ = tbox[6 * L + d], le_ = tbox[6 * L + 3 + d];
+					const double rb_ = tbox[6 * R + d], re_ = tbox[6 * R + 3 + d];
+					if (ml0 != 0.0f && mr0 != 0.0f) {
+						bb[d] = fmin(lb_, rb_);
+						be[d] = fmax(le_, re_);
+					} else if (ml0 != 0.0f) {
+						bb[d] = lb_;
+						be[d] = le_;
+					} else {
+						bb[d] = rb_;
+						be[d] = re_;
+					}
+				}
+				const double* gb = gbox + 6 * ni;
+				double max_span = -1.0, extent = 0.0;
 				for (int d = 0; d < 3; d++) {
 					const double span = gb[3 + d] - gb[d];
 					if (span > max_span) {
 						max_span = span;
-						xdim = d;
+						extent = be[d] - bb[d];
 					}
 				}
-			}
-			const bool tried1 = nparts <= 64 * bucket && (be[xdim] - bb[xdim] <= 0.5);
-			double Xc1[3];
-			float r2max = 0.0f;
-			if (tried1) {
-				uint32_t xc[3];
+				tried1 = nd.pend - nd.pbeg <= 64 * bucket && extent <= 0.5;
 				for (int d = 0; d < 3; d++) {
 					Xc1[d] = 0.5 * (bb[d] + be[d]);
-					xc[d] = fixed_from_double(Xc1[d]);
+					s_xc[threadIdx.x][d] = fixed_from_double(Xc1[d]);
 				}
+			}
+			s_child[threadIdx.x] = inner ? nd.child : -1;
+			s_beg[threadIdx.x] = tried1 ? nd.pbeg : 0;
+			s_end[threadIdx.x] = tried1 ? nd.pend : 0;
+			s_r2[threadIdx.x] = 0u;
+		}
+		__syncthreads();
+		for (int i = 0; i < cnt; i++) {
+			const int pb = s_beg[i], pe = s_end[i];
+			const bool alone = pe - pb <= UPS_ALONE;
+			if (pe == pb || (alone && (i & 7) != w)) {
+				continue;
+			}
+			const uint32_t cx = s_xc[i][0], cy = s_xc[i][1], cz = s_xc[i][2];
+			float r2max = 0.0f;
 #pragma unroll 4
-				for (int p = nd.pbeg + lane; p < nd.pend; p += 32) {
-					const float dx = fixed_dist(x0[p], xc[0]);
-					const float dy = fixed_dist(x1[p], xc[1]);
-					const float dz = fixed_dist(x2[p], xc[2]);
-					const float r2 = dx * dx + dy * dy + dz * dz;
-					r2max = fmaxf(r2max, r2);
-				}
-				r2max = warp_max(r2max);
+			for (int p = pb + (alone ? lane : (int) threadIdx.x); p < pe; p += alone ? 32 : UPS_TPB) {
+				const float dx = fixed_dist(x0[p], cx);
+				const float dy = fixed_dist(x1[p], cy);
+				const float dz = fixed_dist(x2[p], cz);
+				const float r2 = dx * dx + dy * dy + dz * dz;
+				r2max = fmaxf(r2max, r2);
 			}
-			double sX[3];
-			{
-				const double Xl[3] = { fixed_to_double(nl.x), fixed_to_double(nl.y), fixed_to_double(nl.z) };
-				const double Xr[3] = { fixed_to_double(nr.x), fixed_to_double(nr.y), fixed_to_double(nr.z) };
-				const double radius1 = tried1 ? (double) sqrtf(r2max) : 0.0;
-				double N[3];
-				double norminv = 0.0;
-				for (int d = 0; d < 3; d++) {
-					N[d] = Xl[d] - Xr[d];
-					norminv += N[d] * N[d];
-				}
-				norminv = 1.0 / sqrt(norminv);
-				for (int d = 0; d < 3; d++) {
-					N[d] *= norminv;
-					N[d] = fabs(N[d]);
-				}
-				double r = 0.0, Xc2[3];
-				const double Rl = nl.radius, Rr = nr.radius;
-				if (mr0 != 0.0f) {
-					if (ml0 != 0.0f) {
-						for (int d = 0; d < 3; d++) {
-							const double a = Xl[d] + N[d] * Rl, b = Xr[d] + N[d] * Rr;
-							const double xmax = (a < b) ? b : a;  // std::max
-							const double c = Xl[d] - N[d] * Rl, e = Xr[d] - N[d] * Rr;
-							const double xmin = (e < c) ? e : c;  // std::min
-							Xc2[d] = (xmax + xmin) * 0.5;
-							const double t = (xmax - xmin) * 0.5;
-							r += t * t;
-						}
-					} else {
-						for (int d = 0; d < 3; d++) {
-							Xc2[d] = Xr[d];
-						}
-						r = Rr * Rr;
+			r2max = warp_max(r2max);
+			if (lane == 0) {
+				atomicMax(s_r2 + i, __float_as_uint(r2max));
+			}
+		}
+		__syncthreads();
+		if (inner) {
+			const double Xl[3] = { fixed_to_double(nl.x), fixed_to_double(nl.y), fixed_to_double(nl.z) };
+			const double Xr[3] = { fixed_to_double(nr.x), fixed_to_double(nr.y), fixed_to_double(nr.z) };
+			const double radius1 = tried1 ? (double) sqrtf(__uint_as_float(s_r2[threadIdx.x])) : 0.0;
+			double N[3];
+			double norminv = 0.0;
+			for (int d = 0; d < 3; d++) {
+				N[d] = Xl[d] - Xr[d];
+				norminv += N[d] * N[d];
+			}
+			norminv = 1.0 / sqrt(norminv);
+			for (int d = 0; d < 3; d++) {
+				N[d] *= norminv;
+				N[d] = fabs(N[d]);
+			}
+			double r = 0.0, Xc2[3];
+			const double Rl = nl.radius, Rr = nr.radius;
+			if (mr0 != 0.0f) {
+				if (ml0 != 0.0f) {
+					for (int d = 0; d < 3; d++) {
+						const double a = Xl[d] + N[d] * Rl, b = Xr[d] + N[d] * Rr;
+						const double xmax = (a < b) ? b : a;  // std::max
+						const double c = Xl[d] - N[d] * Rl, e = Xr[d] - N[d] * Rr;
+						const double xmin = (e < c) ? e : c;  // std::min
+						Xc2[d] = (xmax + xmin) * 0.5;
+						const double t = (xmax - xmin) * 0.5;
+						r += t * t;
 					}
 				} else {
 					for (int d = 0; d < 3; d++) {
-						Xc2[d] = Xl[d];
+						Xc2[d] = Xr[d];
 					}
-					r = Rl * Rl;
+					r = Rr * Rr;
 				}
-				const double radius2 = sqrt(r);
-				double Xc[3];
-				float radius;
-				if (tried1 && radius1 < radius2) {
-					for (int d = 0; d < 3; d++) {
-						Xc[d] = Xc1[d];
-					}
-					radius = (float) radius1;
-				} else {
-					for (int d = 0; d < 3; d++) {
-						Xc[d] = Xc2[d];
-					}
-					radius = (float) radius2;
-				}
-				r = 0.0;
+			} else {
 				for (int d = 0; d < 3; d++) {
-					const double span = be[d] - bb[d];
-					r += (span * 0.5) * (span * 0.5);
+					Xc2[d] = Xl[d];
 				}
-				r = sqrt(r);
-				if (r < radius) {
-					radius = (float) r;
-					for (int d = 0; d < 3; d++) {
-						Xc[d] = (bb[d] + be[d]) * 0.5;
-					}
-				}
+				r = Rl * Rl;
+			}
+			const double radius2 = sqrt(r);
+			const bool use1 = tried1 && radius1 < radius2;
+			double Xc[3];
+			float radius = (float) (use1 ? radius1 : radius2);
+			for (int d = 0; d < 3; d++) {
+				Xc[d] = use1 ? Xc1[d] : Xc2[d];
+			}
+			r = 0.0;
+			for (int d = 0; d < 3; d++) {
+				const double span = be[d] - bb[d];
+				r += (span * 0.5) * (span * 0.5);
+			}
+			r = sqrt(r);
+			if (r < radius) {
+				radius = (float) r;
 				for (int d = 0; d < 3; d++) {
-					sX[d] = Xc[d];
-				}
-				NodeW o = nd;
-				o.x = fixed_from_double(Xc[0]);
-				o.y = fixed_from_double(Xc[1]);
-				o.z = fixed_from_double(Xc[2]);
-				o.radius = radius;
-				if (lane == 0) {
-					nodes[ni] = o;
-					for (int d = 0; d < 3; d++) {
-						tbox[6 * ni + d] = bb[d];
-						tbox[6 * ni + 3 + d] = be[d];
-						nbox[6 * ni + d] = range_fixed_from_double(bb[d]);
-						nbox[6 * ni + 3 + d] = range_fixed_from_double(be[d]);
-					}
+					Xc[d] = (bb[d] + be[d]) * 0.5;
 				}
 			}
-			// M2M of both children in double (tree.cpp:481-494): lane 0 the left, lane 1 the right,
-			// then left + right
-			double Mo[NM];
-			for (int k = 0; k < NM; k++) {
-				Mo[k] = 0.0;
+			NodeW o = nd;
+			o.x = fixed_from_double(Xc[0]);
+			o.y = fixed_from_double(Xc[1]);
+			o.z = fixed_from_double(Xc[2]);
+			o.radius = radius;
+			nodes[ni] = o;
+			for (int d = 0; d < 3; d++) {
+				s_X[threadIdx.x][d] = Xc[d];
+				tbox[6 * ni + d] = bb[d];
+				tbox[6 * ni + 3 + d] = be[d];
+				nbox[6 * ni + d] = range_fixed_from_double(bb[d]);
+				nbox[6 * ni + 3 + d] = range_fixed_from_double(be[d]);
 			}
-			if (lane < 2) {
-				const int64_t c = lane == 0 ? L : R;
-				const NodeW cn = lane == 0 ? nl : nr;
-				double Ma[NM];
-				for (int k = 0; k < NM; k++) {
-					Ma[k] = (double) multi[NMULT_STRIDE * c + k];
-				}
-				Ops::m2m(Mo, Ma, fixed_to_double(cn.x) - sX[0], fixed_to_double(cn.y) - sX[1], fixed_to_double(cn.z) - sX[2]);
+		}
+		__syncthreads();
+		// M2M of both children in double (tree.cpp:481-494), left + right
+		const int i = 16 * (w >> 2) + (lane >> 1);
+		if (16 * (w >> 2) < cnt) {
+			const int child = i < cnt ? s_child[i] : -1;
+			const bool on = child >= 0, left = !(lane & 1);
+			const int64_t c = on ? child + (lane & 1) : 0;
+			double x = 0.0, y = 0.0, z = 0.0;
+			if (on) {
+				const NodeW cn = nodes[c];
+				x = fixed_to_double(cn.x) - s_X[i][0];
+				y = fixed_to_double(cn.y) - s_X[i][1];
+				z = fixed_to_double(cn.z) - s_X[i][2];
 			}
-			for (int k = 0; k < NM; k++) {
-				const double right = __shfl_down_sync(0xffffffffu, Mo[k], 1);
-				if (lane == 0) {
-					multi[NMULT_STRIDE * ni + k] = (float) (Mo[k] + right);
-				}
+			const float* Ma = multi + NMULT_STRIDE * c;
+			float* out = multi + NMULT_STRIDE * (first + i);
+			switch (w & 3) {
+			case 0:
+				m2m_store<Ops, 0>(out, Ma, x, y, z, on, left);
+				break;
+			case 1:
+				m2m_store<Ops, 1>(out, Ma, x, y, z, on, left);
+				break;
+			case 2:
+				m2m_store<Ops, 2>(out, Ma, x, y, z, on, left);
+				break;
+			default:
+				m2m_store<Ops, 3>(out, Ma, x, y, z, on, left);
 			}
 		}
 	}
@@ -1206,7 +1280,10 @@ ct_status tree_build_t(Ctx* c, Box* b, const ct_tree_params* p) {
 			continue;  // the deepest level is all leaves
 		}
 		c->launches++;
-		k_upsweep<Ops><<<(int) std::min<int64_t>((e - a + UTPB / 32 - 1) / (UTPB / 32), (int64_t) c->nsm * 16), UTPB, 0, st>>>(a, e, b->nodes, b->nbox, b->multi,
+		// as many nodes a block as leave four blocks an SM (two are resident): a level of few nodes is a
+		// block each, so that the passes over the particles run side by side
+		const int group = (int) std::max<int64_t>(1, std::min<int64_t>(UPS_NODES, (e - a) / (4 * c->nsm)));
+		k_upsweep<Ops><<<(int) std::min<int64_t>((e - a + group - 1) / group, (int64_t) c->nsm * 64), UPS_TPB, 0, st>>>(a, e, group, b->nodes, b->nbox, b->multi,
 				b->tbox, b->gbox, b->x[0], b->x[1], b->x[2], p->bucket);
 	}
 	CT_CUDA(c, cudaGetLastError());
