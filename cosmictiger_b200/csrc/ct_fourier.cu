@@ -374,88 +374,144 @@ __global__ void __launch_bounds__(FT_TPB) k_ic_lattice(int N, uint32_t* __restri
 // moves by dx (periodic) and the velocity by prefac dx.  Particle (I0 N + I1) N + I2 sits at
 // lattice point I, and the kernel's 6^3 weights there are products of per-axis weights that
 // depend only on I0, I1, I2, so the 216-term sum is taken as 6-term sums along x, y and z (double
-// precision, as the reference accumulates).  One block takes DISP_ROWS rows (x, y .. y + 7) of one
-// x: the x sums of the rows it needs (8 and their y neighbours) into shared memory, then per row the
-// y sums and, from those, the z sums and the update.  As three passes over double grids the same
-// sums moved 36 bytes a point through memory; here a point is read from the field (which the L2
-// keeps) and updated.  256^3: 1,260 us an axis with weights evaluated per point, now 90.
-// The largest dx in units of the mean spacing goes to dxmax (float bits: a positive float orders
-// like its bits).
+// precision, as the reference accumulates), in two passes: along x into a double grid, each thread
+// eight points of a line (a field value is read and converted to double 13 / 8 times; in one pass over
+// tiles 10 times); then y and z with the update, the y sums of DISP_ROWS rows of one x in shared memory,
+// where a thread keeps to one z and its columns.  256^3, an axis: 276 us in one pass, now 46 + 140,
+// against 90 for the bytes of both; four blocks an SM (2lpt 3.72 ms; two 3.88, three 3.80).  The largest
+// dx in units of the mean spacing goes to dxmax (float bits: a positive float orders like its bits).
 constexpr int DISP_ROWS = 8;
+constexpr int DISP_X = 8;
 
 // An index at most one grid length outside 0 .. n - 1.
 __device__ __forceinline__ int wrap1(int i, int n) {
 	return i < 0 ? i + n : (i >= n ? i - n : i);
 }
 
-__global__ void __launch_bounds__(FT_TPB, 5) k_ic_displace(int N, const float* __restrict__ R, AxisTables t, double scale, float D, float prefac,
-		double box_size_inv, uint32_t* __restrict__ X, float* __restrict__ V, unsigned int* dxmax) {
-	extern __shared__ double s_rows[];  // [rows][N] sums along x, then [N] sums along x and y
-	const int I0 = blockIdx.y, y0 = blockIdx.x * DISP_ROWS;
-	const int ny = min(DISP_ROWS, N - y0);
-	// rows y0's first neighbour .. the last row's last, wrapped (a lattice point's cell never falls
-	// by more than one below its index, and rises with it)
-	const int r0 = __ldg(t.cell + y0) + CLOUD_MIN;
-	const int nrow = __ldg(t.cell + y0 + ny - 1) + CLOUD_MAX - r0 + 1;  // at most DISP_ROWS + 6
-	double* s_y = s_rows + (size_t) (DISP_ROWS + 6) * N;
-	const int c0 = __ldg(t.cell + I0) + CLOUD_MIN;
-	int plane[6];  // (a grid has at most 2^30 points)
-	double wx[6];
-#pragma unroll
-	for (int j = 0; j < 6; j++) {
-		plane[j] = wrap1(c0 + j, N) * N * N;
-		wx[j] = __ldg(t.weight + j * N + I0);
+// Sums along x: points x0 .. x0 + 7 (x0 = 8 blockIdx.y) of the line (y, z).
+__global__ void __launch_bounds__(FT_TPB) k_ic_sum_x(int N, const float* __restrict__ R, AxisTables t, double* __restrict__ G) {
+	const int line = blockIdx.x * FT_TPB + threadIdx.x, plane = N * N;  // (a grid has at most 2^30 points)
+	if (line >= plane) {
+		return;
 	}
-	for (int r = 0; r < nrow; r++) {
-		const int p = wrap1(r0 + r, N) * N;
-		for (int z = threadIdx.x; z < N; z += FT_TPB) {
+	const int x0 = blockIdx.y * DISP_X, nx = min(DISP_X, N - x0);
+	const int c0 = __ldg(t.cell + x0);
+	// a lattice point's cell is its index or, where I / N rounds below itself, one less
+	bool regular = nx == DISP_X;
+	for (int i = 1; i < nx; i++) {
+		regular = regular && __ldg(t.cell + x0 + i) == c0 + i;
+	}
+	if (regular) {
+		double v[DISP_X + 5];
+#pragma unroll
+		for (int j = 0; j < DISP_X + 5; j++) {
+			v[j] = (double) R[wrap1(c0 + CLOUD_MIN + j, N) * plane + line];
+		}
+#pragma unroll
+		for (int i = 0; i < DISP_X; i++) {
 			double acc = 0.0;
 #pragma unroll
 			for (int j = 0; j < 6; j++) {
-				acc += wx[j] * (double) R[plane[j] + p + z];
+				acc += __ldg(t.weight + j * N + x0 + i) * v[i + j];
 			}
-			s_rows[r * N + z] = acc;
+			G[(x0 + i) * plane + line] = acc;
+		}
+	} else {
+		for (int i = 0; i < nx; i++) {
+			const int c = __ldg(t.cell + x0 + i) + CLOUD_MIN;
+			double acc = 0.0;
+#pragma unroll
+			for (int j = 0; j < 6; j++) {
+				acc += __ldg(t.weight + j * N + x0 + i) * (double) R[wrap1(c + j, N) * plane + line];
+			}
+			G[(x0 + i) * plane + line] = acc;
+		}
+	}
+}
+
+// Sums along y and z, scaled by the inverse transform's normalisation, and the update of rows
+// (x, 8 blockIdx.x ..) of x = blockIdx.y.
+__global__ void __launch_bounds__(FT_TPB, 4) k_ic_displace(int N, const double* __restrict__ G, AxisTables t, double scale, float D, float prefac,
+		double box_size_inv, uint32_t* __restrict__ X, float* __restrict__ V, unsigned int* dxmax) {
+	extern __shared__ double s_y[];  // [DISP_ROWS][N]
+	const int x = blockIdx.y, y0 = blockIdx.x * DISP_ROWS;
+	const int ny = min(DISP_ROWS, N - y0);
+	const int c0 = __ldg(t.cell + y0);
+	bool regular = ny == DISP_ROWS;
+	for (int i = 1; i < ny; i++) {
+		regular = regular && __ldg(t.cell + y0 + i) == c0 + i;
+	}
+	for (int z = threadIdx.x; z < N; z += FT_TPB) {
+		const double* col = G + (size_t) x * N * N + z;
+		if (regular) {
+			double v[DISP_ROWS + 5];
+#pragma unroll
+			for (int j = 0; j < DISP_ROWS + 5; j++) {
+				v[j] = col[wrap1(c0 + CLOUD_MIN + j, N) * N];
+			}
+#pragma unroll
+			for (int i = 0; i < DISP_ROWS; i++) {
+				double acc = 0.0;
+#pragma unroll
+				for (int j = 0; j < 6; j++) {
+					acc += __ldg(t.weight + j * N + y0 + i) * v[i + j];
+				}
+				s_y[i * N + z] = acc;
+			}
+		} else {
+			for (int i = 0; i < ny; i++) {
+				const int c = __ldg(t.cell + y0 + i) + CLOUD_MIN;
+				double acc = 0.0;
+#pragma unroll
+				for (int j = 0; j < 6; j++) {
+					acc += __ldg(t.weight + j * N + y0 + i) * col[wrap1(c + j, N) * N];
+				}
+				s_y[i * N + z] = acc;
+			}
 		}
 	}
 	__syncthreads();
 	float mymax = 0.f;
-	for (int y = 0; y < ny; y++) {
-		const int first = __ldg(t.cell + y0 + y) + CLOUD_MIN - r0;
-		double wy[6];
+	for (int z = threadIdx.x; z < N; z += FT_TPB) {
+		const int p0 = (x * N + y0) * N + z;
+		// the rows' positions and velocities are read before any is written: a read behind a write that
+		// might be to the same place waits for it, eight trips to memory one after another
+		uint32_t xr[DISP_ROWS];
+		float vr[DISP_ROWS];
+#pragma unroll
+		for (int y = 0; y < DISP_ROWS; y++) {
+			xr[y] = y < ny ? X[p0 + y * N] : 0u;
+			vr[y] = y < ny ? V[p0 + y * N] : 0.f;
+		}
+		const int c = __ldg(t.cell + z) + CLOUD_MIN;
+		int at[6];
+		double wz[6];
 #pragma unroll
 		for (int j = 0; j < 6; j++) {
-			wy[j] = __ldg(t.weight + j * N + y0 + y);
+			at[j] = wrap1(c + j, N);
+			wz[j] = __ldg(t.weight + j * N + z);
 		}
-		for (int z = threadIdx.x; z < N; z += FT_TPB) {
-			double acc = 0.0;
 #pragma unroll
-			for (int j = 0; j < 6; j++) {
-				acc += wy[j] * s_rows[(first + j) * N + z];
-			}
-			s_y[z] = acc;
-		}
-		__syncthreads();
-		const int base = (I0 * N + y0 + y) * N;
-		for (int z = threadIdx.x; z < N; z += FT_TPB) {
-			const int c = __ldg(t.cell + z) + CLOUD_MIN;
-			double dx = 0.0;
+		for (int y = 0; y < DISP_ROWS; y++) {
+			if (y < ny) {
+				double dx = 0.0;
 #pragma unroll
-			for (int j = 0; j < 6; j++) {
-				dx += __ldg(t.weight + j * N + z) * s_y[wrap1(c + j, N)];
+				for (int j = 0; j < 6; j++) {
+					dx += wz[j] * s_y[y * N + at[j]];
+				}
+				dx *= scale;
+				dx *= -D * box_size_inv;
+				double q = fixed_to_double(xr[y]) + dx;
+				if (q >= 1.0) {
+					q -= 1.0;
+				} else if (q < 0.0) {
+					q += 1.0;
+				}
+				X[p0 + y * N] = fixed_from_double(q);
+				V[p0 + y * N] = (float) (vr[y] + prefac * dx);
+				mymax = fmaxf(mymax, (float) (dx * N));
 			}
-			dx *= scale;
-			dx *= -D * box_size_inv;
-			double x = fixed_to_double(X[base + z]) + dx;
-			if (x >= 1.0) {
-				x -= 1.0;
-			} else if (x < 0.0) {
-				x += 1.0;
-			}
-			X[base + z] = fixed_from_double(x);
-			V[base + z] += prefac * dx;
-			mymax = fmaxf(mymax, (float) (dx * N));
 		}
-		__syncthreads();
 	}
 	for (int o = 16; o; o >>= 1) {
 		mymax = fmaxf(mymax, __shfl_xor_sync(0xffffffffu, mymax, o));
@@ -1076,11 +1132,13 @@ extern "C" ct_status ct_initialize(ct_ctx* ctx, int box_id, const ct_ic_params* 
 	cufftComplex* Y = nullptr;
 	float* R = nullptr;
 	AxisTables ax = {};
+	double* G = nullptr;
 	unsigned int* dmax = nullptr;  // six displacement maxima, then the table's factor
 	CT_TRY(S.alloc(&dP, P.size(), "power table"));
 	CT_TRY(S.alloc(&A, ncx, "mode amplitudes"));
 	CT_TRY(S.alloc(&Y, ncx, "k-space field"));
 	CT_TRY(S.alloc(&R, n, "real-space field"));
+	CT_TRY(S.alloc(&G, n, "interpolation pass"));
 	CT_TRY(S.alloc(&ax.filter, N, "axis tables"));
 	CT_TRY(S.alloc(&ax.cell, N, "axis tables"));
 	CT_TRY(S.alloc(&ax.weight, 6 * (size_t) N, "axis tables"));
@@ -1102,11 +1160,12 @@ extern "C" ct_status ct_initialize(ct_ctx* ctx, int box_id, const ct_ic_params* 
 	k_ic_uniforms<<<ft_grid(c, (int64_t) N * N), FT_TPB, 0, st>>>(N, A);
 	k_ic_amplitude<<<gx, FT_TPB, 0, st>>>(N, box, factor, dtab, A);
 	// interpolation at the lattice points and update of axis dim
-	const size_t disp_smem = sizeof(double) * (DISP_ROWS + 7) * N;  // 120 KB at the largest grid
+	const size_t disp_smem = sizeof(double) * DISP_ROWS * N;  // 64 KB at the largest grid
 	CT_CUDA(c, cudaFuncSetAttribute(k_ic_displace, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) disp_smem));
 	auto displace = [&](int dim, float D, float prefac, unsigned int* mx) {
-		c->launches++;
-		k_ic_displace<<<dim3((N + DISP_ROWS - 1) / DISP_ROWS, N), FT_TPB, disp_smem, st>>>(N, R, ax, scale, D, prefac, box_inv, b->x[dim], b->v[dim], mx);
+		c->launches += 2;
+		k_ic_sum_x<<<dim3((N * N + FT_TPB - 1) / FT_TPB, (N + DISP_X - 1) / DISP_X), FT_TPB, 0, st>>>(N, R, ax, G);
+		k_ic_displace<<<dim3((N + DISP_ROWS - 1) / DISP_ROWS, N), FT_TPB, disp_smem, st>>>(N, G, ax, scale, D, prefac, box_inv, b->x[dim], b->v[dim], mx);
 	};
 	// the field of dim1, dim2 in real space
 	auto field = [&](int dim1, int dim2, float* out) {
