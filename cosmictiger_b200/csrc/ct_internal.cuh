@@ -193,6 +193,31 @@ inline float elapsed_ms(cudaEvent_t a, cudaEvent_t b) {
 // Frees the context's kick buffers (called by ct_ctx_destroy).
 void kick_buffers_release(Ctx* c);
 
+// Kernels launched one after another for the levels of a tree, where a launch takes as long as a level
+// of few nodes: with launch_behind a grid starts while the one before it in the stream runs, and waits
+// in front_done, its first statement, until that one has ended and its writes can be seen.  (A grid
+// starts once all blocks of the one before have, so the earlier one never waits for room.)  One
+// 16^3 step: walk 111 -> 77 us (11 levels), L2L 60 -> 36, upsweep some 20 less, the call 896 -> 812.
+#ifdef __CUDACC__
+__device__ __forceinline__ void front_done() {
+	cudaTriggerProgrammaticLaunchCompletion();
+	cudaGridDependencySynchronize();
+}
+template<class... P, class... A>
+inline cudaError_t launch_behind(void (*kernel)(P...), int blocks, int threads, cudaStream_t st, const A&... args) {
+	cudaLaunchAttribute attr = {};
+	attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	attr.val.programmaticStreamSerializationAllowed = 1;
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = dim3(blocks);
+	cfg.blockDim = dim3(threads);
+	cfg.stream = st;
+	cfg.attrs = &attr;
+	cfg.numAttrs = 1;
+	return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+#endif
+
 // Allocation with budget accounting.
 ct_status dalloc(Ctx* c, void** p, size_t bytes, const char* what);
 void dfree(Ctx* c, void* p, size_t bytes);

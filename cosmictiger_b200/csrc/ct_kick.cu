@@ -104,7 +104,9 @@ struct WalkOut {
 	int* pp_list;
 	int* pass_cur;   // pass-down lists of this level (eout/dout)
 	int* pass_prev;  // pass-down lists of the level above
-	unsigned long long* cursor;  // [0] ecc [1] dcc [2] cp [3] pc [4] pp [5] pass (this level)
+	unsigned long long* cursor;  // [0] ecc [1] dcc [2] cp [3] pc [4] pp
+	unsigned long long* pass_cursor;  // pass-down entries of this level
+	unsigned long long* pass_next;    // of the next (cleared by this level)
 	long long cap_cc, cap_leaf, cap_pass;
 	int* stage;   // per-warp staging, NLIST * stage_cap ints per warp
 	int stage_cap;
@@ -224,6 +226,10 @@ struct CheckStream {
 
 __global__ void __launch_bounds__(WALK_TPB) k_walk(int64_t lb, int64_t le, const NodeW* __restrict__ nodes, const int32_t* __restrict__ nbox,
 		const int32_t* __restrict__ parent, WalkOut o, WalkParams p) {
+	front_done();
+	if (blockIdx.x == 0 && threadIdx.x == 0) {
+		*o.pass_next = 0;
+	}
 	const int lane = threadIdx.x & 31;
 	const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 	const int nw = (gridDim.x * blockDim.x) >> 5;
@@ -401,12 +407,12 @@ __global__ void __launch_bounds__(WALK_TPB) k_walk(int64_t lb, int64_t le, const
 			}
 		} else {
 			// Ewald pass-down: children of the opened checks
-			const int2 eo = flush(sl[S_EOUT], n_eout, cap, o.pass_cur, o.cursor + 5, o.cap_pass, lane, o.flags);
+			const int2 eo = flush(sl[S_EOUT], n_eout, cap, o.pass_cur, o.pass_cursor, o.cap_pass, lane, o.flags);
 			// direct pass-down: children of opened checks, then the leaf checks (kick.cu:424-430)
 			const int nn = min(n_next, cap), nl = min(n_leaf, cap);
 			unsigned long long off = 0;
 			if (lane == 0 && nn + nl) {
-				off = atomicAdd(o.cursor + 5, (unsigned long long) (nn + nl));
+				off = atomicAdd(o.pass_cursor, (unsigned long long) (nn + nl));
 			}
 			off = __shfl_sync(0xffffffffu, off, 0);
 			int2 dout = make_int2(0, 0);
@@ -821,6 +827,7 @@ __device__ __forceinline__ void l2l_part_of(int64_t i, const NodeW* __restrict__
 template<class Ops>
 __global__ void __launch_bounds__(32 * L2L_PARTS) k_l2l(int64_t lb, int64_t le, const NodeW* __restrict__ nodes, const int32_t* __restrict__ parent,
 		const float* __restrict__ dL, const float* __restrict__ dL2, const float* __restrict__ dL3, float* __restrict__ Lx, int do_phi) {
+	front_done();
 	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 	for (int64_t i = lb + blockIdx.x * (int64_t) 32 + lane; i < le; i += (int64_t) gridDim.x * 32) {
 		if (w == 0) {
@@ -1845,11 +1852,12 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 			const int64_t lb = b->level_start[k], le = b->level_start[k + 1];
 			o.pass_cur = K.pass + (k & 1) * K.cap_pass;
 			o.pass_prev = K.pass + ((k + 1) & 1) * K.cap_pass;
-			// pass-down cursor restarts every level (its buffer alternates)
-			CT_CUDA(c, cudaMemsetAsync(o.cursor + 5, 0, sizeof(unsigned long long), st));
+			// the pass-down cursor restarts every level (its buffer alternates, and so does it)
+			o.pass_cursor = o.cursor + 5 + (k & 1);
+			o.pass_next = o.cursor + 5 + ((k + 1) & 1);
 			const int64_t nwn = std::min<int64_t>((le - lb + 3) / 4, (int64_t) K.nwarps / 4);
 			c->launches++;
-			k_walk<<<(int) std::max<int64_t>(nwn, 1), WALK_TPB, 0, st>>>(lb, le, b->nodes, b->nbox, b->parent, o, wp);
+			CT_CUDA(c, launch_behind(k_walk, (int) std::max<int64_t>(nwn, 1), WALK_TPB, st, lb, le, b->nodes, b->nbox, b->parent, o, wp));
 		}
 		CT_CUDA(c, cudaGetLastError());
 		cudaEventRecord(c->ev[1], st);
@@ -1908,8 +1916,8 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 			const int64_t lb = b->level_start[k], le = b->level_start[k + 1];
 			const int64_t g = (le - lb + 31) / 32;
 			c->launches++;
-			k_l2l<Ops><<<(int) std::max<int64_t>(1, std::min<int64_t>(g, c->nsm * 16)), 32 * L2L_PARTS, 0, st>>>(lb, le, b->nodes, b->parent, K.dL, K.dL2, K.dL3,
-					K.Lx, kp->do_phi);
+			CT_CUDA(c, launch_behind(k_l2l<Ops>, (int) std::max<int64_t>(1, std::min<int64_t>(g, c->nsm * 16)), 32 * L2L_PARTS, st, lb, le, b->nodes, b->parent,
+					K.dL, K.dL2, K.dL3, K.Lx, kp->do_phi));
 		}
 		cudaEventRecord(c->ev[3], st);
 		// leaves' tiles; a binary tree of nn nodes and nsub roots has (nn + nsub) / 2 leaves

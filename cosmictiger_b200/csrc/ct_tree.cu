@@ -959,6 +959,7 @@ __global__ void __launch_bounds__(UPS_TPB, 2) k_upsweep(int64_t lb, int64_t le, 
 	__shared__ unsigned int s_r2[UPS_NODES];            // largest squared distance (a positive float orders like its bits)
 	__shared__ int s_child[UPS_NODES];
 	__shared__ double s_X[UPS_NODES][3];
+	front_done();
 	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 	const int64_t ngroups = (le - lb + group - 1) / group;
 	for (int64_t gi = blockIdx.x; gi < ngroups; gi += gridDim.x) {
@@ -1283,8 +1284,8 @@ ct_status tree_build_t(Ctx* c, Box* b, const ct_tree_params* p) {
 		// as many nodes a block as leave four blocks an SM (two are resident): a level of few nodes is a
 		// block each, so that the passes over the particles run side by side
 		const int group = (int) std::max<int64_t>(1, std::min<int64_t>(UPS_NODES, (e - a) / (4 * c->nsm)));
-		k_upsweep<Ops><<<(int) std::min<int64_t>((e - a + group - 1) / group, (int64_t) c->nsm * 64), UPS_TPB, 0, st>>>(a, e, group, b->nodes, b->nbox, b->multi,
-				b->tbox, b->gbox, b->x[0], b->x[1], b->x[2], p->bucket);
+		CT_CUDA(c, launch_behind(k_upsweep<Ops>, (int) std::min<int64_t>((e - a + group - 1) / group, (int64_t) c->nsm * 64), UPS_TPB, st, a, e, group, b->nodes,
+				b->nbox, b->multi, b->tbox, b->gbox, b->x[0], b->x[1], b->x[2], p->bucket));
 	}
 	CT_CUDA(c, cudaGetLastError());
 	CT_CUDA(c, cudaMemcpyAsync(h_tot, c->d_flags, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
