@@ -1,5 +1,4 @@
 // C ABI of the gravity step: contexts, boxes, transfers, drift, rung sort, direct Ewald.
-#include <cub/cub.cuh>
 
 #include <algorithm>
 #include <cstdio>

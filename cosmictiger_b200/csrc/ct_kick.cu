@@ -19,7 +19,6 @@
 //   k_leaf       M2P, P2P (sources staged in shared memory as floats relative to the leaf
 //                centre, compensated per-batch accumulation), L2P and the kick
 //                (gravity.cu:157-211,246-404, kick.cu:53-177).
-#include <cub/cub.cuh>
 #include <cstdlib>
 #include <mutex>
 
@@ -749,22 +748,99 @@ __global__ void __launch_bounds__(128, 5) k_p2l(int64_t nn, const int32_t* __res
 	}
 }
 
-// Sort keys of the three node orders: the bit length of the node's list length of each kind (P2L
-// lists count only at leaves), and the node indices to be sorted with them.  Sorting by the bit
-// length (a stable sort) puts the longest lists first and keeps tree order among lists of
-// similar length, so that warps working at the same time read nearby source nodes.
-constexpr int ORDER_KEY_BITS = 6;  // bit lengths 0..32
-__global__ void k_order_keys(int64_t nn, const NodeW* __restrict__ nodes, const int2* __restrict__ ecc, const int2* __restrict__ dcc,
-		const int2* __restrict__ cp, const int2* __restrict__ pp, uint32_t* __restrict__ key, int32_t* __restrict__ idx) {
-	for (int64_t i = blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < nn; i += (int64_t) gridDim.x * blockDim.x) {
-		const uint32_t le = (uint32_t) ecc[i].y, ld = (uint32_t) dcc[i].y, lp = (nodes[i].flags & 1) ? (uint32_t) cp[i].y : 0u;
-		key[i] = 32u - __clz(le);
-		key[nn + i] = 32u - __clz(ld);
-		key[2 * nn + i] = 32u - __clz(lp);
-		// leaves with particles by their source leaves times sinks (at least 1)
-		const uint32_t np = (uint32_t) (nodes[i].pend - nodes[i].pbeg);
-		key[3 * nn + i] = (nodes[i].flags & 1) && np ? 32u - __clz(max(1u, (uint32_t) min(0x7fffffffull, (unsigned long long) pp[i].y * np))) : 0u;
-		idx[i] = (int32_t) i;
+// The node orders of the node-indexed kernels: nodes by the bit length of their list of a kind, longest
+// first, and about in tree order among lists of similar length, so that warps working at the same time
+// read nearby source nodes.  Kinds: Ewald M2L, direct M2L, P2L (leaves only), P2P (leaves with
+// particles, by source leaves times sinks, at least 1).  A count and a placing, each a launch over all
+// four kinds (one block does both when it holds the nodes); a block's nodes keep together.  Four radix
+// sorts of the same keys took 20 us for up to 3,000 nodes and 75 above, most of it launches.
+constexpr int ORDER_KINDS = 4;
+constexpr int ORDER_BINS = 33;  // bit lengths 0..32
+constexpr int ORDER_TPB = 1024;
+constexpr int ORDER_ITEMS = 4;  // nodes a thread
+constexpr int ORDER_SPAN = ORDER_TPB * ORDER_ITEMS;
+
+struct OrderArgs {
+	int64_t nn;
+	const NodeW* nodes;
+	const int2 *ecc, *dcc, *cp, *pp;
+	int32_t* order;  // [ORDER_KINDS][nn]
+	int* count;      // [ORDER_KINDS][ORDER_BINS] nodes, then as many placed so far (zero before)
+};
+__device__ __forceinline__ void order_keys(const OrderArgs& a, int64_t i, int (&key)[ORDER_KINDS]) {
+	const NodeW nd = a.nodes[i];
+	const bool leaf = nd.flags & 1;
+	const uint32_t np = (uint32_t) (nd.pend - nd.pbeg);
+	key[0] = 32 - __clz((uint32_t) a.ecc[i].y);
+	key[1] = 32 - __clz((uint32_t) a.dcc[i].y);
+	key[2] = leaf ? 32 - __clz((uint32_t) a.cp[i].y) : 0;
+	key[3] = leaf && np ? 32 - __clz(max(1u, (uint32_t) min(0x7fffffffull, (unsigned long long) a.pp[i].y * np))) : 0;
+}
+// Counts the block's nodes into s_hist; rank: each node's place among the block's of its kind and bin.
+__device__ __forceinline__ void order_count(const OrderArgs& a, int (*s_hist)[ORDER_BINS], int (*key)[ORDER_KINDS], int (*rank)[ORDER_KINDS]) {
+	const int lane = threadIdx.x & 31;
+	for (int e = threadIdx.x; e < ORDER_KINDS * ORDER_BINS; e += ORDER_TPB) {
+		s_hist[0][e] = 0;
+	}
+	__syncthreads();
+#pragma unroll
+	for (int t = 0; t < ORDER_ITEMS; t++) {
+		const int64_t i = blockIdx.x * (int64_t) ORDER_SPAN + t * ORDER_TPB + threadIdx.x;
+		const bool on = i < a.nn;
+		if (on) {
+			order_keys(a, i, key[t]);
+		}
+#pragma unroll
+		for (int k = 0; k < ORDER_KINDS; k++) {
+			key[t][k] = on ? key[t][k] : ORDER_BINS;
+			const unsigned same = __match_any_sync(0xffffffffu, key[t][k]);
+			const int first = __ffs(same) - 1;
+			int at = 0;
+			if (on && lane == first) {
+				at = atomicAdd(&s_hist[k][key[t][k]], __popc(same));
+			}
+			rank[t][k] = __shfl_sync(0xffffffffu, at, first) + __popc(same & ((1u << lane) - 1u));
+		}
+	}
+	__syncthreads();
+}
+__global__ void __launch_bounds__(ORDER_TPB) k_order_count(const OrderArgs a) {
+	__shared__ int s_hist[ORDER_KINDS][ORDER_BINS];
+	int key[ORDER_ITEMS][ORDER_KINDS], rank[ORDER_ITEMS][ORDER_KINDS];
+	front_done();
+	order_count(a, s_hist, key, rank);
+	for (int e = threadIdx.x; e < ORDER_KINDS * ORDER_BINS; e += ORDER_TPB) {
+		if (s_hist[0][e]) {
+			atomicAdd(a.count + e, s_hist[0][e]);
+		}
+	}
+}
+__global__ void __launch_bounds__(ORDER_TPB) k_order_place(const OrderArgs a) {
+	__shared__ int s_hist[ORDER_KINDS][ORDER_BINS], s_at[ORDER_KINDS][ORDER_BINS];
+	int key[ORDER_ITEMS][ORDER_KINDS], rank[ORDER_ITEMS][ORDER_KINDS];
+	front_done();
+	order_count(a, s_hist, key, rank);
+	for (int e = threadIdx.x; e < ORDER_KINDS * ORDER_BINS; e += ORDER_TPB) {
+		const int k = e / ORDER_BINS, bin = e - k * ORDER_BINS;
+		int at = 0;  // the nodes of longer lists
+		for (int q = bin + 1; q < ORDER_BINS; q++) {
+			at += gridDim.x == 1 ? s_hist[k][q] : a.count[k * ORDER_BINS + q];
+		}
+		if (gridDim.x > 1 && s_hist[k][bin]) {
+			at += atomicAdd(a.count + ORDER_KINDS * ORDER_BINS + e, s_hist[k][bin]);
+		}
+		s_at[k][bin] = at;
+	}
+	__syncthreads();
+#pragma unroll
+	for (int t = 0; t < ORDER_ITEMS; t++) {
+		const int64_t i = blockIdx.x * (int64_t) ORDER_SPAN + t * ORDER_TPB + threadIdx.x;
+		if (i < a.nn) {
+#pragma unroll
+			for (int k = 0; k < ORDER_KINDS; k++) {
+				a.order[k * a.nn + s_at[k][key[t][k]] + rank[t][k]] = (int32_t) i;
+			}
+		}
 	}
 }
 
@@ -1865,26 +1941,21 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 		// and the leaf kick changes nothing if something did not)
 		// ---- interactions
 		CT_CUDA(c, cudaMemsetAsync(counters, 0, 16 * sizeof(double), st));
-		// node orders of the node-indexed kernels, longest lists first (radix sort of the
-		// list lengths' bit lengths; nodes without a list of a kind sort last)
+		// work counters of the node-indexed kernels and the counts of their orders, then the orders
 		ct_status s3 = CT_OK;
-		uint32_t* okey = (uint32_t*) scratch(c, 46, sizeof(uint32_t) * 8 * nn, &s3);
-		int32_t* oidx = (int32_t*) scratch(c, 47, sizeof(int32_t) * 5 * nn, &s3);
-		unsigned long long* onext = (unsigned long long*) scratch(c, 48, 4 * sizeof(unsigned long long), &s3);
+		const size_t onext_bytes = 4 * sizeof(unsigned long long) + 2 * sizeof(int) * ORDER_KINDS * ORDER_BINS;
+		int32_t* oidx = (int32_t*) scratch(c, 47, sizeof(int32_t) * ORDER_KINDS * nn, &s3);
+		unsigned long long* onext = (unsigned long long*) scratch(c, 48, onext_bytes, &s3);
 		CT_TRY(s3);
-		size_t sort_bytes = 0;
-		CT_CUDA(c, cub::DeviceRadixSort::SortPairsDescending(nullptr, sort_bytes, okey, okey + 4 * nn, oidx, oidx + nn, (int) nn, 0, ORDER_KEY_BITS, st));
-		void* sort_tmp = scratch(c, 49, sort_bytes + 256, &s3);
-		CT_TRY(s3);
-		c->launches++;
-		k_order_keys<<<(int) std::max<int64_t>(1, std::min<int64_t>((nn + 255) / 256, c->nsm * 8)), 256, 0, st>>>(nn, b->nodes, o.ecc, o.dcc, o.cp, o.pp, okey,
-				oidx);
-		for (int k = 0; k < 4; k++) {
-			size_t tb = sort_bytes;
-			CT_CUDA(c, cub::DeviceRadixSort::SortPairsDescending(sort_tmp, tb, okey + k * nn, okey + (4 + k) * nn, oidx, oidx + (1 + k) * nn, (int) nn, 0,
-					ORDER_KEY_BITS, st));
+		CT_CUDA(c, cudaMemsetAsync(onext, 0, onext_bytes, st));
+		const OrderArgs oa = { nn, b->nodes, o.ecc, o.dcc, o.cp, o.pp, oidx, (int*) (onext + 4) };
+		const int oblocks = (int) ((nn + ORDER_SPAN - 1) / ORDER_SPAN);
+		if (oblocks > 1) {
+			c->launches++;
+			CT_CUDA(c, launch_behind(k_order_count, oblocks, ORDER_TPB, st, oa));
 		}
-		CT_CUDA(c, cudaMemsetAsync(onext, 0, 4 * sizeof(unsigned long long), st));
+		c->launches++;
+		CT_CUDA(c, launch_behind(k_order_place, oblocks, ORDER_TPB, st, oa));
 		const size_t dl_bytes = sizeof(float) * NEXP_STRIDE * nn;
 		CT_CUDA(c, cudaMemsetAsync(K.dL, 0, dl_bytes, st));
 		// The three kernels run side by side on three streams, each into its own expansion
@@ -1896,16 +1967,16 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 			CT_CUDA(c, cudaStreamWaitEvent(c->side[k], c->fork_ev, 0));
 		}
 		c->launches++;
-		k_m2l_ewald<Ops><<<resident_blocks(c, k_m2l_ewald<Ops>, 128), 128, 0, st>>>(nn, oidx + nn, onext, b->nodes, b->multi, o.ecc, o.ecc_list, K.dL,
+		k_m2l_ewald<Ops><<<resident_blocks(c, k_m2l_ewald<Ops>, 128), 128, 0, st>>>(nn, oidx, onext, b->nodes, b->multi, o.ecc, o.ecc_list, K.dL,
 				kp->do_phi, counters);
 		CT_CUDA(c, cudaMemsetAsync(K.dL2, 0, dl_bytes, c->side[0]));
 		c->launches++;
 		CT_CUDA(c, cudaFuncSetAttribute(k_m2l_direct<Ops>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) M2L_DIRECT_SMEM));
-		k_m2l_direct<Ops><<<resident_blocks(c, k_m2l_direct<Ops>, 128, M2L_DIRECT_SMEM), 128, M2L_DIRECT_SMEM, c->side[0]>>>(nn, oidx + 2 * nn, onext + 1,
+		k_m2l_direct<Ops><<<resident_blocks(c, k_m2l_direct<Ops>, 128, M2L_DIRECT_SMEM), 128, M2L_DIRECT_SMEM, c->side[0]>>>(nn, oidx + nn, onext + 1,
 				b->nodes, b->multi, o.dcc, o.dcc_list, K.dL2, kp->do_phi);
 		CT_CUDA(c, cudaMemsetAsync(K.dL3, 0, dl_bytes, c->side[1]));
 		c->launches++;
-		k_p2l<Ops><<<resident_blocks(c, k_p2l<Ops>, 128), 128, 0, c->side[1]>>>(nn, oidx + 3 * nn, onext + 2, b->nodes, o.cp, o.cp_list, b->x[0], b->x[1],
+		k_p2l<Ops><<<resident_blocks(c, k_p2l<Ops>, 128), 128, 0, c->side[1]>>>(nn, oidx + 2 * nn, onext + 2, b->nodes, o.cp, o.cp_list, b->x[0], b->x[1],
 				b->x[2], K.dL3, counters);
 		for (int k = 0; k < 2; k++) {
 			CT_CUDA(c, cudaEventRecord(c->join_ev[k], c->side[k]));
@@ -1958,7 +2029,7 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 			cudaEventRecord(c->ev[4], st);
 			const int64_t leaf_warps = (int64_t) c->nsm * 24;
 			if (c->tune.warps_per_tile == 1 && tw == 32 && nleaf >= LEAF_WAVES * leaf_warps) {
-				pa.order = oidx + 4 * nn;
+				pa.order = oidx + 3 * nn;
 				pa.nn = nn;
 				pa.next = onext + 3;
 				c->launches++;
