@@ -382,6 +382,7 @@ __global__ void __launch_bounds__(FT_TPB) k_ic_lattice(int N, uint32_t* __restri
 // dx in units of the mean spacing goes to dxmax (float bits: a positive float orders like its bits).
 constexpr int DISP_ROWS = 8;
 constexpr int DISP_X = 8;
+constexpr int IC_MAX_N = 1024;  // points of a grid's axis, at most
 
 // An index at most one grid length outside 0 .. n - 1.
 __device__ __forceinline__ int wrap1(int i, int n) {
@@ -1071,7 +1072,7 @@ extern "C" ct_status ct_initialize(ct_ctx* ctx, int box_id, const ct_ic_params* 
 	}
 	Box* b = c->boxes[box_id];
 	const int N = p->nfour;
-	if (N < 4 || N > 1024 || N % 2 != 0) {
+	if (N < 4 || N > IC_MAX_N || N % 2 != 0) {
 		// (cuFFT's 3-D plans take 32-bit sizes)
 		return fail(c, CT_ERR_ARG, "ct_initialize: nfour must be even, 4 .. 1024");
 	}
@@ -1160,12 +1161,16 @@ extern "C" ct_status ct_initialize(ct_ctx* ctx, int box_id, const ct_ic_params* 
 	k_ic_uniforms<<<ft_grid(c, (int64_t) N * N), FT_TPB, 0, st>>>(N, A);
 	k_ic_amplitude<<<gx, FT_TPB, 0, st>>>(N, box, factor, dtab, A);
 	// interpolation at the lattice points and update of axis dim
-	const size_t disp_smem = sizeof(double) * DISP_ROWS * N;  // 64 KB at the largest grid
-	CT_CUDA(c, cudaFuncSetAttribute(k_ic_displace, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) disp_smem));
+	const size_t disp_smem = sizeof(double) * DISP_ROWS * N;
+	// (the limit belongs to the kernel, whatever context launches it: always the largest grid's 64 KB, so
+	// that calls on other grids from other threads never lower it)
+	CT_CUDA(c, cudaFuncSetAttribute(k_ic_displace, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) sizeof(double) * DISP_ROWS * IC_MAX_N));
 	auto displace = [&](int dim, float D, float prefac, unsigned int* mx) {
 		c->launches += 2;
 		k_ic_sum_x<<<dim3((N * N + FT_TPB - 1) / FT_TPB, (N + DISP_X - 1) / DISP_X), FT_TPB, 0, st>>>(N, R, ax, G);
 		k_ic_displace<<<dim3((N + DISP_ROWS - 1) / DISP_ROWS, N), FT_TPB, disp_smem, st>>>(N, G, ax, scale, D, prefac, box_inv, b->x[dim], b->v[dim], mx);
+		const cudaError_t e = cudaGetLastError();
+		return e == cudaSuccess ? CT_OK : cuda_check(c, e, "interpolation");
 	};
 	// the field of dim1, dim2 in real space
 	auto field = [&](int dim1, int dim2, float* out) {
@@ -1175,7 +1180,7 @@ extern "C" ct_status ct_initialize(ct_ctx* ctx, int box_id, const ct_ic_params* 
 	};
 	for (int dim = 0; dim < 3; dim++) {
 		CT_TRY(field(dim, 3, R));
-		displace(dim, D1, prefac1, dmax + dim);
+		CT_TRY(displace(dim, D1, prefac1, dmax + dim));
 	}
 	if (p->twolpt) {
 		float* R1 = nullptr;
@@ -1198,7 +1203,7 @@ extern "C" ct_status ct_initialize(ct_ctx* ctx, int box_id, const ct_ic_params* 
 			c->launches++;
 			k_ic_correction<<<gx, FT_TPB, 0, st>>>(d2k, Y, N, box, dim, ax.filter);
 			CT_TRY(fft_check(c, cufftExecC2R(S.plans[0], Y, R), "cufftExecC2R"));
-			displace(dim, -D2, prefac2, dmax + 3 + dim);
+			CT_TRY(displace(dim, -D2, prefac2, dmax + 3 + dim));
 		}
 	}
 	CT_CUDA(c, cudaGetLastError());
