@@ -749,6 +749,14 @@ __global__ void k_gather_particles(int64_t b, int64_t n, const int32_t* idx, con
 	}
 }
 
+// One of the fields alone, its values set aside in src.
+template<class T>
+__global__ void k_gather_field(int64_t b, int64_t n, const int32_t* idx, const T* src, T* out) {
+	for (int64_t i = b + blockIdx.x * (int64_t) blockDim.x + threadIdx.x; i < n; i += (int64_t) gridDim.x * blockDim.x) {
+		out[i] = src[idx[i]];
+	}
+}
+
 // ---------------------------------------------------------------- upsweep
 template<class T>
 __device__ __forceinline__ T warp_max(T v) {
@@ -1241,6 +1249,25 @@ ct_status tree_build_t(Ctx* c, Box* b, const ct_tree_params* p) {
 	la.theta = p->theta;
 	la.hsoft = p->hsoft;
 	CT_CUDA(c, cudaMemsetAsync(c->d_flags, 0, 4 * sizeof(int), st));
+	// A build that ends before its gather (node arrays or the gather's scratch out of memory, a barrier that
+	// gave up) has moved positions, and idx with them: a launch ends between phases, and a particle changes
+	// place together with its index.  Velocities and rungs follow before the error returns, field by field
+	// through the partition scratch, which takes no memory.
+	auto stopped = [&](ct_status why) {
+		for (int d = 0; d < 4 && np > 0; d++) {
+			void* field = d < 3 ? (void*) (b->v[d] + pb) : (void*) (b->rung + pb);
+			const size_t size = d < 3 ? sizeof(float) : sizeof(int8_t);
+			CT_CUDA(c, cudaMemcpyAsync((char*) la.posL + size * pb, field, size * np, cudaMemcpyDeviceToDevice, st));
+			c->launches++;
+			if (d < 3) {
+				k_gather_field<<<grid_for(c, np, 256), 256, 0, st>>>(pb, n, la.idx, (const float*) la.posL, b->v[d]);
+			} else {
+				k_gather_field<<<grid_for(c, np, 256), 256, 0, st>>>(pb, n, la.idx, (const int8_t*) la.posL, b->rung);
+			}
+			CT_CUDA(c, cudaGetLastError());
+		}
+		return why;
+	};
 	int32_t* h_tot = (int32_t*) c->pinned;
 	LevelCtl* hc = (LevelCtl*) ((char*) c->pinned + 64);
 	for (la.resume = 0;; la.resume = 1) {
@@ -1258,13 +1285,16 @@ ct_status tree_build_t(Ctx* c, Box* b, const ct_tree_params* p) {
 		CT_CUDA(c, cudaMemcpyAsync(hc, la.ctl, sizeof(LevelCtl), cudaMemcpyDeviceToHost, st));
 		CT_CUDA(c, cudaStreamSynchronize(st));
 		if (hc->error) {
-			return fail(c, CT_ERR_CUDA, "tree build: the blocks of the cooperative grid did not meet");
+			return stopped(fail(c, CT_ERR_CUDA, "tree build: the blocks of the cooperative grid did not meet"));
 		}
 		if (hc->status == 0) {
 			break;
 		}
 		// the levels so far stay; the level that did not fit starts again with room for its children
-		CT_TRY(ensure_nodes(c, b, hc->need));
+		const ct_status room = ensure_nodes(c, b, hc->need);
+		if (room != CT_OK) {
+			return stopped(room);
+		}
 	}
 	std::vector<int64_t> levels(hc->start, hc->start + hc->level + 2);
 	b->level_start = levels;  // level k = [levels[k], levels[k+1])
@@ -1277,7 +1307,9 @@ ct_status tree_build_t(Ctx* c, Box* b, const ct_tree_params* p) {
 		float* t1 = (float*) scratch(c, 18, sizeof(float) * n, &s2);
 		float* t2 = (float*) scratch(c, 19, sizeof(float) * n, &s2);
 		int8_t* tr = (int8_t*) scratch(c, 20, n + 16, &s2);
-		CT_TRY(s2);
+		if (s2 != CT_OK) {
+			return stopped(s2);
+		}
 		if (np > 0) {
 			c->launches += 2;
 			k_stage_particles<<<grid_for(c, np, 256), 256, 0, st>>>(pb, n, b->v[0], b->v[1], b->v[2], b->rung, t0, t1, t2, tr);
