@@ -949,15 +949,7 @@ ct_status ct_box_destroy(ct_ctx* ctx, int box_id) {
 	}
 	dfree(c, b->pot, sizeof(float) * b->g_cap);
 	dfree(c, b->rung, n + 16);
-	const int64_t cap = b->node_cap;
-	dfree(c, b->nodes, sizeof(NodeW) * cap);
-	dfree(c, b->nbox, sizeof(int32_t) * 6 * cap);
-	dfree(c, b->multi, sizeof(float) * NMULT_STRIDE * cap);
-	dfree(c, b->key, sizeof(uint64_t) * cap);
-	dfree(c, b->depth, sizeof(int32_t) * cap);
-	dfree(c, b->parent, sizeof(int32_t) * cap);
-	dfree(c, b->gbox, sizeof(double) * 6 * cap);
-	dfree(c, b->tbox, sizeof(double) * 6 * cap);
+	nodes_release(c, b);
 	dfree(c, b->d_sub_off, sizeof(int64_t) * (b->sub_cap + 1));
 	dfree(c, b->d_sub_sums, sizeof(double) * 9 * b->sub_cap);
 	dfree(c, b->d_sub_maxrung, sizeof(int) * b->sub_cap);

@@ -97,7 +97,8 @@ struct Box {
 	float* pot = nullptr;
 	// tree
 	int64_t nnodes = 0;
-	int64_t node_cap = 0;
+	int64_t node_cap = 0;              // nodes that all of the following arrays hold
+	int64_t node_have[8] = {};         // nodes that each of them holds (more, when the others failed to grow)
 	std::vector<int64_t> level_start;  // node index where each level begins (host copy)
 	NodeW* nodes = nullptr;
 	int32_t* nbox = nullptr;    // tight box, fixed<int,29>, 6 per node (b0 b1 b2 e0 e1 e2)
@@ -138,6 +139,9 @@ struct Box {
 
 // Frees a box's lightcone buffers (ct_lightcone.cu).
 void lightcone_release(Ctx* c, Box* b);
+
+// Frees a box's node arrays (ct_tree.cu).
+void nodes_release(Ctx* c, Box* b);
 
 struct FtPlans;  // cuFFT plans kept between calls (ct_fourier.cu)
 void fourier_release(Ctx* c);  // frees them (called by ct_ctx_destroy)

@@ -1168,16 +1168,33 @@ __global__ void __launch_bounds__(UPS_TPB, 2) k_upsweep(int64_t lb, int64_t le, 
 	}
 }
 
+// The node arrays in the order of Box::node_have, with their elements a node.
+template<class F>
+ct_status each_node_array(Box* b, F f) {
+	CT_TRY(f(&b->nodes, b->node_have[0], 1, "tree nodes"));
+	CT_TRY(f(&b->nbox, b->node_have[1], 6, "node boxes"));
+	CT_TRY(f(&b->multi, b->node_have[2], NMULT_STRIDE, "multipoles"));
+	CT_TRY(f(&b->key, b->node_have[3], 1, "node keys"));
+	CT_TRY(f(&b->depth, b->node_have[4], 1, "node depth"));
+	CT_TRY(f(&b->parent, b->node_have[5], 1, "node parent"));
+	CT_TRY(f(&b->gbox, b->node_have[6], 6, "node geometric box"));
+	return f(&b->tbox, b->node_have[7], 6, "node tight box");
+}
+
 template<class T>
-ct_status grow(Ctx* c, T** p, int64_t old_n, int64_t new_n, int per, const char* what) {
+ct_status grow(Ctx* c, T** p, int64_t& have, int64_t need, int per, const char* what) {
+	if (need <= have) {
+		return CT_OK;
+	}
 	T* q = nullptr;
-	CT_TRY(dalloc(c, (void**) &q, sizeof(T) * per * new_n, what));
+	CT_TRY(dalloc(c, (void**) &q, sizeof(T) * per * need, what));
 	if (*p) {
-		CT_CUDA(c, cudaMemcpyAsync(q, *p, sizeof(T) * per * old_n, cudaMemcpyDeviceToDevice, c->stream));
+		CT_CUDA(c, cudaMemcpyAsync(q, *p, sizeof(T) * per * have, cudaMemcpyDeviceToDevice, c->stream));
 		CT_CUDA(c, cudaStreamSynchronize(c->stream));
-		dfree(c, *p, sizeof(T) * per * old_n);
+		dfree(c, *p, sizeof(T) * per * have);
 	}
 	*p = q;
+	have = need;
 	return CT_OK;
 }
 
@@ -1187,15 +1204,7 @@ ct_status ensure_nodes(Ctx* c, Box* b, int64_t need) {
 	}
 	int64_t cap = std::max<int64_t>(need, b->node_cap * 3 / 2);
 	cap = std::max<int64_t>(cap, 1024);
-	const int64_t old = b->node_cap;
-	CT_TRY(grow(c, &b->nodes, old, cap, 1, "tree nodes"));
-	CT_TRY(grow(c, &b->nbox, old, cap, 6, "node boxes"));
-	CT_TRY(grow(c, &b->multi, old, cap, NMULT_STRIDE, "multipoles"));
-	CT_TRY(grow(c, &b->key, old, cap, 1, "node keys"));
-	CT_TRY(grow(c, &b->depth, old, cap, 1, "node depth"));
-	CT_TRY(grow(c, &b->parent, old, cap, 1, "node parent"));
-	CT_TRY(grow(c, &b->gbox, old, cap, 6, "node geometric box"));
-	CT_TRY(grow(c, &b->tbox, old, cap, 6, "node tight box"));
+	CT_TRY(each_node_array(b, [&](auto** p, int64_t& have, int per, const char* what) { return grow(c, p, have, cap, per, what); }));
 	b->node_cap = cap;
 	return CT_OK;
 }
@@ -1344,6 +1353,16 @@ ct_status tree_build_t(Ctx* c, Box* b, const ct_tree_params* p) {
 }
 
 }  // namespace
+
+void nodes_release(Ctx* c, Box* b) {
+	each_node_array(b, [&](auto** p, int64_t& have, int per, const char*) {
+		dfree(c, *p, sizeof(**p) * per * have);
+		*p = nullptr;
+		have = 0;
+		return (ct_status) CT_OK;
+	});
+	b->node_cap = 0;
+}
 
 ct_status tree_build(Ctx* c, Box* b, const ct_tree_params* p) {
 	if (c->order == 5) {
