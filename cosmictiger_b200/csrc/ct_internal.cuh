@@ -88,7 +88,7 @@ struct Box {
 	int64_t cap = 0;         // particles the x, v, rung arrays hold
 	int64_t g_cap = 0;       // particles the g, pot arrays hold
 	int sub_cap = 0;         // sub-boxes the per-box arrays hold
-	int64_t rung_begin = 0;  // tree covers [rung_begin, n)
+	int64_t rung_begin = 0;  // start of the active range of a single box
 	// particles (SoA)
 	uint32_t* x[3] = { nullptr, nullptr, nullptr };
 	float* v[3] = { nullptr, nullptr, nullptr };
@@ -135,6 +135,11 @@ struct Box {
 	uint64_t* lc_cand = nullptr;   // candidate (particle, image) pairs of one drift
 	int64_t lc_cand_cap = 0;
 	unsigned long long* d_lc_ctr = nullptr;  // [0] candidates, [1] entries
+	// The tree and the kick cover particles [tree_begin(), n): an ensemble is kicked with all its
+	// particles active, whatever rung state a caller has set on it.
+	int64_t tree_begin() const {
+		return nsub > 1 ? 0 : rung_begin;
+	}
 };
 
 // Frees a box's lightcone buffers (ct_lightcone.cu).

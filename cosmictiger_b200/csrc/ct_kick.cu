@@ -1872,7 +1872,7 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 	cudaStream_t st = c->stream;
 	KickBuffers& K = kbuf(c);
 	const int64_t nn = b->nnodes;
-	const int64_t np = b->n - b->rung_begin;
+	const int64_t np = b->n - b->tree_begin();
 	// per-node list descriptors
 	CT_TRY(ensure(c, &K.per_node, K.per_node_n, (size_t) 7 * nn, "walk descriptors"));
 	CT_TRY(ensure(c, &K.dL, K.dL_n, (size_t) NEXP_STRIDE * nn, "expansion deltas"));

@@ -1218,7 +1218,7 @@ template<class Ops>
 ct_status tree_build_t(Ctx* c, Box* b, const ct_tree_params* p) {
 	cudaStream_t st = c->stream;
 	const int64_t n = b->n;
-	const int64_t pb = b->rung_begin;
+	const int64_t pb = b->tree_begin();
 	const int64_t np = n - pb;
 	b->tree_valid = false;
 	if (np > INT32_MAX / 2) {
