@@ -766,6 +766,8 @@ struct OrderArgs {
 	const int2 *ecc, *dcc, *cp, *pp;
 	int32_t* order;  // [ORDER_KINDS][nn]
 	int* count;      // [ORDER_KINDS][ORDER_BINS] nodes, then as many placed so far (zero before)
+	const int* bad;  // the walk's flags: its lists did not fit, or a check failed
+	unsigned long long* next;  // [ORDER_KINDS] the kernels' work counters
 };
 __device__ __forceinline__ void order_keys(const OrderArgs& a, int64_t i, int (&key)[ORDER_KINDS]) {
 	const NodeW nd = a.nodes[i];
@@ -819,6 +821,13 @@ __global__ void __launch_bounds__(ORDER_TPB) k_order_place(const OrderArgs a) {
 	__shared__ int s_hist[ORDER_KINDS][ORDER_BINS], s_at[ORDER_KINDS][ORDER_BINS];
 	int key[ORDER_ITEMS][ORDER_KINDS], rank[ORDER_ITEMS][ORDER_KINDS];
 	front_done();
+	if (a.bad[0] | a.bad[1]) {
+		// the walk has to be made again: the orders' kernels find all nodes taken
+		if (blockIdx.x == 0 && threadIdx.x < ORDER_KINDS) {
+			a.next[threadIdx.x] = (unsigned long long) a.nn;
+		}
+		return;
+	}
 	order_count(a, s_hist, key, rank);
 	for (int e = threadIdx.x; e < ORDER_KINDS * ORDER_BINS; e += ORDER_TPB) {
 		const int k = e / ORDER_BINS, bin = e - k * ORDER_BINS;
@@ -1521,8 +1530,13 @@ __global__ void __launch_bounds__(LEAF_TPB, 6) k_p2p_leaf(P2PArgs a) {
 }
 
 // The tile list: tw sinks a tile (order within each kind is immaterial: every tile computes its own
-// sinks), one atomic a warp and kind.
-__global__ void __launch_bounds__(256) k_leaf_tiles(int64_t nn, const NodeW* __restrict__ nodes, int tw, int64_t cap, int2* __restrict__ items, unsigned long long* count) {
+// sinks), one atomic a warp and kind.  Empty when the walk has to be made again (bad: its flags), so
+// that nothing is summed and nothing is kicked.
+__global__ void __launch_bounds__(256) k_leaf_tiles(int64_t nn, const NodeW* __restrict__ nodes, int tw, int64_t cap, const int* bad, int2* __restrict__ items,
+		unsigned long long* count) {
+	if (bad[0] | bad[1]) {
+		return;
+	}
 	const int lane = threadIdx.x & 31;
 	for (int64_t i0 = blockIdx.x * (int64_t) blockDim.x + (threadIdx.x - lane); i0 < nn; i0 += (int64_t) gridDim.x * blockDim.x) {
 		const int64_t i = i0 + lane;
@@ -1570,7 +1584,6 @@ struct KickTileArgs {
 	const float* multi;
 	const float* Lx;
 	TileList tiles;
-	const int* bad;  // the walk's flags: nothing is kicked when its lists did not fit
 	const int2* pc;
 	const int* pc_list;
 	const float4* F;
@@ -1600,7 +1613,7 @@ __global__ void __launch_bounds__(128, 3) k_leaf_kick(KickTileArgs a) {
 		acc[q] = 0.0;
 	}
 	int maxr = 0;
-	const int64_t nbig = a.tiles.big(), nitems = (a.bad[0] | a.bad[1]) ? 0 : nbig + a.tiles.small();
+	const int64_t nbig = a.tiles.big(), nitems = nbig + a.tiles.small();
 	for (int64_t it = warp_take(a.next, 1); it < nitems; it = warp_take(a.next, 1)) {
 		const int2 item = a.tiles.items[it < nbig ? it : a.tiles.cap - 1 - (it - nbig)];
 		const NodeW self = a.nodes[item.x];
@@ -1937,8 +1950,8 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 		}
 		CT_CUDA(c, cudaGetLastError());
 		cudaEventRecord(c->ev[1], st);
-		// (whether the lists fitted is read with the results: the kernels that follow run on what fitted,
-		// and the leaf kick changes nothing if something did not)
+		// (whether the lists fitted is read with the results: if they did not, the kernels that follow find
+		// no work)
 		// ---- interactions
 		CT_CUDA(c, cudaMemsetAsync(counters, 0, 16 * sizeof(double), st));
 		// work counters of the node-indexed kernels and the counts of their orders, then the orders
@@ -1948,7 +1961,7 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 		unsigned long long* onext = (unsigned long long*) scratch(c, 48, onext_bytes, &s3);
 		CT_TRY(s3);
 		CT_CUDA(c, cudaMemsetAsync(onext, 0, onext_bytes, st));
-		const OrderArgs oa = { nn, b->nodes, o.ecc, o.dcc, o.cp, o.pp, oidx, (int*) (onext + 4) };
+		const OrderArgs oa = { nn, b->nodes, o.ecc, o.dcc, o.cp, o.pp, oidx, (int*) (onext + 4), c->d_flags, onext };
 		const int oblocks = (int) ((nn + ORDER_SPAN - 1) / ORDER_SPAN);
 		if (oblocks > 1) {
 			c->launches++;
@@ -2006,7 +2019,7 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 			float4* F = (float4*) scratch(c, 44, sizeof(float4) * b->n, &s2);
 			CT_TRY(s2);
 			c->launches++;
-			k_leaf_tiles<<<(int) std::max<int64_t>(1, std::min<int64_t>((nn + 255) / 256, c->nsm * 8)), 256, 0, st>>>(nn, b->nodes, tw, tile_cap, items, tcount);
+			k_leaf_tiles<<<(int) std::max<int64_t>(1, std::min<int64_t>((nn + 255) / 256, c->nsm * 8)), 256, 0, st>>>(nn, b->nodes, tw, tile_cap, c->d_flags, items, tcount);
 			const TileList tiles { items, tile_cap, tcount };
 			P2PArgs pa;
 			pa.nsub = b->nsub;
@@ -2065,7 +2078,6 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 			ka.multi = b->multi;
 			ka.Lx = K.Lx;
 			ka.tiles = tiles;
-			ka.bad = c->d_flags;
 			ka.pc = o.pc;
 			ka.pc_list = o.pc_list;
 			ka.F = F;
