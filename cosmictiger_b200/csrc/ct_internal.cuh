@@ -223,7 +223,7 @@ inline cudaError_t launch_behind(void (*kernel)(P...), int blocks, int threads, 
 	cfg.stream = st;
 	cfg.attrs = &attr;
 	cfg.numAttrs = 1;
-	return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+	return cudaLaunchKernelEx(&cfg, kernel, args...);  // (converts as a call would, no casts)
 }
 #endif
 
