@@ -216,7 +216,7 @@ __global__ void k_ic_axis(int N, float box_size, AxisTables t) {
 	}
 }
 
-// Grid of one (x, y) row of modes or points a block row: blockIdx.y = I1, blockIdx.z = I0.
+// A mode times the inverse window, axis by axis.
 __device__ __forceinline__ float2 filtered(float2 v, float fx, float fy, float fz) {
 	v = make_float2(v.x * fx, v.y * fx);
 	v = make_float2(v.x * fy, v.y * fy);

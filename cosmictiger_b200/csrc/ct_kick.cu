@@ -13,12 +13,16 @@
 //                down to both of its children.
 // Every node's lists land contiguously in global memory (per-warp staging), so that the
 // interaction kernels that follow read them with one pass per node:
-//   k_m2l        Ewald and direct M2L plus P2L into the node's own expansion delta (warp per
-//                node, lanes over sources, butterfly reduction; gravity.cu:44-155,213-244);
-//   k_l2l        top-down L2L: L(node) = L2L(L(parent)) + delta (kick.cu:246-258);
-//   k_leaf       M2P, P2P (sources staged in shared memory as floats relative to the leaf
-//                centre, compensated per-batch accumulation), L2P and the kick
-//                (gravity.cu:157-211,246-404, kick.cu:53-177).
+//   k_order_count, k_order_place  the nodes by list length of each kind, longest first;
+//   k_m2l_ewald, k_m2l_direct, k_p2l  Ewald M2L, direct M2L and P2L side by side, each into
+//                expansion sums of its own (a warp a node, lanes over sources;
+//                gravity.cu:44-155,213-244);
+//   k_l2l        top-down L2L: L(node) = L2L(L(parent)) + the three sums (kick.cu:246-258);
+//   k_leaf_tiles the leaves' tiles of at most 32 sinks;
+//   k_p2p, k_p2p_leaf  P2P by tiles or by whole leaves (sources staged in shared memory as
+//                floats relative to the leaf centre, compensated per-batch accumulation;
+//                gravity.cu:246-404);
+//   k_leaf_kick  M2P, L2P and the kick (gravity.cu:157-211, kick.cu:53-177).
 #include <cstdlib>
 #include <mutex>
 

@@ -27,7 +27,11 @@ namespace {
 
 // ---------------------------------------------------------------- the levels
 // One cooperative launch builds every level: a resident grid whose blocks meet at grid barriers
-// (1.2 us from the last arrival) between the phases of a level.  What bounded the build before was the
+// (1.2 us from the last arrival) between the phases of a level.  The launch is cooperative, for
+// which CUDA guarantees that all blocks of the grid are resident together: a barrier waits for blocks
+// that run, never for one without room, and that holds for each grid by itself, however many contexts
+// build at a time and at whatever priority.  A barrier that has waited 30 s all the same ends the launch
+// with an error.  What bounded the build before was the
 // level's structure, not its data: twelve launches, two scans and a host round trip a level (16^3
 // particles: 0.87 ms for 11 levels and 64 KB of positions; 10^6 clustered particles: 2.7 ms for 28
 // levels).  By the number of nodes on the level:
@@ -35,9 +39,11 @@ namespace {
 //   particles and by the whole block up to BLOCK_LINE, which is quickest for one node.  A child is
 //   counted by the block that makes it, so that the level takes one barrier.
 //   many: a warp partitions up to WARP_FEW particles (WARP_MANY where there are two nodes a warp), and
-//   warps take nodes from all shares, since the shares' work is uneven in a clustered box; three
-//   barriers.
-// Larger nodes go tile by tile over the whole grid, three barriers more.
+//   warps take nodes from all shares, since the shares' work is uneven in a clustered box; the level
+//   ends with two barriers (numbering, partition).
+// Larger nodes go tile by tile over the whole grid: four barriers for a level with any (numbering,
+// ballots, positions, swaps).  A level whose nodes were not counted as they were made (the first, and
+// each behind a level of many nodes or of tiles) counts them itself, one barrier more.
 constexpr int LTPB = 512;             // threads of a level block
 constexpr int LWARPS = LTPB / 32;
 constexpr int SUB = 1024;             // particles whose ballots a warp's lanes hold, one each
@@ -315,7 +321,7 @@ __device__ __forceinline__ int warp_partition(const LevelArgs& a, const NodeW& n
 struct LevelShared {
 	uint16_t pos[LWARPS][SUB];
 	int scan[3][LWARPS];
-	int sum[2][LWARPS];
+	int sum[LWARPS];
 	int totals[7][LWARPS];
 	unsigned mask[LWARPS];
 	int tot[3];
@@ -353,12 +359,12 @@ __device__ __forceinline__ void tile_positions(const LevelArgs& a, LevelShared& 
 	const int here = __reduce_add_sync(0xffffffffu, __popc(mine));
 	__syncthreads();
 	if (lane == 0) {
-		sh.sum[0][w] = here;
+		sh.sum[w] = here;
 	}
 	__syncthreads();
 	int lt = lt_prev;
 	for (int i = 0; i < w; i++) {
-		lt += sh.sum[0][i];
+		lt += sh.sum[i];
 	}
 	const int sb = tb + sub * w, n = min(sub, pend - sb);
 	if (n > 0) {
@@ -772,14 +778,6 @@ __device__ __forceinline__ T warp_min(T v) {
 	}
 	return v;
 }
-template<class T>
-__device__ __forceinline__ T warp_sum(T v) {
-	for (int o = 16; o; o >>= 1) {
-		v += __shfl_xor_sync(0xffffffffu, v, o);
-	}
-	return v;
-}
-
 constexpr int UTPB = 128;
 
 // Sums of N doubles per lane over the warp: afterwards lane l has the sums of entries k with
@@ -1230,7 +1228,7 @@ ct_status tree_build_t(Ctx* c, Box* b, const ct_tree_params* p) {
 	ct_status s1 = CT_OK;
 	const int nroot = b->nsub;
 	CT_TRY(ensure_nodes(c, b, nroot + 1));
-	// one block an SM (two boxes built by two contexts fit side by side), fewer for a few particles
+	// one block an SM (half of what fits, so that two contexts build side by side), fewer for a few particles
 	const int nblk = (int) std::max<int64_t>(1, std::min<int64_t>(c->nsm, std::max<int64_t>(np / 64, nroot)));
 	LevelArgs la;
 	la.idx = (int32_t*) scratch(c, 0, sizeof(int32_t) * n, &s1);
