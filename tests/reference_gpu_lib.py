@@ -27,6 +27,21 @@ def available():
     return os.path.exists(LIB)
 
 
+def require():
+    """An instance of the library.  It can only be built where the reference's sources are; its
+    tests skip where neither they nor the built library are, and fail where the sources are but
+    the build left it out."""
+    if not available():
+        import pytest
+
+        from __graft_entry__ import REFERENCE_DIR
+
+        if os.path.isfile(os.path.join(REFERENCE_DIR, "src", "kick.cu")):
+            pytest.fail("oracle/_ref/libctref_gpu.so is not built (make -C oracle refgpu)")
+        pytest.skip("oracle/_ref/libctref_gpu.so not built (needs the reference's sources)")
+    return ReferenceGPU()
+
+
 class ReferenceGPU:
     """The reference's device heap (cuda_mem_init) is set up once per process, with the size of
     the first instance.  Its allocator traps the kernel when the heap runs out

@@ -22,9 +22,7 @@ def ctx():
 def ref():
     from tests import reference_gpu_lib
 
-    if not reference_gpu_lib.available():
-        pytest.fail("oracle/_ref/libctref_gpu.so is not built (make -C oracle refgpu)")
-    return reference_gpu_lib.ReferenceGPU()
+    return reference_gpu_lib.require()
 
 
 def _state(n=24, seed=21, vscale=1.0, nrung=3):

@@ -32,9 +32,7 @@ def rel_rms(a, b):
 
 @pytest.fixture(scope="module")
 def ref():
-    if not rg.available():
-        pytest.fail("oracle/_ref/libctref_gpu.so is not built (make -C oracle refgpu)")
-    return rg.ReferenceGPU()
+    return rg.require()
 
 
 @pytest.fixture(scope="module")
