@@ -1588,6 +1588,7 @@ struct KickTileArgs {
 	const float* multi;
 	const float* Lx;
 	TileList tiles;
+	const int* bad;  // the walk's flags: nothing is kicked when its lists did not fit
 	const int2* pc;
 	const int* pc_list;
 	const float4* F;
@@ -1617,7 +1618,7 @@ __global__ void __launch_bounds__(128, 3) k_leaf_kick(KickTileArgs a) {
 		acc[q] = 0.0;
 	}
 	int maxr = 0;
-	const int64_t nbig = a.tiles.big(), nitems = nbig + a.tiles.small();
+	const int64_t nbig = a.tiles.big(), nitems = (a.bad[0] | a.bad[1]) ? 0 : nbig + a.tiles.small();
 	for (int64_t it = warp_take(a.next, 1); it < nitems; it = warp_take(a.next, 1)) {
 		const int2 item = a.tiles.items[it < nbig ? it : a.tiles.cap - 1 - (it - nbig)];
 		const NodeW self = a.nodes[item.x];
@@ -2082,6 +2083,7 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 			ka.multi = b->multi;
 			ka.Lx = K.Lx;
 			ka.tiles = tiles;
+			ka.bad = c->d_flags;
 			ka.pc = o.pc;
 			ka.pc_list = o.pc_list;
 			ka.F = F;
