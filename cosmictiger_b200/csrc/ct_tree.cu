@@ -973,6 +973,8 @@ constexpr int UPS_ALONE = 256;   // particles that one warp goes through by itse
 // were bound by the issue of double operations (430 us at 33,000 nodes) and a large node's pass by 256
 // dependent reads.  All levels, order 7: 256^3 particles 2,275 us -> 1,580; 64 boxes of 64^3 930 -> 610; a
 // 64^3 box's upper rungs 575 -> 230; 16^3 81 -> 77 (5 to 8 us a level: one chain of reads, roots and the shift).
+// Two blocks an SM bound it to 128 registers, at which order 7 spills 52 bytes; one block without spills
+// took 0.85 ms more of the build of 256^3 particles.
 template<class Ops>
 __global__ void __launch_bounds__(UPS_TPB, 2) k_upsweep(int64_t lb, int64_t le, int group, NodeW* nodes, int32_t* nbox, float* multi, double* tbox, const double* gbox,
 		const uint32_t* x0, const uint32_t* x1, const uint32_t* x2, int bucket) {
