@@ -22,7 +22,7 @@ def test_kick_after_lists_that_did_not_fit():
     extra = []
     for _ in range(3):
         ctx = ct.Context(order=7)
-        ctx.box(200 * 10 ** 6).close()  # 5 GB in the context's pool: no allocation below goes to the driver
+        ctx.box(200 * 10 ** 6).close()  # 5 GB in the context's pool: no allocation below goes to the CUDA driver
         box = ctx.box(n)
         times, launches, out = [], [], []
         for _ in range(2):
