@@ -2016,6 +2016,10 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 		CT_CUDA(c, cudaMemsetAsync(tcount, 0, 3 * sizeof(unsigned long long), st));
 		cudaEventRecord(c->ev[4], st);
 		cudaEventRecord(c->ev[5], st);
+		if (b->nsub > 1) {
+			CT_CUDA(c, cudaMemsetAsync(b->d_sub_sums, 0, sizeof(double) * 9 * b->nsub, st));
+			CT_CUDA(c, cudaMemsetAsync(b->d_sub_maxrung, 0, sizeof(int) * b->nsub, st));
+		}
 		cudaEventRecord(c->ev[12], st);  // no particles: zero P2P and leaf-kick times
 		if (np > 0) {
 			ct_status s2 = CT_OK;
@@ -2075,10 +2079,6 @@ ct_status kick_t(Ctx* c, Box* b, const ct_kick_params* kp, ct_kick_return* out) 
 			ka.sub_h = b->d_sub_h;
 			ka.sub_GM = b->d_sub_GM;
 			ka.sub_first = b->d_sub_first;
-			if (b->nsub > 1) {
-				CT_CUDA(c, cudaMemsetAsync(b->d_sub_sums, 0, sizeof(double) * 9 * b->nsub, st));
-				CT_CUDA(c, cudaMemsetAsync(b->d_sub_maxrung, 0, sizeof(int) * b->nsub, st));
-			}
 			ka.nodes = b->nodes;
 			ka.multi = b->multi;
 			ka.Lx = K.Lx;

@@ -33,3 +33,22 @@ def test_rung_state_of_an_ensemble(begin):
     assert a[1:] == b[1:]
     for k in a[0]:
         assert np.array_equal(a[0][k], b[0][k]), k
+
+
+def test_ensemble_without_particles():
+    """Boxes that hold nothing return zeros, also when no box of the ensemble holds anything."""
+    import cosmictiger_b200 as ct
+
+    ctx = ct.Context(order=7)
+    # an earlier ensemble of that size leaves its sums in the memory that the next one gets
+    for counts in ([500, 700], [0, 0]):
+        n = sum(counts)
+        rng = np.random.default_rng(1)
+        box = ctx.ensemble(counts)
+        box.upload(*(ics.to_fixed32(q) for q in rng.random((3, n))), np.ones((n, 3), np.float32), np.full(n, 1, np.int8))
+        box.tree_create(0.7, 1e-3, 32)
+        got = box.kick_ensemble(ct.KickParams.make(theta=0.7, h=1e-3, GM=1e-3, eta=ics.eta_default(), t0=1e-3))
+        box.close()
+    ctx.close()
+    for r in got:
+        assert [getattr(r, f) for f, _ in r._fields_] == [0] * len(r._fields_)
